@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(128) k_cells_update(SoA<R> s, const uint8_t *_
         const R dg = dvgap ? (R)dvgap[i] : (R)0;
         const int ct = ctype[i];
         StepOut<R> o{};
-        for (int64_t t = 0; t < nsteps; ++t) tpord_step<R>(c, ct, m, k, is, dg, &o);
+        for (int64_t t = 0; t < nsteps; ++t) tpord_update(c, ct, m, k, is, dg, &o);
         store_cell(c, s, i);
         s.v[i] = c.v;
         if (dvdt) dvdt[i] = (double)o.dvdt;

@@ -164,7 +164,7 @@ __device__ __forceinline__ void grid_step_voxel(const GridDev<R> &gd, const Step
     load_cell(c, gd.s, k);
     c.v = vc;
     StepOut<R> o{};
-    tpord_step<R>(c, ctl & kCtlType, gd.model, kst, ist, du, &o);
+    tpord_update(c, ctl & kCtlType, gd.model, kst, ist, du, &o);
     store_cell(c, gd.s, k);
     Vn[g] = c.v;
     if (gd.det) grid_detect(gd, ck, k, (float)vc, (float)c.v, (float)o.dvdt);

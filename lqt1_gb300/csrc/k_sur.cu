@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(128) k_sur_datagen(const SurCell *__restrict__
                     xr[43] = cls == 2;
                     CellState<float> cc = c;
                     StepOut<float> oc;
-                    tpord_step<float>(cc, ct, m, kmac, 0.f, 0.f, &oc);
+                    tpord_update(cc, ct, m, kmac, 0.f, 0.f, &oc);
                     state38(cc, xc);
                     float2 *cp[8];
                     conc_ptrs(cc, cp);
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(128) k_sur_datagen(const SurCell *__restrict__
             }
         }
         const float ist = (ph >= sc.stim_on && ph < sc.stim_off) ? sc.stim : (slot >= 0 ? 0.f : ipert);
-        tpord_step<float>(c, ct, m, k, ist, 0.f, &o);
+        tpord_update(c, ct, m, k, ist, 0.f, &o);
     }
     if (counts) counts[i] = nrec;
 }

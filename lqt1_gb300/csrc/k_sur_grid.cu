@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
         // 2. coarse TPORd step of the macro length, overlapping layer 1
         if (elig) {
             StepOut<float> o;
-            tpord_step<float>(c, ct, gd.model, sg.kmac, 0.f, 0.f, &o);
+            tpord_update(c, ct, gd.model, sg.kmac, 0.f, 0.f, &o);
         }
         // 3. the rest of the network
         bool have_net = false;

@@ -2,7 +2,8 @@
 // TPORd::update(), SingleCell/TPORd.cc:379-1021; GPU copies GPU3D.cu:425-1220,
 // new_11.cu:459-1239) for the sm_103a kernels.
 //
-// One source serves two arithmetic forms through a precision policy:
+// One source serves two arithmetic forms through a precision policy (the mixed
+// form has a second, faster writing, tpord_f32.cuh):
 //   R = double : the plain FP64 form.  Divisions, exp and log follow the
 //                reference expression by expression; integer powers are
 //                multiplications and constant-tau decays are precomputed on
@@ -523,3 +524,5 @@ __device__ __forceinline__ void tpord_step(CellState<R> &c, int ctype, const Mod
 }
 
 }  // namespace lqt
+
+#include "tpord_f32.cuh"

@@ -1,0 +1,54 @@
+"""The mixed form's fast step (tpord_f32.cuh) against the FP64 oracle at the
+voltages where its rewritten terms change form: the GHK polynomial's limit
+(|V F/RT| = 0.5) and its value at V = 0, the INa branch at -40 mV, and far
+outside the action potential, where the bounded exponentials saturate.
+
+Tolerances: a gate is a convex combination of its old value and its steady
+state, each within a few FP32 roundings of exponentials whose arguments stay
+below 2^6 (argument rounding 2^-19, so 2e-6 of the value): 1e-5.  V: the
+currents carry the same relative error; 1e-5 of the change in the step and of
+the sum of the current magnitudes they are taken from, plus the rounding of V."""
+import numpy as np
+import pytest
+
+import lqt1_gb300 as lq
+from oracle import orc
+
+pytestmark = pytest.mark.gpu
+
+RT_F = 8314.0 * 310.0 / 96485.0
+EDGES = np.array([0.0, 1e-6, -1e-6, 1e-3, -1e-3, 0.5 * RT_F, np.nextafter(np.float32(0.5 * RT_F), 100),
+                  -0.5 * RT_F, 0.0026, -0.0026, -40.0, np.nextafter(np.float32(-40), 0), -40.00001])
+
+
+@pytest.mark.parametrize("dt", [0.02, 0.2])
+@pytest.mark.parametrize("vrange", [(-120.0, 80.0), (-250.0, 290.0)])
+@pytest.mark.parametrize("n", [1, 33, 4099])
+def test_step_against_oracle(n, vrange, dt):
+    rng = np.random.default_rng(n)
+    s0 = orc.random_states(n, seed=n)
+    v = rng.uniform(*vrange, n)
+    m = min(n, len(EDGES))
+    v[:m] = EDGES[:m]
+    s0[:, 0] = v.astype(np.float32)
+    s0[:, 9:] = s0[:, 9:].astype(np.float32)
+    types = rng.integers(0, 5, n).astype(np.uint8)
+    for om, lm in ((orc.model("default"), lq.model("default")),
+                   (orc.model("baseline", gks_scale=0.5, pca_scale=2.0, gks_iso_scale=1.5),
+                    lq.model("baseline", gks_scale=0.5, pca_scale=2.0, gks_iso_scale=1.5))):
+        # at V = 0 the reference's GHK terms are 0/0: its limit, 1e-6 mV away
+        so = s0.copy()
+        so[so[:, 0] == 0.0, 0] = 1e-6
+        ref = orc.cells_update(so, types, om, dt=dt, nsteps=1)
+        c = lq.TPORdCells(types, precision=lq.MIXED, model=lm, dt=dt)
+        c.set_state(s0)
+        c.update(1)
+        got = c.get_state()
+        cur = c.get_currents()
+        c.close()
+        assert np.all(np.isfinite(got))
+        gates = [j for j in range(9, 37) if j not in (12, 13)]
+        assert np.abs(got[:, gates] - ref[:, gates]).max() <= 1e-5
+        total = np.abs(cur[:, :5]).sum(1) + np.abs(cur[:, 5]) + np.abs(v)
+        dv = np.abs(got[:, 0] - ref[:, 0])
+        assert np.all(dv <= 1e-5 * (np.abs(ref[:, 0] - s0[:, 0]) + dt * 4 * total + np.abs(v)) + 2e-5)

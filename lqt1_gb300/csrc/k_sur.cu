@@ -59,26 +59,28 @@ __global__ void __launch_bounds__(128) k_sur_datagen(const SurCell *__restrict__
     const int cls = sur_class(ct);
     StepOut<float> o{};
     int64_t slot = -1, nrec = 0;
-    float xc[kMlpNState];   // coarse end state (hi parts) of the pending sample
-    float loc[8];           // and its concentration lo parts
+    float xc[kMlpNState] = {};   // coarse end state (hi parts) of the pending sample
+    float loc[8] = {};           // and its concentration lo parts
     float ipert = 0.f;
+    // completes the pending sample at the end of its macro step: fine minus coarse
+    auto finish = [&]() {
+        if (slot < 0) return;
+        float x1[kMlpNState];
+        state38(c, x1);
+        float2 *cp[8];
+        conc_ptrs(c, cp);
+        float *d = D + slot * kMlpNState;
+        d[0] = x1[0] - xc[0];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) d[1 + j] = (cp[j]->x - xc[1 + j]) + (cp[j]->y - loc[j]);
+#pragma unroll
+        for (int j = 9; j < kMlpNState; ++j) d[j] = x1[j] - xc[j];
+        slot = -1;
+    };
     for (int64_t st = 0; st < sc.nsteps; ++st) {
         const int64_t ph = st % sc.bcl_steps;
         if (st % nsub == 0) {
-            if (slot >= 0) {
-                // finish the pending sample: fine minus coarse
-                float x1[kMlpNState];
-                state38(c, x1);
-                float2 *cp[8];
-                conc_ptrs(c, cp);
-                float *d = D + slot * kMlpNState;
-                d[0] = x1[0] - xc[0];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) d[1 + j] = (cp[j]->x - xc[1 + j]) + (cp[j]->y - loc[j]);
-#pragma unroll
-                for (int j = 9; j < kMlpNState; ++j) d[j] = x1[j] - xc[j];
-                slot = -1;
-            }
+            finish();
             const bool stim_ahead = ph + nsub > sc.stim_on && ph < sc.stim_off;
             ipert = 0.f;
             if (st >= sc.warm_steps && !stim_ahead && fabsf(o.dvdt) <= dvdt_max && st + nsub <= sc.nsteps &&
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(128) k_sur_datagen(const SurCell *__restrict__
         const float ist = (ph >= sc.stim_on && ph < sc.stim_off) ? sc.stim : (slot >= 0 ? 0.f : ipert);
         tpord_update(c, ct, m, k, ist, 0.f, &o);
     }
+    finish();   // a sample of the cell's very last macro step
     if (counts) counts[i] = nrec;
 }
 

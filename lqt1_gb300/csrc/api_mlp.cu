@@ -15,14 +15,6 @@
 
 using namespace lqt;
 
-namespace lqt {
-cudaError_t launch_mse_grad(const float *Y, const float *T, int64_t B, int nvalid, __nv_bfloat16 *dY, double *loss,
-                            cudaStream_t st);
-cudaError_t launch_colsum(const __nv_bfloat16 *X, int64_t B, int N, float *g, cudaStream_t st);
-cudaError_t launch_adam(float *p, const float *g, float *m, float *v, __nv_bfloat16 *pb, int64_t n, float lr,
-                        float b1, float b2, float eps, float c1, float c2, cudaStream_t st);
-}  // namespace lqt
-
 namespace {
 // parameter block layout (FP32 master and BF16 copy share offsets)
 constexpr int64_t kOW1 = 0, kOB1 = kOW1 + kMlpHid * kMlpIn;
@@ -36,18 +28,16 @@ struct lqt_mlp {
     DevMem mem;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;
     __nv_bfloat16 *Pb = nullptr;
-    __nv_bfloat16 *W2t = nullptr, *W3t = nullptr;   // transposed BF16 weights for the data gradients
     float *norm = nullptr;          // in_mean[48], in_scale[48], out_scale[48], out_bound[48]
     int *err = nullptr;
     double *loss = nullptr;
     int64_t adam_t = 0;
     int nvalid = kMlpNState;
     int layout = 0;                 // descriptor stride-field assignment (0 = LBO along K)
-    // training workspace
-    int64_t ws_batch = 0;
-    float *Z1 = nullptr, *Z2 = nullptr, *Y = nullptr;
-    __nv_bfloat16 *H1 = nullptr, *H2 = nullptr, *dY = nullptr, *dZ1 = nullptr, *dZ2 = nullptr;
-    float *Gpart = nullptr;         // split-K slices of the weight gradients (ordered reduction)
+    // training workspace: gradient slices and loss sums
+    int ws_slices = 0;
+    float *Gpart = nullptr;
+    double *lossp = nullptr;
     DevMem ws;
     MlpDev dev() const
     {
@@ -78,95 +68,31 @@ static int upload_params(lqt_mlp *m, const std::vector<float> &p)
     return LQT_OK;
 }
 
-// K slices of the weight-gradient GEMMs (K = batch): 64 rows (one staging
-// chunk) each, at most 128 slices, so that the three GEMMs fill the SMs.
-static int splitk_for(int64_t B) { return (int)std::min<int64_t>(128, std::max<int64_t>(1, B / 64)); }
-
-static int ensure_ws(lqt_mlp *m, int64_t B)
+// Forward, loss gradient and backward of a batch, into the slices; then their
+// sum in m->G and, for lr > 0, the Adam step.
+static int grad_step(lqt_mlp *m, const __nv_bfloat16 *X, const float *T, int64_t B, float lr)
 {
-    if (B <= m->ws_batch) return LQT_OK;
-    m->ws.reset();
-    int rc = m->ws.alloc((void **)&m->Z1, B * kMlpHid * 4) | m->ws.alloc((void **)&m->Z2, B * kMlpHid * 4) |
-             m->ws.alloc((void **)&m->Y, B * kMlpOut * 4) | m->ws.alloc((void **)&m->H1, B * kMlpHid * 2) |
-             m->ws.alloc((void **)&m->H2, B * kMlpHid * 2) | m->ws.alloc((void **)&m->dY, B * kMlpOut * 2) |
-             m->ws.alloc((void **)&m->dZ1, B * kMlpHid * 2) | m->ws.alloc((void **)&m->dZ2, B * kMlpHid * 2) |
-             m->ws.alloc((void **)&m->Gpart,
-                         (int64_t)std::max(1, gemm_splitk_slices((int)B, splitk_for(B))) * kMlpHid * kMlpHid * 4);
-    if (rc) return LQT_ERR_NOMEM;
-    m->ws_batch = B;
-    return LQT_OK;
-}
-
-static GemmArgs gemm(const __nv_bfloat16 *A, int64_t lda, int ta, const __nv_bfloat16 *B, int64_t ldb, int tb, int M,
-                     int N, int K)
-{
-    GemmArgs g{};
-    g.A = A;
-    g.B = B;
-    g.err = nullptr;
-    g.lda = lda;
-    g.ldb = ldb;
-    g.ta = ta;
-    g.tb = tb;
-    g.M = M;
-    g.N = N;
-    g.K = K;
-    return g;
-}
-
-// Forward + MSE gradient + backward into m->G (no update).
-static int forward_backward(lqt_mlp *m, const __nv_bfloat16 *X, const float *T, int64_t B)
-{
-    // every GEMM reports a tensor-core wait that ran out in m->err (checked
-    // where the host waits: lqt_mlp_gradients, lqt_mlp_train_step with a
-    // loss, lqt_mlp_get_params)
+    // a tensor-core wait that ran out is reported in m->err (checked where the
+    // host waits: lqt_mlp_gradients, lqt_mlp_train_step with a loss)
     if (B <= 0 || B % 16 != 0 || B > (int64_t)INT32_MAX) return fail(LQT_ERR_INVALID, "batch must be a positive multiple of 16");
-    int rc = ensure_ws(m, B);
-    if (rc) return rc;
-    cudaStream_t st = m->stream;
-    const int b = (int)B;
-    const __nv_bfloat16 *W1 = m->Pb + kOW1, *W2 = m->Pb + kOW2, *W3 = m->Pb + kOW3;
-    GemmArgs g = gemm(X, kMlpIn, 0, W1, kMlpIn, 1, b, kMlpHid, kMlpIn);
-    g.epi = kEpiStore; g.bias = m->P + kOB1; g.C = m->Z1; g.Cb = m->H1; g.act = 1;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    g = gemm(m->H1, kMlpHid, 0, W2, kMlpHid, 1, b, kMlpHid, kMlpHid);
-    g.epi = kEpiStore; g.bias = m->P + kOB2; g.C = m->Z2; g.Cb = m->H2; g.act = 1;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    g = gemm(m->H2, kMlpHid, 0, W3, kMlpHid, 1, b, kMlpOut, kMlpHid);
-    g.epi = kEpiStore; g.bias = m->P + kOB3; g.C = m->Y;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    CK(cudaMemsetAsync(m->loss, 0, 8, st));
-    CK(launch_mse_grad(m->Y, T, B, m->nvalid, m->dY, m->loss, st));
-    // data gradients: W^T as N x K operands with K contiguous
-    CK(launch_transpose_w(W2, W3, m->W2t, m->W3t, st));
-    g = gemm(m->dY, kMlpOut, 0, m->W3t, kMlpOut, 1, b, kMlpHid, kMlpOut);
-    g.epi = kEpiDact; g.Z = m->Z2; g.Cb = m->dZ2;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    g = gemm(m->dZ2, kMlpHid, 0, m->W2t, kMlpHid, 1, b, kMlpHid, kMlpHid);
-    g.epi = kEpiDact; g.Z = m->Z1; g.Cb = m->dZ1;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    CK(cudaMemsetAsync(m->G, 0, kNParam * 4, st));
-    const int ks = splitk_for(B);
-    g = gemm(m->dY, kMlpOut, 1, m->H2, kMlpHid, 0, kMlpOut, kMlpHid, b);
-    g.epi = kEpiAtomic; g.C = m->G + kOW3; g.ksplit = ks; g.partial = m->Gpart;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    g = gemm(m->dZ2, kMlpHid, 1, m->H1, kMlpHid, 0, kMlpHid, kMlpHid, b);
-    g.epi = kEpiAtomic; g.C = m->G + kOW2; g.ksplit = ks; g.partial = m->Gpart;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    g = gemm(m->dZ1, kMlpHid, 1, X, kMlpIn, 0, kMlpHid, kMlpIn, b);
-    g.epi = kEpiAtomic; g.C = m->G + kOW1; g.ksplit = ks; g.partial = m->Gpart;
-    g.err = m->err;
-    CK(launch_gemm_bf16(g, st));
-    CK(launch_colsum(m->dY, B, kMlpOut, m->G + kOB3, st));
-    CK(launch_colsum(m->dZ2, B, kMlpHid, m->G + kOB2, st));
-    CK(launch_colsum(m->dZ1, B, kMlpHid, m->G + kOB1, st));
+    const int slices = mlp_grad_slices(B);
+    if (slices > m->ws_slices) {
+        m->ws.reset();
+        m->ws_slices = 0;
+        if (m->ws.alloc((void **)&m->Gpart, (size_t)slices * kNParam * 4) | m->ws.alloc((void **)&m->lossp, slices * 8))
+            return LQT_ERR_NOMEM;
+        m->ws_slices = slices;
+    }
+    const float b1 = 0.9f, b2 = 0.999f;
+    float c1 = 1.f, c2 = 1.f;
+    CK(launch_mlp_grad(X, T, B, m->nvalid, m->dev(), m->Gpart, m->lossp, m->err, m->stream));
+    if (lr > 0) {
+        m->adam_t += 1;
+        c1 = 1.f - std::pow(b1, (float)m->adam_t);
+        c2 = 1.f - std::pow(b2, (float)m->adam_t);
+    }
+    CK(launch_mlp_update(m->Gpart, m->lossp, slices, m->G, m->loss, m->P, m->M, m->V, m->Pb, lr, b1, b2, 1e-8f, c1, c2,
+                         m->stream));
     return LQT_OK;
 }
 
@@ -180,8 +106,6 @@ int lqt_mlp_create(uint64_t seed, void *stream, lqt_mlp **out)
     int rc = m->mem.alloc((void **)&m->P, kNParam * 4) | m->mem.alloc((void **)&m->G, kNParam * 4) |
              m->mem.alloc((void **)&m->M, kNParam * 4) | m->mem.alloc((void **)&m->V, kNParam * 4) |
              m->mem.alloc((void **)&m->Pb, kNParam * 2) | m->mem.alloc((void **)&m->norm, 4 * kMlpIn * 4) |
-             m->mem.alloc((void **)&m->W2t, kMlpHid * kMlpHid * 2) |
-             m->mem.alloc((void **)&m->W3t, kMlpHid * kMlpOut * 2) |
              m->mem.alloc((void **)&m->err, 16) | m->mem.alloc((void **)&m->loss, 16);
     if (rc) {
         delete m;
@@ -277,7 +201,7 @@ int lqt_mlp_infer(lqt_mlp *m, const void *x_bf16_dev, float *y_dev, int64_t n)
 int lqt_mlp_gradients(lqt_mlp *m, const void *x_bf16_dev, const float *t_dev, int64_t batch, double *loss)
 {
     if (!m || !x_bf16_dev || !t_dev) return fail(LQT_ERR_INVALID, "lqt_mlp_gradients: NULL");
-    int rc = forward_backward(m, (const __nv_bfloat16 *)x_bf16_dev, t_dev, batch);
+    int rc = grad_step(m, (const __nv_bfloat16 *)x_bf16_dev, t_dev, batch, 0.f);
     if (rc) return rc;
     double l = 0;
     int err = 0;
@@ -292,12 +216,8 @@ int lqt_mlp_gradients(lqt_mlp *m, const void *x_bf16_dev, const float *t_dev, in
 int lqt_mlp_train_step(lqt_mlp *m, const void *x_bf16_dev, const float *t_dev, int64_t batch, float lr, double *loss)
 {
     if (!m || !x_bf16_dev || !t_dev || !(lr > 0)) return fail(LQT_ERR_INVALID, "lqt_mlp_train_step: NULL or lr <= 0");
-    int rc = forward_backward(m, (const __nv_bfloat16 *)x_bf16_dev, t_dev, batch);
+    int rc = grad_step(m, (const __nv_bfloat16 *)x_bf16_dev, t_dev, batch, lr);
     if (rc) return rc;
-    m->adam_t += 1;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.f - std::pow(b1, (float)m->adam_t), c2 = 1.f - std::pow(b2, (float)m->adam_t);
-    CK(launch_adam(m->P, m->G, m->M, m->V, m->Pb, kNParam, lr, b1, b2, 1e-8f, c1, c2, m->stream));
     if (loss) {
         double l = 0;
         int err = 0;

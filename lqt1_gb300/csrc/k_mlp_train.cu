@@ -1,9 +1,24 @@
-// k_mlp_train.cu -- training kernels of the learned surrogate: a BF16
-// GEMM on the 5th-generation tensor cores (tcgen05.mma into a TMEM
-// accumulator, FP32) with the epilogues the forward and backward passes need,
-// the loss gradient and the Adam update.  Training runs once, off the
-// simulation's hot path; the per-macro-step inference uses the tcgen05 kernel
-// in k_sur_grid.cu / k_mlp_tc.cu.
+// k_mlp_train.cu -- one training step of the learned surrogate's network
+// (48 -> 128 -> 128 -> 48, SiLU, BF16 operands, FP32 accumulation) in two
+// kernels.
+//
+// k_mlp_grad: forward, loss gradient, backward and weight gradients of 128
+// batch rows per CTA without leaving the SM.  The weights (56 KB), the row
+// tile's inputs, both hidden tiles and the three gradient tiles live in shared
+// memory (208 KB), the accumulators in TMEM (480 of 512 columns).  Every tile
+// is stored once, as 8 x 8 core matrices of 8 rows x 16 bytes: read K-major it
+// is the operand of a forward or data-gradient GEMM, read MN-major (the
+// descriptor's strides exchanged, the transpose bits of the instruction set)
+// the same bytes are the transposed operand of a weight gradient, and W2 and
+// W3 those of a data gradient.  A CTA keeps its weight gradients in TMEM over
+// all of its tiles and writes one slice of them at the end.
+// k_mlp_update: adds the slices in a fixed order (the same bits on every run),
+// and applies Adam to the FP32 master weights and their BF16 copy.
+//
+// What bounds it: one tile's serial chain of five GEMMs and their epilogues
+// (a batch of 8192 is 64 tiles on 152 SMs); tensor time and traffic are below
+// 2 us.  As 17 launches that passed every tile through L2 a batch took 254 us
+// with its input preparation (GB300, 16 batches of 8192); this form takes 41.
 #include <algorithm>
 
 #include <cuda_bf16.h>
@@ -17,339 +32,468 @@ namespace lqt {
 
 namespace {
 
-constexpr int kTM = 128;                   // rows per CTA (TMEM lanes)
-constexpr int kKC = 64;                    // K per staged chunk (4 MMAs of K = 16)
-constexpr int kMaxN = 256;                 // N per CTA (one MMA)
+constexpr int kTM = 128;                   // batch rows per tile (TMEM lanes)
+constexpr int kThreads = 256;              // two warps per 32 rows: one half of the columns each
 constexpr uint32_t kWaitLimit = 1u << 24;  // bounded mbarrier polls
-// dynamic shared memory per CTA: A chunk, B chunk, mbarrier and TMEM slot;
-// padded to 60 KB so that at most 3 CTAs share an SM (3 x 128 TMEM columns
-// of the SM's 512: tcgen05.alloc never has to wait)
-constexpr uint32_t kOffA = 0;
-constexpr uint32_t kOffB = kOffA + kTM * kKC * 2;
-constexpr uint32_t kOffBar = kOffB + kMaxN * kKC * 2;
-constexpr uint32_t kSmemBytes = 60 * 1024;
-constexpr int kEpPitch = 33;               // epilogue slab row pitch (floats): no bank conflicts
-static_assert(kOffBar + 16 <= kSmemBytes, "shared memory plan");
-static_assert(kTM * kEpPitch * 4 <= kOffBar, "epilogue slab fits the staging buffers");
 
-__device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + __expf(-z)); }
+// shared-memory plan (bytes): core-matrix tiles
+constexpr uint32_t kT128 = kTM * kMlpHid * 2, kT48 = kTM * kMlpIn * 2;
+constexpr uint32_t kOffW1 = 0;                                  // [128][48]
+constexpr uint32_t kOffW2 = kOffW1 + kMlpHid * kMlpIn * 2;      // [128][128]
+constexpr uint32_t kOffW3 = kOffW2 + kMlpHid * kMlpHid * 2;     // [48][128]
+constexpr uint32_t kOffX = kOffW3 + kMlpOut * kMlpHid * 2;      // [128][48] inputs
+constexpr uint32_t kOffH1 = kOffX + kT48;                       // [128][128] hidden
+constexpr uint32_t kOffH2 = kOffH1 + kT128;
+constexpr uint32_t kOffDY = kOffH2 + kT128;                     // [128][48] output gradient
+constexpr uint32_t kOffDZ2 = kOffDY + kT48;                     // [128][128] pre-activation gradients
+constexpr uint32_t kOffDZ1 = kOffDZ2 + kT128;
+constexpr uint32_t kOffBias = kOffDZ1 + kT128;                  // b1[128], b2[128], b3[48]
+constexpr uint32_t kNBias = 2 * kMlpHid + kMlpOut;
+constexpr uint32_t kOffBar = kOffBias + kNBias * 4;
+constexpr uint32_t kSmemBytes = kOffBar + 32;
+static_assert(kMlpIn == kMlpOut, "one 48-column tile type");
+static_assert(kOffBias % 16 == 0 && kOffBar % 8 == 0 && kSmemBytes <= 227 * 1024, "shared memory");
 
-// K per slice of a split-K GEMM: whole staging chunks.
-__host__ __device__ inline int splitk_chunk(int K, int ksplit)
+// TMEM columns: pre-activation 1; pre-activation 2, then the outputs, then
+// the two data gradients; the weight gradients
+constexpr uint32_t kColZ1 = 0, kColWork = 128, kColG2 = 256, kColG3 = 384, kColG1 = 432, kTmemCols = 512;
+
+// Slice layout (floats): the parameter block's order W1 b1 W2 b2 W3 b3
+constexpr int kOW1 = 0, kOB1 = kOW1 + kMlpHid * kMlpIn, kOW2 = kOB1 + kMlpHid, kOB2 = kOW2 + kMlpHid * kMlpHid,
+              kOW3 = kOB2 + kMlpHid, kOB3 = kOW3 + kMlpOut * kMlpHid, kNP = kOB3 + kMlpOut;
+static_assert(kNP == kMlpNParam32, "parameter block");
+
+// 1 / (1 + exp(-z)): the hardware reciprocal with one Newton step on its exact
+// residual (an FMA), which is the correctly rounded quotient but for about one
+// argument in a million; exp(-z) is held at 1e30, where the result is 0 beside
+// anything it is added to.
+__device__ __forceinline__ float sigm(float z)
 {
-    return ((K + ksplit - 1) / ksplit + kKC - 1) / kKC * kKC;
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
+    const float d = 1.0f + fminf(e, 1e30f);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(fmaf(-d, r, 1.0f), r, r);
 }
 
-// C[o] += the split-K slices of element o, added in slice order.
-__global__ void k_splitk_reduce(const float *__restrict__ partial, int64_t mn, int slices, float *__restrict__ C)
+// Copy `rows` valid rows of a row-major [R][K] BF16 matrix into core matrices, zeros below them.
+__device__ __forceinline__ void stage_tile(uint8_t *dst, const __nv_bfloat16 *src, int R, int K, int rows)
 {
-    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < mn; o += (int64_t)gridDim.x * blockDim.x) {
-        // unrolled: the slices' loads are issued together, the additions
-        // stay in slice order
-        float acc = 0.f;
-#pragma unroll 16
-        for (int z = 0; z < slices; ++z) acc += partial[(int64_t)z * mn + o];
-        C[o] += acc;
+    for (int c = threadIdx.x; c < R * (K / 8); c += kThreads) {
+        const int r = c / (K / 8), kg = c % (K / 8);
+        *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(r, kg * 8, K)) =
+            r < rows ? *reinterpret_cast<const uint4 *>(src + (int64_t)r * K + kg * 8) : make_uint4(0, 0, 0, 0);
     }
 }
 
-// One 8-element K chunk of row r of op(X) (X[r][k] = ta ? src[k * ld + r] :
-// src[r * ld + k]) for k = k0 .. k0 + 7, zero outside rows < R and k < kend.
-__device__ __forceinline__ uint4 load_chunk8(const __nv_bfloat16 *src, int64_t ld, int t, int r, int R, int k0,
-                                             int kend)
+// An operand tile of F features: read K-major (rows = M or N, features = K)
+// or MN-major (features = M or N, rows = K).  Per MMA K advances by 16.
+struct Operand {
+    uint32_t addr, lbo, sbo, step;
+};
+__device__ __forceinline__ Operand kmajor(const uint8_t *p, int F)
 {
-    if (r >= R) return make_uint4(0, 0, 0, 0);
-    if (!t && k0 + 8 <= kend && (ld & 7) == 0 && (k0 & 7) == 0)
-        return *reinterpret_cast<const uint4 *>(src + (int64_t)r * ld + k0);
-    uint32_t p[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint16_t h[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int k = k0 + 2 * i + j;
-            __nv_bfloat16 v = __float2bfloat16(0.0f);
-            if (k < kend) v = t ? src[(int64_t)k * ld + r] : src[(int64_t)r * ld + k];
-            h[j] = __bfloat16_as_ushort(v);
-        }
-        p[i] = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
-    }
-    return make_uint4(p[0], p[1], p[2], p[3]);
+    return Operand{tc::smem_u32(p), 128u, (uint32_t)(F / 8) * 128u, 256u};
+}
+__device__ __forceinline__ Operand mnmajor(const uint8_t *p, int F)
+{
+    const uint32_t row8 = (uint32_t)(F / 8) * 128u;     // next 8 rows
+    return Operand{tc::smem_u32(p), row8, 128u, 2u * row8};
+}
+// D[128 x N] (+)= A B^T over K; at, bt = operand MN-major.
+__device__ __forceinline__ void mma_all(uint32_t d, const Operand &a, bool at, const Operand &b, bool bt, int N, int K,
+                                        bool accum)
+{
+    const uint32_t id = tc::idesc_bf16_f32(128, N) | (at ? 1u << 15 : 0u) | (bt ? 1u << 16 : 0u);
+    for (int k = 0; k < K / 16; ++k)
+        tc::mma_bf16(d, tc::smem_desc(a.addr + k * a.step, a.lbo, a.sbo), tc::smem_desc(b.addr + k * b.step, b.lbo, b.sbo),
+                     id, (accum || k > 0) ? 1u : 0u);
 }
 
-// C[M][N] (epilogue) = op(A)[M][K] * op(B)[K][N].  One CTA of 128 threads per
-// 128-row tile and (for the split weight gradients) K range: the tile's A rows
-// and all N rows of op(B)^T are staged chunk by chunk in the K-major core
-// layout; one elected thread issues the MMAs and commits to an mbarrier; the
-// accumulator (row m in TMEM lane m) goes through the epilogue by its thread.
-__global__ void __launch_bounds__(128) k_gemm_tc(GemmArgs g)
+// Sum over the tile's 128 rows of two neighbouring columns of a BF16 tile of
+// F features, this thread's share of the rows: [row0, row0 + 128 / parts).
+// The lanes of a warp start at different rows, so that their reads fall into
+// different banks.
+__device__ __forceinline__ float2 column_sums(const uint8_t *tile, int F, int col, int row0, int nrows)
 {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kOffBar);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kOffBar + 8);
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int m0 = blockIdx.y * kTM;
-    const int npad = (g.N + 15) / 16 * 16;
-    uint32_t ncols = 32;
-    while ((int)ncols < npad) ncols <<= 1;
-    int kbeg = 0, kend = g.K;
-    if (g.epi == kEpiAtomic && g.ksplit > 1) {
-        const int chunk = splitk_chunk(g.K, g.ksplit);
-        kbeg = blockIdx.z * chunk;
-        kend = min(g.K, kbeg + chunk);
-    }
-    // this CTA's slice of a split-K GEMM with a workspace: plain stores
-    float *const slab = (g.epi == kEpiAtomic && g.partial) ? g.partial + (int64_t)blockIdx.z * g.M * g.N : nullptr;
-    if (tid == 0) {
-        tc::mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) tc::tmem_alloc(tslot, ncols);
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = *tslot;
-    const uint32_t idesc = tc::idesc_bf16_f32(kTM, npad);
-    uint32_t phase = 0;
-    bool ok = true;
-    int nchunk = 0;
-    for (int k0 = kbeg; k0 < kend && ok; k0 += kKC, ++nchunk) {
-        // stage: consecutive threads take consecutive rows (coalesced for the
-        // transposed operands, whose rows are contiguous in memory)
-        for (int c = tid; c < kTM * (kKC / 8); c += 128) {
-            const int r = c % kTM, kg = c / kTM;
-            *reinterpret_cast<uint4 *>(smem + kOffA + tc::kmaj_off(r, kg * 8, kKC)) =
-                load_chunk8(g.A, g.lda, g.ta, m0 + r, g.M, k0 + kg * 8, kend);
-        }
-        for (int c = tid; c < npad * (kKC / 8); c += 128) {
-            const int r = c % npad, kg = c / npad;
-            // op(B)^T row n: B[n][k] when stored transposed (tb), else B[k][n]
-            *reinterpret_cast<uint4 *>(smem + kOffB + tc::kmaj_off(r, kg * 8, kKC)) =
-                load_chunk8(g.B, g.ldb, !g.tb, r, g.N, k0 + kg * 8, kend);
-        }
-        tc::fence_proxy_async();
-        tc::fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc::fence_after();
-            const uint32_t lbo = 128, sbo = (kKC / 8) * 128;
-            const uint32_t a0 = tc::smem_u32(smem + kOffA), b0 = tc::smem_u32(smem + kOffB);
-            for (int kk = 0; kk < kKC / 16; ++kk)
-                tc::mma_bf16(tmem, tc::smem_desc(a0 + kk * 256, lbo, sbo), tc::smem_desc(b0 + kk * 256, lbo, sbo),
-                             idesc, (nchunk > 0 || kk > 0) ? 1u : 0u);
-            tc::mma_commit(bar);
-        }
-        // the chunk's smem is reused only after its MMAs completed; the
-        // decision is made for the whole CTA at once
-        const bool w_ok = tc::mbar_wait(bar, phase, kWaitLimit);
-        if (!__syncthreads_and(w_ok ? 1 : 0)) {
-            if (!w_ok) tc::mbar_wait(bar, phase, kWaitLimit);   // let the MMAs in flight land before TMEM is freed
-            if (tid == 0 && g.err) atomicExch(g.err, 2);
-            ok = false;
-        }
-        phase ^= 1;
-        tc::fence_after();
-        __syncthreads();
-    }
-    if (ok && nchunk > 0) {
-        // epilogue in 32-column slabs: each thread moves its row (TMEM lane)
-        // into shared memory, then every warp writes whole row segments, so
-        // the stores (or atomics) of a warp are 32 consecutive elements
-        float *ep = reinterpret_cast<float *>(smem);          // the staging buffers are free now
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-        const int lane = tid & 31;
-        for (int n0 = 0; n0 < g.N; n0 += 32) {
-            float v[32];
-            tc::tmem_ld32(taddr + n0, v);                     // whole warp
-#pragma unroll
-            for (int i = 0; i < 32; ++i) ep[tid * kEpPitch + i] = v[i];
-            __syncthreads();
-            // a warp takes rows warp, warp + 4, ...: the loop is unrolled and
-            // the pointers restrict-qualified, so that its global loads (the
-            // bias once, Z of every row) are issued together instead of one
-            // latency per row behind the previous row's stores
-            const int n = n0 + lane;
-            const bool nin = n < g.N;
-            const float *__restrict__ Zp = g.Z;
-            float *__restrict__ Cp = g.C;
-            __nv_bfloat16 *__restrict__ Cbp = g.Cb;
-            constexpr int kRows = kTM / 4;
-            if (g.epi == kEpiDact) {
-                float zv[kRows];
-#pragma unroll
-                for (int i = 0; i < kRows; ++i) {
-                    const int m = m0 + warp + 4 * i;
-                    zv[i] = (nin && m < g.M) ? Zp[(int64_t)m * g.N + n] : 0.f;
-                }
-#pragma unroll
-                for (int i = 0; i < kRows; ++i) {
-                    const int r = warp + 4 * i, m = m0 + r;
-                    if (!nin || m >= g.M) continue;
-                    const float x = ep[r * kEpPitch + lane], z = zv[i], sz = sigm(z);
-                    Cbp[(int64_t)m * g.N + n] = __float2bfloat16(x * (sz + z * sz * (1.0f - sz)));
-                }
-            } else if (g.epi == kEpiStore) {
-                const float bn = (nin && g.bias) ? g.bias[n] : 0.f;
+    float2 s = make_float2(0.f, 0.f);
+    const int turn = (col >> 3) & 7;
 #pragma unroll 8
-                for (int i = 0; i < kRows; ++i) {
-                    const int r = warp + 4 * i, m = m0 + r;
-                    if (!nin || m >= g.M) continue;
-                    const int64_t o = (int64_t)m * g.N + n;
-                    const float x = ep[r * kEpPitch + lane] + bn;
-                    if (Cp) Cp[o] = x;
-                    if (Cbp) Cbp[o] = __float2bfloat16(g.act ? x * sigm(x) : x);
-                }
-            } else {
-#pragma unroll 8
-                for (int i = 0; i < kRows; ++i) {
-                    const int r = warp + 4 * i, m = m0 + r;
-                    if (!nin || m >= g.M) continue;
-                    const int64_t o = (int64_t)m * g.N + n;
-                    const float x = ep[r * kEpPitch + lane];
-                    if (slab) slab[o] = x;
-                    else atomicAdd(&Cp[o], x);
-                }
-            }
-            __syncthreads();
-        }
+    for (int r = 0; r < nrows; ++r) {
+        const int row = row0 + (r & ~7) + ((r + turn) & 7);
+        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(tile + tc::kmaj_off(row, col, F)));
+        s.x += v.x;
+        s.y += v.y;
     }
-    tc::fence_before();
-    __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem, ncols);
+    return s;
+}
+
+__device__ __forceinline__ uint32_t pack2(float a, float b)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t *>(&h);
 }
 
 }  // namespace
 
-cudaError_t launch_gemm_bf16(const GemmArgs &g, cudaStream_t st)
+// part: [gridDim.x][kNP] gradient slices; lossp: [gridDim.x] sums of squared
+// errors over the valid outputs.  dY = 2 (Y - T) / (B nvalid).
+__global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *__restrict__ X,
+                                                          const float *__restrict__ T, int64_t B, int nvalid,
+                                                          MlpDev w, float *__restrict__ part,
+                                                          double *__restrict__ lossp, int *err)
 {
-    if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaSuccess;
-    if (g.N > kMaxN) return cudaErrorInvalidValue;
-    static std::atomic<uint64_t> attr_done{0};
-    cudaError_t e = tc::smem_attr_once(k_gemm_tc, kSmemBytes, attr_done);
-    if (e != cudaSuccess) return e;
-    const int slices = gemm_splitk_slices(g.K, g.epi == kEpiAtomic ? g.ksplit : 1);
-    dim3 grid(1, (g.M + kTM - 1) / kTM, slices > 0 ? slices : 1);
-    k_gemm_tc<<<grid, 128, kSmemBytes, st>>>(g);
-    e = cudaGetLastError();
-    if (e == cudaSuccess && slices > 0 && g.partial) {
-        const int64_t mn = (int64_t)g.M * g.N;
-        k_splitk_reduce<<<(unsigned)std::min<int64_t>((mn + 255) / 256, 1024), 256, 0, st>>>(g.partial, mn, slices,
-                                                                                            g.C);
-        e = cudaGetLastError();
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ double lred[kThreads / 32];
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kOffBar);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kOffBar + 8);
+    float *bias = reinterpret_cast<float *>(smem + kOffBias);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int half = warp >> 2;                        // columns [64 half, 64 half + 64) of the hidden tiles
+    const int row = (warp & 3) * 32 + lane;            // row of the tile = TMEM lane
+    const int c0 = half * 64;
+
+    stage_tile(smem + kOffW1, w.w1t, kMlpHid, kMlpIn, kMlpHid);
+    stage_tile(smem + kOffW2, w.w2t, kMlpHid, kMlpHid, kMlpHid);
+    stage_tile(smem + kOffW3, w.w3t, kMlpOut, kMlpHid, kMlpOut);
+    for (int i = tid; i < (int)kNBias; i += kThreads)
+        bias[i] = i < kMlpHid ? w.b1[i] : (i < 2 * kMlpHid ? w.b2[i - kMlpHid] : w.b3[i - 2 * kMlpHid]);
+    if (tid == 0) {
+        tc::mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    return e;
-}
+    if (warp == 0) tc::tmem_alloc(tslot, kTmemCols);
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tm = *tslot;
+    const uint32_t tl = tm + ((uint32_t)((warp & 3) * 32) << 16);   // this warp's TMEM lanes
+    const float scale = 2.0f / (float)(B * nvalid);
+    const bool wide = (reinterpret_cast<uintptr_t>(T) & 15) == 0;   // target rows readable 16 bytes at a time
+    uint32_t phase = 0;
+    bool ok = true, first = true;
+    float lhi = 0.f, llo = 0.f;                        // this thread's squared errors, a compensated pair
+    // bias gradients: two columns and a share of the rows per thread
+    float2 g1 = make_float2(0.f, 0.f), g2 = g1, g3 = g1;
+    const int bc = (tid & 63) * 2, br = (tid >> 6) * 32;            // hidden: 64 pairs x 4 shares of 32 rows
+    const int oc = (tid % 24) * 2, orow = (tid / 24) * 16;          // outputs: 24 pairs x 8 shares of 16 rows (192 threads)
 
-// Only slices that hold at least one chunk of K are launched, so every slice
-// of the workspace is written before the reduction reads it.
-int gemm_splitk_slices(int K, int ksplit)
-{
-    if (ksplit <= 1 || K <= 0) return 0;
-    const int chunk = splitk_chunk(K, ksplit);
-    return (K + chunk - 1) / chunk;
-}
+    // writes before it are visible to the MMAs, TMEM reads before it are done
+    auto publish = [&]() {
+        tc::fence_proxy_async();
+        tc::fence_before();
+        __syncthreads();
+    };
+    // the MMAs committed so far are complete; the CTA takes one decision
+    auto arrived = [&]() -> bool {
+        const bool w_ok = tc::mbar_wait(bar, phase, kWaitLimit);
+        if (!__syncthreads_and(w_ok ? 1 : 0)) {
+            if (!w_ok) tc::mbar_wait(bar, phase, kWaitLimit);       // let the MMAs in flight land before TMEM is freed
+            if (tid == 0 && err) atomicExch(err, 2);
+            return false;
+        }
+        phase ^= 1;
+        tc::fence_after();
+        return true;
+    };
+    // hidden layer: pre-activations in z, SiLU to the operand tile
+    auto hidden = [&](uint32_t col, const float *b, uint8_t *dst, float *z) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            tc::tmem_ld32(tl + col + c0 + 32 * q, z + 32 * q);
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+                uint32_t p[4];
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    const int k = 32 * q + i + j;
+                    z[k] += b[c0 + k];
+                    z[k + 1] += b[c0 + k + 1];
+                    p[j / 2] = pack2(z[k] * sigm(z[k]), z[k + 1] * sigm(z[k + 1]));
+                }
+                *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + 32 * q + i, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
+            }
+        }
+    };
+    // pre-activation gradient: the work columns times SiLU'(z)
+    auto dact = [&](const float *z, uint8_t *dst) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            float v[32];
+            tc::tmem_ld32(tl + kColWork + c0 + 32 * q, v);
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+                uint32_t p[4];
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    float d[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float zz = z[32 * q + i + j + u], sz = sigm(zz);
+                        d[u] = v[i + j + u] * (sz + zz * sz * (1.0f - sz));
+                    }
+                    p[j / 2] = pack2(d[0], d[1]);
+                }
+                *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + 32 * q + i, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
+            }
+        }
+    };
 
-// dst[c][r] = src[r][c] for the hidden and output weights (BF16): the
-// backward pass's data-gradient GEMMs read W as an N x K operand with K
-// contiguous, which the staging then copies with 16-byte loads.
-__global__ void k_transpose_w(const __nv_bfloat16 *__restrict__ w2, const __nv_bfloat16 *__restrict__ w3,
-                              __nv_bfloat16 *__restrict__ w2t, __nv_bfloat16 *__restrict__ w3t)
-{
-    const int n2 = kMlpHid * kMlpHid, n3 = kMlpOut * kMlpHid;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n2 + n3; i += gridDim.x * blockDim.x) {
-        if (i < n2) {
-            const int r = i / kMlpHid, c = i - r * kMlpHid;
-            w2t[c * kMlpHid + r] = w2[i];
+    const int64_t ntiles = (B + kTM - 1) / kTM;
+    for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        const int64_t m0 = tile * kTM;
+        const int rows = (int)(B - m0 < kTM ? B - m0 : kTM);
+        const bool live = row < rows;
+        stage_tile(smem + kOffX, X + m0 * kMlpIn, kTM, kMlpIn, rows);
+        // this thread's targets: outputs 0..31 (first half) or 32..47
+        float tg[32];
+        const float *trow = T + (m0 + row) * kMlpOut + 32 * half;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (live && 32 * half + j < kMlpOut)
+                q = wide ? __ldg(reinterpret_cast<const float4 *>(trow + j)) : make_float4(trow[j], trow[j + 1], trow[j + 2], trow[j + 3]);
+            tg[j] = q.x;
+            tg[j + 1] = q.y;
+            tg[j + 2] = q.z;
+            tg[j + 3] = q.w;
+        }
+        publish();
+        if (tid == 0) {
+            tc::fence_after();
+            mma_all(tm + kColZ1, kmajor(smem + kOffX, kMlpIn), false, kmajor(smem + kOffW1, kMlpIn), false, kMlpHid, kMlpIn, false);
+            tc::mma_commit(bar);
+        }
+        if (!(ok = arrived())) break;
+        float z[64];
+        hidden(kColZ1, bias, smem + kOffH1, z);
+        publish();
+        if (tid == 0) {
+            tc::fence_after();
+            mma_all(tm + kColWork, kmajor(smem + kOffH1, kMlpHid), false, kmajor(smem + kOffW2, kMlpHid), false, kMlpHid, kMlpHid, false);
+            tc::mma_commit(bar);
+        }
+        if (!(ok = arrived())) break;
+        hidden(kColWork, bias + kMlpHid, smem + kOffH2, z);        // z: pre-activation 2 from here on
+        publish();
+        if (tid == 0) {
+            tc::fence_after();
+            mma_all(tm + kColWork, kmajor(smem + kOffH2, kMlpHid), false, kmajor(smem + kOffW3, kMlpHid), false, kMlpOut, kMlpHid, false);
+            tc::mma_commit(bar);
+        }
+        if (!(ok = arrived())) break;
+        // outputs: loss and its gradient
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (32 * half + 16 * q >= kMlpOut) break;              // (uniform in a warp)
+            const int o = 32 * half + 16 * q;
+            float y[16];
+            tc::tmem_ld16(tl + kColWork + o, y);
+#pragma unroll
+            for (int i = 0; i < 16; i += 8) {
+                uint32_t p[4];
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    float g[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int c = o + i + j + u;
+                        float d = (y[i + j + u] + bias[2 * kMlpHid + c]) - tg[16 * q + i + j + u];
+                        if (c >= nvalid || !live) d = 0.f;
+                        g[u] = scale * d;
+                        // (lhi, llo) += d^2: the square's rounding error by an FMA, the sum's by TwoSum
+                        const float sq = __fmul_rn(d, d), se = fmaf(d, d, -sq);
+                        const float s = __fadd_rn(lhi, sq), bb = __fsub_rn(s, lhi);
+                        llo += __fadd_rn(__fsub_rn(lhi, __fsub_rn(s, bb)), __fsub_rn(sq, bb)) + se;
+                        lhi = s;
+                    }
+                    p[j / 2] = pack2(g[0], g[1]);
+                }
+                *reinterpret_cast<uint4 *>(smem + kOffDY + tc::kmaj_off(row, o + i, kMlpOut)) = make_uint4(p[0], p[1], p[2], p[3]);
+            }
+        }
+        publish();
+        if (tid == 0) {
+            tc::fence_after();
+            mma_all(tm + kColWork, kmajor(smem + kOffDY, kMlpOut), false, mnmajor(smem + kOffW3, kMlpHid), true, kMlpHid, kMlpOut, false);
+            tc::mma_commit(bar);
+            // W3 gradient, transposed: [hidden][output]
+            mma_all(tm + kColG3, mnmajor(smem + kOffH2, kMlpHid), true, mnmajor(smem + kOffDY, kMlpOut), true, kMlpOut, kTM, !first);
+        }
+        if (tid < 192) {
+            const float2 s = column_sums(smem + kOffDY, kMlpOut, oc, orow, 16);
+            g3.x += s.x;
+            g3.y += s.y;
+        }
+        if (!(ok = arrived())) break;
+        dact(z, smem + kOffDZ2);
+        publish();
+        if (tid == 0) {
+            tc::fence_after();
+            mma_all(tm + kColWork, kmajor(smem + kOffDZ2, kMlpHid), false, mnmajor(smem + kOffW2, kMlpHid), true, kMlpHid, kMlpHid, false);
+            tc::mma_commit(bar);
+            // W2 gradient, transposed: [in][out]
+            mma_all(tm + kColG2, mnmajor(smem + kOffH1, kMlpHid), true, mnmajor(smem + kOffDZ2, kMlpHid), true, kMlpHid, kTM, !first);
+        }
+        {
+            const float2 s = column_sums(smem + kOffDZ2, kMlpHid, bc, br, 32);
+            g2.x += s.x;
+            g2.y += s.y;
+        }
+        if (!(ok = arrived())) break;
+        // pre-activation 1 is still in its columns
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            tc::tmem_ld32(tl + kColZ1 + c0 + 32 * q, z + 32 * q);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) z[32 * q + i] += bias[c0 + 32 * q + i];
+        }
+        dact(z, smem + kOffDZ1);
+        publish();
+        if (tid == 0) {
+            tc::fence_after();
+            // W1 gradient: [out][in]
+            mma_all(tm + kColG1, mnmajor(smem + kOffDZ1, kMlpHid), true, mnmajor(smem + kOffX, kMlpIn), true, kMlpIn, kTM, !first);
+            tc::mma_commit(bar);
+        }
+        {
+            const float2 s = column_sums(smem + kOffDZ1, kMlpHid, bc, br, 32);
+            g1.x += s.x;
+            g1.y += s.y;
+        }
+        if (!(ok = arrived())) break;               // and with it every earlier MMA: the tiles may be overwritten
+        first = false;
+    }
+    if (ok) {
+        float *out = part + (int64_t)blockIdx.x * kNP;
+        float v[32];
+        // [in][out] accumulators: a warp writes 32 neighbouring inputs of one output
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            tc::tmem_ld32(tl + kColG2 + c0 + 32 * q, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) out[kOW2 + (c0 + 32 * q + i) * kMlpHid + row] = v[i];
+        }
+        // 48 columns: 0..31 by the first half's warps, 32..47 by the second's
+        if (half == 0) {
+            tc::tmem_ld32(tl + kColG3, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) out[kOW3 + i * kMlpHid + row] = v[i];
+            tc::tmem_ld32(tl + kColG1, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) out[kOW1 + row * kMlpIn + i] = v[i];
         } else {
-            const int j = i - n2, r = j / kMlpHid, c = j - r * kMlpHid;
-            w3t[c * kMlpOut + r] = w3[j];
+            tc::tmem_ld16(tl + kColG3 + 32, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) out[kOW3 + (32 + i) * kMlpHid + row] = v[i];
+            tc::tmem_ld16(tl + kColG1 + 32, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) out[kOW1 + row * kMlpIn + 32 + i] = v[i];
         }
-    }
-}
-
-// ---- loss gradient and Adam -------------------------------------------------
-// dY = 2 (Y - T) mask / (B * nvalid); loss += sum (Y - T)^2 mask (FP64 atomics per block).
-__global__ void k_mse_grad(const float *__restrict__ Y, const float *__restrict__ T, int64_t B, int nvalid,
-                           __nv_bfloat16 *__restrict__ dY, double *__restrict__ loss)
-{
-    __shared__ double red[256];
-    double acc = 0.0;
-    const float s = 2.0f / (float)(B * nvalid);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < B * kMlpOut;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int c = (int)(i % kMlpOut);
-        float d = 0.0f;
-        if (c < nvalid) {
-            d = Y[i] - T[i];
-            acc += (double)d * d;
+        // bias gradients: the rows' shares added in order
+        float *cs = reinterpret_cast<float *>(smem + kOffDZ2);          // the tiles are free now
+        cs[(tid >> 6) * 128 + bc] = g1.x;
+        cs[(tid >> 6) * 128 + bc + 1] = g1.y;
+        cs[512 + (tid >> 6) * 128 + bc] = g2.x;
+        cs[512 + (tid >> 6) * 128 + bc + 1] = g2.y;
+        if (tid < 192) {
+            cs[1024 + (tid / 24) * 48 + oc] = g3.x;
+            cs[1024 + (tid / 24) * 48 + oc + 1] = g3.y;
         }
-        dY[i] = __float2bfloat16(s * d);
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        double l = (double)lhi + (double)llo;
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+        if (lane == 0) lred[warp] = l;
         __syncthreads();
+        if (tid < 128) {
+            out[kOB1 + tid] = ((cs[tid] + cs[128 + tid]) + cs[256 + tid]) + cs[384 + tid];
+            out[kOB2 + tid] = ((cs[512 + tid] + cs[640 + tid]) + cs[768 + tid]) + cs[896 + tid];
+        } else if (tid < 128 + kMlpOut) {
+            float s = 0.f;
+            for (int q = 0; q < 8; ++q) s += cs[1024 + q * 48 + tid - 128];
+            out[kOB3 + tid - 128] = s;
+        } else if (tid == 255) {
+            double s = 0.0;
+            for (int q = 0; q < kThreads / 32; ++q) s += lred[q];
+            lossp[blockIdx.x] = s;
+        }
     }
-    if (threadIdx.x == 0) atomicAdd(loss, red[0]);
+    tc::fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tm, kTmemCols);
 }
 
-// Column sums of a BF16 [B][N] matrix into FP32 g[N] (bias gradients).
-__global__ void k_colsum(const __nv_bfloat16 *__restrict__ X, int64_t B, int N, float *__restrict__ g)
+// G[i] = the slices of parameter i added in slice order (four runs of slices,
+// then the four sums in order); with lr > 0 one Adam step with bias correction
+// c1, c2 on the FP32 master weights and their BF16 copy.  loss = sum of lossp.
+__global__ void __launch_bounds__(256) k_mlp_update(const float *__restrict__ part, const double *__restrict__ lossp,
+                                                    int slices, float *__restrict__ g, double *__restrict__ loss,
+                                                    float *__restrict__ p, float *__restrict__ m, float *__restrict__ v,
+                                                    __nv_bfloat16 *__restrict__ pb, float lr, float b1, float b2,
+                                                    float eps, float c1, float c2)
 {
-    const int n = blockIdx.x;
+    __shared__ float red[4][64];
+    const int q = threadIdx.x >> 6, j = threadIdx.x & 63;
+    const int i = blockIdx.x * 64 + j;
+    const int s0 = q * slices / 4, s1 = (q + 1) * slices / 4;
     float acc = 0.f;
-    for (int64_t r = threadIdx.x; r < B; r += blockDim.x) acc += __bfloat162float(X[r * N + n]);
-    __shared__ float red[256];
-    red[threadIdx.x] = acc;
+    if (i < kNP) {
+#pragma unroll 16
+        for (int s = s0; s < s1; ++s) acc += part[(int64_t)s * kNP + i];
+    }
+    red[q][j] = acc;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
+    if (q == 0 && i < kNP) {
+        const float gi = ((red[0][j] + red[1][j]) + red[2][j]) + red[3][j];
+        g[i] = gi;
+        if (lr > 0.f) {
+            const float mi = b1 * m[i] + (1.f - b1) * gi;
+            const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+            m[i] = mi;
+            v[i] = vi;
+            const float pn = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+            p[i] = pn;
+            pb[i] = __float2bfloat16(pn);
+        }
     }
-    if (threadIdx.x == 0) g[n] = red[0];
-}
-
-// Adam with bias correction; master weights FP32, a BF16 copy for the kernels.
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-                       __nv_bfloat16 *__restrict__ pb, int64_t n, float lr, float b1, float b2, float eps, float c1,
-                       float c2)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float pn = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        p[i] = pn;
-        if (pb) pb[i] = __float2bfloat16(pn);
+    if (blockIdx.x == 0 && threadIdx.x == 64) {
+        double s = 0.0;
+        for (int k = 0; k < slices; ++k) s += lossp[k];
+        *loss = s;
     }
 }
 
-cudaError_t launch_mse_grad(const float *Y, const float *T, int64_t B, int nvalid, __nv_bfloat16 *dY, double *loss,
-                            cudaStream_t st)
+static int device_sms()
 {
-    k_mse_grad<<<256, 256, 0, st>>>(Y, T, B, nvalid, dY, loss);
-    return cudaGetLastError();
+    int dev = 0, nsm = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
 }
-cudaError_t launch_colsum(const __nv_bfloat16 *X, int64_t B, int N, float *g, cudaStream_t st)
+
+// One CTA per SM at most (208 KB of shared memory and all of TMEM, so
+// tcgen05.alloc never waits), one tile per CTA while the batch allows it.
+int mlp_grad_slices(int64_t B)
 {
-    k_colsum<<<N, 256, 0, st>>>(X, B, N, g);
-    return cudaGetLastError();
+    const int64_t tiles = (B + kTM - 1) / kTM;
+    return (int)std::min<int64_t>(tiles, device_sms());
 }
-cudaError_t launch_transpose_w(const __nv_bfloat16 *w2, const __nv_bfloat16 *w3, __nv_bfloat16 *w2t,
-                               __nv_bfloat16 *w3t, cudaStream_t st)
+
+cudaError_t launch_mlp_grad(const __nv_bfloat16 *X, const float *T, int64_t B, int nvalid, const MlpDev &w, float *part,
+                            double *lossp, int *err, cudaStream_t st)
 {
-    k_transpose_w<<<(kMlpHid * (kMlpHid + kMlpOut) + 255) / 256, 256, 0, st>>>(w2, w3, w2t, w3t);
+    if (B <= 0) return cudaSuccess;
+    static std::atomic<uint64_t> attr_done{0};
+    cudaError_t e = tc::smem_attr_once(k_mlp_grad, kSmemBytes, attr_done);
+    if (e != cudaSuccess) return e;
+    k_mlp_grad<<<(unsigned)mlp_grad_slices(B), kThreads, kSmemBytes, st>>>(X, T, B, nvalid, w, part, lossp, err);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adam(float *p, const float *g, float *m, float *v, __nv_bfloat16 *pb, int64_t n, float lr,
-                        float b1, float b2, float eps, float c1, float c2, cudaStream_t st)
+cudaError_t launch_mlp_update(const float *part, const double *lossp, int slices, float *g, double *loss, float *p,
+                              float *m, float *v, __nv_bfloat16 *pb, float lr, float b1, float b2, float eps, float c1,
+                              float c2, cudaStream_t st)
 {
-    const int64_t nb = (n + 255) / 256;
-    k_adam<<<(unsigned)(nb > 1024 ? 1024 : nb), 256, 0, st>>>(p, g, m, v, pb, n, lr, b1, b2, eps, c1, c2);
+    k_mlp_update<<<(kNP + 63) / 64, 256, 0, st>>>(part, lossp, slices, g, loss, p, m, v, pb, lr, b1, b2, eps, c1, c2);
     return cudaGetLastError();
 }
 

@@ -32,31 +32,15 @@ bool mlp_device_view(const lqt_mlp *m, MlpDev *w, const float **norm);
 cudaError_t launch_mlp_infer_tc(const __nv_bfloat16 *X, float *Y, const MlpDev &w, int64_t n, int *err, int swap,
                                 cudaStream_t st);
 
-// C[M][N] (op) = op(A)[M][K] * op(B)[K][N]; A, B BF16 row-major with the
-// given leading dimensions; TA/TB = operand stored transposed.
-enum { kEpiStore = 0, kEpiDact = 1, kEpiAtomic = 2 };
-struct GemmArgs {
-    const __nv_bfloat16 *A, *B;
-    int64_t lda, ldb;
-    int ta, tb;
-    int M, N, K;
-    int epi;
-    const float *bias;           // kEpiStore: + bias[n]
-    float *C;                    // kEpiStore / kEpiAtomic: FP32 out [M][N]
-    __nv_bfloat16 *Cb;           // kEpiStore: BF16 of act(C); kEpiDact: BF16 of acc * silu'(Z)
-    int act;                     // kEpiStore: 1 = SiLU for Cb
-    const float *Z;              // kEpiDact: pre-activation [M][N]
-    int ksplit;                  // kEpiAtomic: split K over grid.z
-    int *err;                    // set to 2 if a tensor-core completion wait ran out (or NULL)
-    float *partial;              // kEpiAtomic with ksplit > 1: [slices][M][N] workspace; the slices
-                                 // are then added into C in slice order (same bits every run);
-                                 // NULL = float atomics into C (order-dependent last bits)
-};
-// Slices of a split-K GEMM and the workspace floats it needs (0 without a split).
-int gemm_splitk_slices(int K, int ksplit);
-cudaError_t launch_gemm_bf16(const GemmArgs &g, cudaStream_t st);
-// W2^T [in][out] and W3^T [in][out] from W2 [out][in], W3 [out][in] (BF16).
-cudaError_t launch_transpose_w(const __nv_bfloat16 *w2, const __nv_bfloat16 *w3, __nv_bfloat16 *w2t,
-                               __nv_bfloat16 *w3t, cudaStream_t st);
+// Training (k_mlp_train.cu): gradient slices of a batch, one per CTA
+// (mlp_grad_slices of them, kMlpNParam32 floats each, and one loss sum each),
+// and their ordered sum with, for lr > 0, one Adam step.
+constexpr int kMlpNParam32 = 2 * kMlpIn * kMlpHid + kMlpHid * kMlpHid + 2 * kMlpHid + kMlpOut;
+int mlp_grad_slices(int64_t B);
+cudaError_t launch_mlp_grad(const __nv_bfloat16 *X, const float *T, int64_t B, int nvalid, const MlpDev &w, float *part,
+                            double *lossp, int *err, cudaStream_t st);
+cudaError_t launch_mlp_update(const float *part, const double *lossp, int slices, float *g, double *loss, float *p,
+                              float *m, float *v, __nv_bfloat16 *pb, float lr, float b1, float b2, float eps, float c1,
+                              float c2, cudaStream_t st);
 
 }  // namespace lqt

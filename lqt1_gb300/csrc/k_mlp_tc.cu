@@ -12,15 +12,16 @@
 // BF16 operand into shared memory.
 //
 // What bounds it: the 256 SiLUs per row.  Each needs an exponential and a
-// division; as ex2 + one reciprocal for two of them (1.5 MUFU, about 11 issue
-// slots in all) a row costs the MUFU pipe about 80 us per million rows, against
+// division; as ex2 + one reciprocal for two of them (1.5 MUFU, about 8 issue
+// slots in all, the FP32 arithmetic two
+// values per instruction) a row costs the MUFU pipe about 80 us per million rows, against
 // 42 us of memory traffic and 30 us of tensor time, so four groups per SM keep
 // that pipe fed while the others' MMAs, loads and stores run.  The quotient is
 // corrected by its exact remainder, so the BF16 activations are those of the
 // IEEE division.  Rows leave through a padded slab per warp: 16-byte
 // shared-memory stores without bank conflicts, then 512-byte global stores.
 // Measured (GB300, the call with its status read-back): 1,000,003 rows 988 ->
-// 167 us, 20,590 rows 60 -> 30 us against one group of one tile per CTA, two
+// 157 us, 20,590 rows 60 -> 30 us against one group of one tile per CTA, two
 // CTAs per SM; the outputs are the same bits.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -77,22 +78,53 @@ __device__ __forceinline__ float mlp_rcp(float x)
     return r;
 }
 
+// Two FP32 values in a register pair: one instruction for both (IEEE rounding
+// per value, as the scalar forms).
+__device__ __forceinline__ uint64_t pair2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void split2(uint64_t p, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // SiLU of two values, x / (1 + exp(-x)), as a BF16 pair.  One reciprocal of
 // the product of the two denominators serves both; each quotient is corrected
 // once by its remainder, which an FMA gives exactly (Markstein's correction),
-// so it is within 2^-40 or so of the division before it is rounded.  exp(-x)
-// is held at 1e18 (x < -41): the product of two stays finite, and the result
-// there, below 1e-16, is lost beside any other activation.
-__device__ __forceinline__ uint32_t silu2_bf16(float x0, float x1)
+// so it is within 2^-40 or so of the division before it is rounded.  (The
+// reciprocals and quotients are carried negated: the remainder is then one
+// FMA.)  exp(-x) is held at 1e18 (x < -41): the product of two stays finite,
+// and the result there, below 1e-16, is lost beside any other activation.
+__device__ __forceinline__ uint32_t silu2_bf16(uint64_t x)
 {
-    const float d0 = 1.0f + fminf(mlp_ex2(x0 * -1.4426950408889634f), 1e18f);
-    const float d1 = 1.0f + fminf(mlp_ex2(x1 * -1.4426950408889634f), 1e18f);
-    const float r = mlp_rcp(d0 * d1);
-    const float r0 = r * d1, r1 = r * d0;
-    float q0 = x0 * r0, q1 = x1 * r1;
-    q0 = fmaf(fmaf(-q0, d0, x0), r0, q0);
-    q1 = fmaf(fmaf(-q1, d1, x1), r1, q1);
-    const __nv_bfloat162 h = __floats2bfloat162_rn(q0, q1);
+    float a0, a1, d0, d1, q0, q1;
+    split2(mul2(x, pair2(-1.4426950408889634f, -1.4426950408889634f)), a0, a1);
+    const uint64_t d = add2(pair2(fminf(mlp_ex2(a0), 1e18f), fminf(mlp_ex2(a1), 1e18f)), pair2(1.0f, 1.0f));
+    split2(d, d0, d1);
+    const float r = mlp_rcp(d0 * -d1);
+    const uint64_t nr = pair2(r * d1, r * d0);
+    uint64_t nq = mul2(x, nr);
+    nq = fma2(fma2(nq, d, x), nr, nq);
+    split2(nq, q0, q1);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(-q0, -q1);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
@@ -215,8 +247,9 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_infer_tc(const __nv_bf
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const float4 b = bs[(c >> 2) + q * 2 + i];
-                        p[2 * i] = silu2_bf16(v[q * 8 + 4 * i] + b.x, v[q * 8 + 4 * i + 1] + b.y);
-                        p[2 * i + 1] = silu2_bf16(v[q * 8 + 4 * i + 2] + b.z, v[q * 8 + 4 * i + 3] + b.w);
+                        const float *u = v + q * 8 + 4 * i;
+                        p[2 * i] = silu2_bf16(add2(pair2(u[0], u[1]), pair2(b.x, b.y)));
+                        p[2 * i + 1] = silu2_bf16(add2(pair2(u[2], u[3]), pair2(b.z, b.w)));
                     }
                     *reinterpret_cast<uint4 *>(xh + tc::kmaj_off(t, c + q * 8, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
                 }

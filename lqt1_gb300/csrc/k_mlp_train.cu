@@ -10,8 +10,8 @@
 // is the operand of a forward or data-gradient GEMM, read MN-major (the
 // descriptor's strides exchanged, the transpose bits of the instruction set)
 // the same bytes are the transposed operand of a weight gradient, and W2 and
-// W3 those of a data gradient.  A CTA keeps its weight gradients in TMEM over
-// all of its tiles and writes one slice of them at the end.
+// W3 those of a data gradient.  Each CTA writes one slice of the gradients (to
+// which its later tiles, in batches above one tile per SM, are added).
 // k_mlp_update: adds the slices in a fixed order (the same bits on every run),
 // and applies Adam to the FP32 master weights and their BF16 copy.
 //
@@ -33,7 +33,7 @@ namespace lqt {
 namespace {
 
 constexpr int kTM = 128;                   // batch rows per tile (TMEM lanes)
-constexpr int kThreads = 256;              // two warps per 32 rows: one half of the columns each
+constexpr int kThreads = 512;              // four warps per 32 rows: 32 columns each
 constexpr uint32_t kWaitLimit = 1u << 24;  // bounded mbarrier polls
 
 // shared-memory plan (bytes): core-matrix tiles
@@ -52,11 +52,13 @@ constexpr uint32_t kNBias = 2 * kMlpHid + kMlpOut;
 constexpr uint32_t kOffBar = kOffBias + kNBias * 4;
 constexpr uint32_t kSmemBytes = kOffBar + 32;
 static_assert(kMlpIn == kMlpOut, "one 48-column tile type");
+static_assert((2048 + 16 * kMlpOut) * 4 <= kT48, "bias sums fit the output-gradient tile");
 static_assert(kOffBias % 16 == 0 && kOffBar % 8 == 0 && kSmemBytes <= 227 * 1024, "shared memory");
 
-// TMEM columns: pre-activation 1; pre-activation 2, then the outputs, then
-// the two data gradients; the weight gradients
-constexpr uint32_t kColZ1 = 0, kColWork = 128, kColG2 = 256, kColG3 = 384, kColG1 = 432, kTmemCols = 512;
+// TMEM columns: the pre-activations; the outputs, then the two data gradients
+// (work); the weight gradients (W2's over pre-activation 2, whose last use is
+// the gradient that W2's is formed from)
+constexpr uint32_t kColZ1 = 0, kColZ2 = 128, kColWork = 256, kColG2 = kColZ2, kColG3 = 384, kColG1 = 432, kTmemCols = 512;
 
 // Slice layout (floats): the parameter block's order W1 b1 W2 b2 W3 b3
 constexpr int kOW1 = 0, kOB1 = kOW1 + kMlpHid * kMlpIn, kOW2 = kOB1 + kMlpHid, kOB2 = kOW2 + kMlpHid * kMlpHid,
@@ -149,9 +151,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
     uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kOffBar + 8);
     float *bias = reinterpret_cast<float *>(smem + kOffBias);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int half = warp >> 2;                        // columns [64 half, 64 half + 64) of the hidden tiles
+    const int quarter = warp >> 2;                     // columns [32 quarter, + 32) of the hidden tiles
     const int row = (warp & 3) * 32 + lane;            // row of the tile = TMEM lane
-    const int c0 = half * 64;
+    const int c0 = quarter * 32, o0 = quarter * 16;    // and [16 quarter, + 16) of the outputs, for three of them
 
     stage_tile(smem + kOffW1, w.w1t, kMlpHid, kMlpIn, kMlpHid);
     stage_tile(smem + kOffW2, w.w2t, kMlpHid, kMlpHid, kMlpHid);
@@ -174,9 +176,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
     bool ok = true, first = true;
     float lhi = 0.f, llo = 0.f;                        // this thread's squared errors, a compensated pair
     // bias gradients: two columns and a share of the rows per thread
-    float2 g1 = make_float2(0.f, 0.f), g2 = g1, g3 = g1;
-    const int bc = (tid & 63) * 2, br = (tid >> 6) * 32;            // hidden: 64 pairs x 4 shares of 32 rows
-    const int oc = (tid % 24) * 2, orow = (tid / 24) * 16;          // outputs: 24 pairs x 8 shares of 16 rows (192 threads)
+    const int bc = (tid & 63) * 2, bs = tid >> 6;      // hidden: 64 pairs x 8 shares of 16 rows
+    const int oc = (tid % 24) * 2, os = tid / 24;      // outputs: 24 pairs x 16 shares of 8 rows (384 threads)
+    float *const out = part + (int64_t)blockIdx.x * kNP;
 
     // writes before it are visible to the MMAs, TMEM reads before it are done
     auto publish = [&]() {
@@ -196,48 +198,50 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
         tc::fence_after();
         return true;
     };
-    // hidden layer: pre-activations in z, SiLU to the operand tile
-    auto hidden = [&](uint32_t col, const float *b, uint8_t *dst, float *z) {
+    // pre-activation (TMEM + bias) of this thread's 32 columns
+    auto load_z = [&](uint32_t col, const float *b, float *z) {
+        tc::tmem_ld32(tl + col + c0, z);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            tc::tmem_ld32(tl + col + c0 + 32 * q, z + 32 * q);
+        for (int i = 0; i < 32; ++i) z[i] += b[c0 + i];
+    };
+    // hidden layer: SiLU to the operand tile
+    auto hidden = [&](uint32_t col, const float *b, uint8_t *dst) {
+        float z[32];
+        load_z(col, b, z);
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-                uint32_t p[4];
+        for (int i = 0; i < 32; i += 8) {
+            uint32_t p[4];
 #pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    const int k = 32 * q + i + j;
-                    z[k] += b[c0 + k];
-                    z[k + 1] += b[c0 + k + 1];
-                    p[j / 2] = pack2(z[k] * sigm(z[k]), z[k + 1] * sigm(z[k + 1]));
-                }
-                *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + 32 * q + i, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
+            for (int j = 0; j < 4; ++j) {
+                const float x = z[i + 2 * j], y = z[i + 2 * j + 1];
+                p[j] = pack2(x * sigm(x), y * sigm(y));
             }
+            *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + i, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
         }
     };
     // pre-activation gradient: the work columns times SiLU'(z)
-    auto dact = [&](const float *z, uint8_t *dst) {
+    auto dact = [&](uint32_t col, const float *b, uint8_t *dst) {
+        float z[32], v[32];
+        load_z(col, b, z);
+        tc::tmem_ld32(tl + kColWork + c0, v);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            float v[32];
-            tc::tmem_ld32(tl + kColWork + c0 + 32 * q, v);
+        for (int i = 0; i < 32; i += 8) {
+            uint32_t p[4];
 #pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-                uint32_t p[4];
+            for (int j = 0; j < 8; j += 2) {
+                float d[2];
 #pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    float d[2];
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const float zz = z[32 * q + i + j + u], sz = sigm(zz);
-                        d[u] = v[i + j + u] * (sz + zz * sz * (1.0f - sz));
-                    }
-                    p[j / 2] = pack2(d[0], d[1]);
+                for (int u = 0; u < 2; ++u) {
+                    const float zz = z[i + j + u], sz = sigm(zz);
+                    d[u] = v[i + j + u] * (sz + zz * sz * (1.0f - sz));
                 }
-                *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + 32 * q + i, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
+                p[j / 2] = pack2(d[0], d[1]);
             }
+            *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + i, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
         }
     };
+    // a slice element: the first tile's value, later tiles added to it
+    auto put = [&](int i, float x) { out[i] = first ? x : out[i] + x; };
 
     const int64_t ntiles = (B + kTM - 1) / kTM;
     for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
@@ -245,13 +249,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
         const int rows = (int)(B - m0 < kTM ? B - m0 : kTM);
         const bool live = row < rows;
         stage_tile(smem + kOffX, X + m0 * kMlpIn, kTM, kMlpIn, rows);
-        // this thread's targets: outputs 0..31 (first half) or 32..47
-        float tg[32];
-        const float *trow = T + (m0 + row) * kMlpOut + 32 * half;
+        // this thread's targets
+        float tg[16];
+        const float *trow = T + (m0 + row) * kMlpOut + o0;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
+        for (int j = 0; j < 16; j += 4) {
             float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (live && 32 * half + j < kMlpOut)
+            if (live && quarter < 3)
                 q = wide ? __ldg(reinterpret_cast<const float4 *>(trow + j)) : make_float4(trow[j], trow[j + 1], trow[j + 2], trow[j + 3]);
             tg[j] = q.x;
             tg[j + 1] = q.y;
@@ -265,16 +269,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
             tc::mma_commit(bar);
         }
         if (!(ok = arrived())) break;
-        float z[64];
-        hidden(kColZ1, bias, smem + kOffH1, z);
+        hidden(kColZ1, bias, smem + kOffH1);
         publish();
         if (tid == 0) {
             tc::fence_after();
-            mma_all(tm + kColWork, kmajor(smem + kOffH1, kMlpHid), false, kmajor(smem + kOffW2, kMlpHid), false, kMlpHid, kMlpHid, false);
+            mma_all(tm + kColZ2, kmajor(smem + kOffH1, kMlpHid), false, kmajor(smem + kOffW2, kMlpHid), false, kMlpHid, kMlpHid, false);
             tc::mma_commit(bar);
         }
         if (!(ok = arrived())) break;
-        hidden(kColWork, bias + kMlpHid, smem + kOffH2, z);        // z: pre-activation 2 from here on
+        hidden(kColZ2, bias + kMlpHid, smem + kOffH2);
         publish();
         if (tid == 0) {
             tc::fence_after();
@@ -283,12 +286,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
         }
         if (!(ok = arrived())) break;
         // outputs: loss and its gradient
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            if (32 * half + 16 * q >= kMlpOut) break;              // (uniform in a warp)
-            const int o = 32 * half + 16 * q;
+        if (quarter < 3) {
             float y[16];
-            tc::tmem_ld16(tl + kColWork + o, y);
+            tc::tmem_ld16(tl + kColWork + o0, y);
 #pragma unroll
             for (int i = 0; i < 16; i += 8) {
                 uint32_t p[4];
@@ -297,8 +297,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
                     float g[2];
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
-                        const int c = o + i + j + u;
-                        float d = (y[i + j + u] + bias[2 * kMlpHid + c]) - tg[16 * q + i + j + u];
+                        const int c = o0 + i + j + u;
+                        float d = (y[i + j + u] + bias[2 * kMlpHid + c]) - tg[i + j + u];
                         if (c >= nvalid || !live) d = 0.f;
                         g[u] = scale * d;
                         // (lhi, llo) += d^2: the square's rounding error by an FMA, the sum's by TwoSum
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
                     }
                     p[j / 2] = pack2(g[0], g[1]);
                 }
-                *reinterpret_cast<uint4 *>(smem + kOffDY + tc::kmaj_off(row, o + i, kMlpOut)) = make_uint4(p[0], p[1], p[2], p[3]);
+                *reinterpret_cast<uint4 *>(smem + kOffDY + tc::kmaj_off(row, o0 + i, kMlpOut)) = make_uint4(p[0], p[1], p[2], p[3]);
             }
         }
         publish();
@@ -318,100 +318,74 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
             mma_all(tm + kColWork, kmajor(smem + kOffDY, kMlpOut), false, mnmajor(smem + kOffW3, kMlpHid), true, kMlpHid, kMlpOut, false);
             tc::mma_commit(bar);
             // W3 gradient, transposed: [hidden][output]
-            mma_all(tm + kColG3, mnmajor(smem + kOffH2, kMlpHid), true, mnmajor(smem + kOffDY, kMlpOut), true, kMlpOut, kTM, !first);
+            mma_all(tm + kColG3, mnmajor(smem + kOffH2, kMlpHid), true, mnmajor(smem + kOffDY, kMlpOut), true, kMlpOut, kTM, false);
         }
-        if (tid < 192) {
-            const float2 s = column_sums(smem + kOffDY, kMlpOut, oc, orow, 16);
-            g3.x += s.x;
-            g3.y += s.y;
-        }
+        const float2 g3 = tid < 384 ? column_sums(smem + kOffDY, kMlpOut, oc, os * 8, 8) : make_float2(0.f, 0.f);
         if (!(ok = arrived())) break;
-        dact(z, smem + kOffDZ2);
+        dact(kColZ2, bias + kMlpHid, smem + kOffDZ2);
         publish();
         if (tid == 0) {
             tc::fence_after();
             mma_all(tm + kColWork, kmajor(smem + kOffDZ2, kMlpHid), false, mnmajor(smem + kOffW2, kMlpHid), true, kMlpHid, kMlpHid, false);
             tc::mma_commit(bar);
             // W2 gradient, transposed: [in][out]
-            mma_all(tm + kColG2, mnmajor(smem + kOffH1, kMlpHid), true, mnmajor(smem + kOffDZ2, kMlpHid), true, kMlpHid, kTM, !first);
+            mma_all(tm + kColG2, mnmajor(smem + kOffH1, kMlpHid), true, mnmajor(smem + kOffDZ2, kMlpHid), true, kMlpHid, kTM, false);
         }
-        {
-            const float2 s = column_sums(smem + kOffDZ2, kMlpHid, bc, br, 32);
-            g2.x += s.x;
-            g2.y += s.y;
-        }
+        const float2 g2 = column_sums(smem + kOffDZ2, kMlpHid, bc, bs * 16, 16);
         if (!(ok = arrived())) break;
-        // pre-activation 1 is still in its columns
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            tc::tmem_ld32(tl + kColZ1 + c0 + 32 * q, z + 32 * q);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) z[32 * q + i] += bias[c0 + 32 * q + i];
-        }
-        dact(z, smem + kOffDZ1);
+        dact(kColZ1, bias, smem + kOffDZ1);
         publish();
         if (tid == 0) {
             tc::fence_after();
             // W1 gradient: [out][in]
-            mma_all(tm + kColG1, mnmajor(smem + kOffDZ1, kMlpHid), true, mnmajor(smem + kOffX, kMlpIn), true, kMlpIn, kTM, !first);
+            mma_all(tm + kColG1, mnmajor(smem + kOffDZ1, kMlpHid), true, mnmajor(smem + kOffX, kMlpIn), true, kMlpIn, kTM, false);
             tc::mma_commit(bar);
         }
-        {
-            const float2 s = column_sums(smem + kOffDZ1, kMlpHid, bc, br, 32);
-            g1.x += s.x;
-            g1.y += s.y;
-        }
+        const float2 g1 = column_sums(smem + kOffDZ1, kMlpHid, bc, bs * 16, 16);
         if (!(ok = arrived())) break;               // and with it every earlier MMA: the tiles may be overwritten
+        // the slice; [in][out] accumulators: a warp writes 32 neighbouring inputs of one output
+        {
+            float v[32];
+            tc::tmem_ld32(tl + kColG2 + c0, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) put(kOW2 + (c0 + i) * kMlpHid + row, v[i]);
+            if (quarter < 3) {
+                tc::tmem_ld16(tl + kColG3 + o0, v);
+                tc::tmem_ld16(tl + kColG1 + o0, v + 16);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) put(kOW3 + (o0 + i) * kMlpHid + row, v[i]);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) put(kOW1 + row * kMlpIn + o0 + i, v[16 + i]);
+            }
+        }
+        // bias gradients: the rows' shares added in order
+        float *cs = reinterpret_cast<float *>(smem + kOffDY);          // (the tiles are free now)
+        cs[bs * 128 + bc] = g1.x;
+        cs[bs * 128 + bc + 1] = g1.y;
+        cs[1024 + bs * 128 + bc] = g2.x;
+        cs[1024 + bs * 128 + bc + 1] = g2.y;
+        if (tid < 384) {
+            cs[2048 + os * 48 + oc] = g3.x;
+            cs[2048 + os * 48 + oc + 1] = g3.y;
+        }
+        __syncthreads();
+        if (tid < 2 * kMlpHid + kMlpOut) {
+            const int n = tid < 2 * kMlpHid ? 8 : 16, step = tid < 2 * kMlpHid ? 128 : 48;
+            const float *q = tid < kMlpHid ? cs + tid : (tid < 2 * kMlpHid ? cs + 1024 + tid - kMlpHid : cs + 2048 + tid - 2 * kMlpHid);
+            float s = 0.f;
+            for (int r = 0; r < n; ++r) s += q[r * step];
+            put(tid < kMlpHid ? kOB1 + tid : (tid < 2 * kMlpHid ? kOB2 + tid - kMlpHid : kOB3 + tid - 2 * kMlpHid), s);
+        }
+        tc::fence_before();
+        __syncthreads();                             // before the next tile's inputs and MMAs
         first = false;
     }
     if (ok) {
-        float *out = part + (int64_t)blockIdx.x * kNP;
-        float v[32];
-        // [in][out] accumulators: a warp writes 32 neighbouring inputs of one output
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            tc::tmem_ld32(tl + kColG2 + c0 + 32 * q, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) out[kOW2 + (c0 + 32 * q + i) * kMlpHid + row] = v[i];
-        }
-        // 48 columns: 0..31 by the first half's warps, 32..47 by the second's
-        if (half == 0) {
-            tc::tmem_ld32(tl + kColG3, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) out[kOW3 + i * kMlpHid + row] = v[i];
-            tc::tmem_ld32(tl + kColG1, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) out[kOW1 + row * kMlpIn + i] = v[i];
-        } else {
-            tc::tmem_ld16(tl + kColG3 + 32, v);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) out[kOW3 + (32 + i) * kMlpHid + row] = v[i];
-            tc::tmem_ld16(tl + kColG1 + 32, v);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) out[kOW1 + row * kMlpIn + 32 + i] = v[i];
-        }
-        // bias gradients: the rows' shares added in order
-        float *cs = reinterpret_cast<float *>(smem + kOffDZ2);          // the tiles are free now
-        cs[(tid >> 6) * 128 + bc] = g1.x;
-        cs[(tid >> 6) * 128 + bc + 1] = g1.y;
-        cs[512 + (tid >> 6) * 128 + bc] = g2.x;
-        cs[512 + (tid >> 6) * 128 + bc + 1] = g2.y;
-        if (tid < 192) {
-            cs[1024 + (tid / 24) * 48 + oc] = g3.x;
-            cs[1024 + (tid / 24) * 48 + oc + 1] = g3.y;
-        }
         double l = (double)lhi + (double)llo;
         for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
         if (lane == 0) lred[warp] = l;
         __syncthreads();
-        if (tid < 128) {
-            out[kOB1 + tid] = ((cs[tid] + cs[128 + tid]) + cs[256 + tid]) + cs[384 + tid];
-            out[kOB2 + tid] = ((cs[512 + tid] + cs[640 + tid]) + cs[768 + tid]) + cs[896 + tid];
-        } else if (tid < 128 + kMlpOut) {
-            float s = 0.f;
-            for (int q = 0; q < 8; ++q) s += cs[1024 + q * 48 + tid - 128];
-            out[kOB3 + tid - 128] = s;
-        } else if (tid == 255) {
+        if (tid == 0) {
             double s = 0.0;
             for (int q = 0; q < kThreads / 32; ++q) s += lred[q];
             lossp[blockIdx.x] = s;
@@ -422,28 +396,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
     if (warp == 0) tc::tmem_dealloc(tm, kTmemCols);
 }
 
-// G[i] = the slices of parameter i added in slice order (four runs of slices,
-// then the four sums in order); with lr > 0 one Adam step with bias correction
-// c1, c2 on the FP32 master weights and their BF16 copy.  loss = sum of lossp.
-__global__ void __launch_bounds__(256) k_mlp_update(const float *__restrict__ part, const double *__restrict__ lossp,
-                                                    int slices, float *__restrict__ g, double *__restrict__ loss,
-                                                    float *__restrict__ p, float *__restrict__ m, float *__restrict__ v,
-                                                    __nv_bfloat16 *__restrict__ pb, float lr, float b1, float b2,
-                                                    float eps, float c1, float c2)
+// G[i] = the slices of parameter i added in slice order; with lr > 0 one Adam
+// step with bias correction c1, c2 on the FP32 master weights and their BF16
+// copy.  loss = sum of lossp.  Bound by the latency of the slices' loads: small
+// blocks over all SMs, 32 loads issued together.
+constexpr int kUpThreads = 64;
+__global__ void __launch_bounds__(kUpThreads) k_mlp_update(const float *__restrict__ part,
+                                                           const double *__restrict__ lossp, int slices,
+                                                           float *__restrict__ g, double *__restrict__ loss,
+                                                           float *__restrict__ p, float *__restrict__ m,
+                                                           float *__restrict__ v, __nv_bfloat16 *__restrict__ pb, float lr,
+                                                           float b1, float b2, float eps, float c1, float c2)
 {
-    __shared__ float red[4][64];
-    const int q = threadIdx.x >> 6, j = threadIdx.x & 63;
-    const int i = blockIdx.x * 64 + j;
-    const int s0 = q * slices / 4, s1 = (q + 1) * slices / 4;
-    float acc = 0.f;
+    const int i = blockIdx.x * kUpThreads + threadIdx.x;
     if (i < kNP) {
-#pragma unroll 16
-        for (int s = s0; s < s1; ++s) acc += part[(int64_t)s * kNP + i];
-    }
-    red[q][j] = acc;
-    __syncthreads();
-    if (q == 0 && i < kNP) {
-        const float gi = ((red[0][j] + red[1][j]) + red[2][j]) + red[3][j];
+        float gi = 0.f;
+#pragma unroll 32
+        for (int s = 0; s < slices; ++s) gi += part[(int64_t)s * kNP + i];
         g[i] = gi;
         if (lr > 0.f) {
             const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -454,8 +423,7 @@ __global__ void __launch_bounds__(256) k_mlp_update(const float *__restrict__ pa
             p[i] = pn;
             pb[i] = __float2bfloat16(pn);
         }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 64) {
+    } else if (i == kNP) {
         double s = 0.0;
         for (int k = 0; k < slices; ++k) s += lossp[k];
         *loss = s;
@@ -493,7 +461,7 @@ cudaError_t launch_mlp_update(const float *part, const double *lossp, int slices
                               float *m, float *v, __nv_bfloat16 *pb, float lr, float b1, float b2, float eps, float c1,
                               float c2, cudaStream_t st)
 {
-    k_mlp_update<<<(kNP + 63) / 64, 256, 0, st>>>(part, lossp, slices, g, loss, p, m, v, pb, lr, b1, b2, eps, c1, c2);
+    k_mlp_update<<<kNP / kUpThreads + 1, kUpThreads, 0, st>>>(part, lossp, slices, g, loss, p, m, v, pb, lr, b1, b2, eps, c1, c2);
     return cudaGetLastError();
 }
 

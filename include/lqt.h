@@ -388,10 +388,11 @@ int lqt_sim_substep_variant(lqt_sim *s, int32_t variant, int32_t *chosen, float 
 
 /* Instrumentation (no counterpart in the reference, which has no timing):
  * run nsteps steps without graph capture, timing each launch of the fused
- * step kernel, of the ghost/clock kernel and (with a surrogate attached) of
- * the surrogate macro-step kernel with CUDA events on the simulation's
- * stream; returns the mean milliseconds per launch (ms_sur: per macro-step
- * launch, 0 when none ran).  NULL outputs are skipped. */
+ * step kernel, of the ghost/clock kernel (0 on small grids, whose step kernel
+ * does its work) and (with a surrogate attached) of the surrogate macro-step
+ * kernel with CUDA events on the simulation's stream; returns the mean
+ * milliseconds per launch (ms_sur: per macro-step launch, 0 when none ran).
+ * NULL outputs are skipped. */
 int lqt_sim_profile(lqt_sim *s, int64_t nsteps, double *ms_step, double *ms_ghost,
                     double *ms_sur);
 

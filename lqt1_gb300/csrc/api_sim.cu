@@ -2,8 +2,8 @@
 //
 // The host loop of the reference (GPU3D.cu:1731-1842, new_11.cu:1755-1890)
 // launches five kernels with a device-wide synchronisation between them and
-// copies all of V back every step.  Here a step is two kernels (k_grid_step,
-// k_ghost) on one stream; runs of steps are captured once into a CUDA graph
+// copies all of V back every step.  Here a step is one kernel (two on larger
+// grids: k_grid_step, k_ghost) on one stream; runs of steps are captured once into a CUDA graph
 // and replayed, the stimulus schedule and time live on the device, the
 // blow-up scan is a counter read on request, and the pseudo-ECG is reduced on
 // the device every `every` steps.
@@ -51,10 +51,11 @@ struct lqt_sim {
     int32_t *vbox_hdr = nullptr, *vli = nullptr;   // V-halo boxes of the 3D substep (k_sur_substep_vbox)
     double *conc = nullptr, *aos = nullptr;
     int32_t *gidx = nullptr, *bnd_dst = nullptr, *bnd_src = nullptr;
+    int32_t *gref = nullptr, *glist = nullptr;   // the mirror map by source voxel (GridDev::gref)
     float *xpos = nullptr;          // 2D/3D: (float)(i * dx), i < max(nx, ny, nz)
     uint8_t *ctl = nullptr;
     float *onset = nullptr;
-    Clock *clk = nullptr;
+    Clock *clk = nullptr;           // [2]: one per V grid
     Win *win = nullptr;
     int64_t win_cap = 0;
     float4 *det = nullptr;
@@ -81,6 +82,8 @@ struct lqt_sim {
     // occupancy variant of k_grid_step (minimum CTAs/SM) and the autotuner
     int minb = 2;
     int sub_minb = 5;               // V-only substep variant (kSubVariants)
+    int64_t small_n = 0;            // voxels up to which a grid is small (kSmallPerSM per SM)
+    bool step_forced = false;       // set by lqt_sim_tune with a variant
     bool sub_forced = false;        // set by lqt_sim_substep_variant: the autotuner keeps it
     int32_t sub_skip_copy = 0;      // failure-path test (lqt_sim_set_wait_test)
     uint32_t sub_wait_limit = 0;
@@ -137,6 +140,9 @@ struct lqt_sim {
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
     bool fp64() const { return p.precision == LQT_FP64; }
+    // A step is one launch: small grids in the mixed form, unless a variant of
+    // the step kernel, or of the substep in effect, was asked for.
+    bool folds() const { return !fp64() && ntissue <= small_n && !step_forced && !(sub_forced && sur && plist_valid); }
 
     template <typename R> GridDev<R> dev() const
     {
@@ -176,6 +182,9 @@ struct lqt_sim {
         g.onset = onset;
         g.bnd_dst = bnd_dst;
         g.bnd_src = bnd_src;
+        g.gref = gref;
+        g.glist = glist;
+        g.fold = folds();
         g.det = det;
         g.apd90 = apd90;
         g.act_thr = (float)p.act_threshold;
@@ -303,8 +312,36 @@ int refresh_windows(lqt_sim *s, int64_t horizon)
     c.s2_on = s->step >= s2.on && s->step < s2.off;
     c.tb = s->time - std::floor(s->time / q.bcl) * q.bcl;
     c.s1_cycle_ok = q.s1_beats <= 0 || std::floor(s->time / q.bcl) < q.s1_beats;
-    CK(cudaMemcpyAsync(s->clk, &c, sizeof(c), cudaMemcpyHostToDevice, s->stream));
+    CK(cudaMemcpyAsync(s->clk + s->cur, &c, sizeof(c), cudaMemcpyHostToDevice, s->stream));
     return LQT_OK;
+}
+
+// The mirror map by source voxel: the one empty voxel that mirrors it, or where
+// its list of them starts (GridDev::gref), and kCtlGhost in its control byte.
+void build_ghost_refs(const TissueMap &tm, std::vector<uint8_t> &ctl, std::vector<int32_t> &gref,
+                      std::vector<int32_t> &glist)
+{
+    const int64_t n = (int64_t)tm.cells.size(), nb = (int64_t)tm.bnd_dst.size();
+    std::vector<int32_t> first(n, -1), next(nb, -1);     // each source's mirror voxels as a chain
+    for (int64_t j = nb - 1; j >= 0; --j) {
+        const int32_t k = tm.tissue_of[tm.bnd_src[j]];
+        if (k < 0) continue;                             // (mirrors itself: nothing to copy)
+        next[j] = first[k];
+        first[k] = (int32_t)j;
+    }
+    gref.assign(n, 0);
+    glist.clear();
+    for (int64_t k = 0; k < n; ++k) {
+        if (first[k] < 0) continue;
+        ctl[k] |= kCtlGhost;
+        if (next[first[k]] < 0) {
+            gref[k] = (int32_t)tm.bnd_dst[first[k]];
+            continue;
+        }
+        gref[k] = ~(int32_t)glist.size();
+        for (int32_t j = first[k]; j >= 0; j = next[j]) glist.push_back((int32_t)tm.bnd_dst[j]);
+        glist.back() |= INT32_MIN;
+    }
 }
 
 // At a macro-step boundary with a surrogate attached: the macro-step kernel.
@@ -339,14 +376,14 @@ int launch_sur_if_due(lqt_sim *s)
     return LQT_OK;
 }
 
-// The step kernels of one step (without the ghost refresh): the fused plain
-// step over all voxels, or, inside a surrogate macro step, the V-only step of
+// The step kernels of one step: the fused plain step over all voxels, or, inside a surrogate macro step, the V-only step of
 // the surrogate voxels and the plain step over the listed ones.
 cudaError_t launch_substep(lqt_sim *s)
 {
     const StepK k = make_stepk(s->p.dt);
     if (s->fp64()) return launch_grid_step<double>(devf<double>(s), k, s->cur, s->dim, s->minb, s->stream);
     const GridDev<float> g = devf<float>(s);
+    if (g.srate && g.fold) return launch_sur_step_small(g, k, s->cur, s->dim, s->stream);
     if (g.srate) {
         cudaError_t e = launch_sur_substep(g, s->p.dt, s->cur, s->dim, s->sub_minb, s->stream);
         if (e != cudaSuccess) return e;
@@ -354,10 +391,12 @@ cudaError_t launch_substep(lqt_sim *s)
     return launch_grid_step<float>(g, k, s->cur, s->dim, s->minb, s->stream);
 }
 
+// The mirror voxels and the clock, where the step kernels leave them to a launch of their own.
 cudaError_t launch_ghost_now(lqt_sim *s)
 {
-    return s->fp64() ? launch_ghost<double>(devf<double>(s), s->cur ^ 1, s->stream)
-                     : launch_ghost<float>(devf<float>(s), s->cur ^ 1, s->stream);
+    if (s->folds()) return cudaSuccess;
+    return s->fp64() ? launch_ghost<double>(devf<double>(s), s->cur, 1, s->stream)
+                     : launch_ghost<float>(devf<float>(s), s->cur, 1, s->stream);
 }
 
 int launch_step(lqt_sim *s)
@@ -446,7 +485,7 @@ int autotune(lqt_sim *s, int per, int64_t *consumed)
     s->minb = best_m;
     // with a surrogate attached: the V-only substep's variant, timed the same
     // way (variants in turn, whole steps, the first round discarded)
-    if (rc == LQT_OK && s->sur && !s->fp64() && !s->sub_forced) {
+    if (rc == LQT_OK && s->sur && !s->fp64() && !s->sub_forced && !s->folds()) {
         float ts[kSubNVariants] = {};
         for (int i = 0; i < per && rc == LQT_OK; ++i) {
             for (int c = 0; c < kSubNVariants && rc == LQT_OK; ++c) {
@@ -640,6 +679,12 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
         }
     }
     s->ntissue = (int64_t)s->tm.cells.size();
+    {
+        int dev = 0, nsm = 152;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        s->small_n = (int64_t)nsm * kSmallPerSM;
+    }
     s->nbnd = (int64_t)s->tm.bnd_dst.size();
     if (s->ntissue == 0) {
         delete s;
@@ -655,7 +700,7 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
     rc |= s->mem.alloc((void **)&s->conc, s->ld * 8 * kNConc);
     const int64_t npad = pad_tiles(n);     // per-voxel rows the staged substep copies in whole tiles
     rc |= s->mem.alloc((void **)&s->ctl, npad);
-    rc |= s->mem.alloc((void **)&s->clk, sizeof(Clock));
+    rc |= s->mem.alloc((void **)&s->clk, 2 * sizeof(Clock));
     rc |= s->mem.alloc((void **)&s->nbad, sizeof(unsigned long long));
     if (dim > 1) {
         rc |= s->mem.alloc((void **)&s->gidx, npad * 4);
@@ -680,12 +725,11 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
         return fail(LQT_ERR_NOMEM, "lqt_sim_create: " + m);
     }
     cudaStream_t st = s->stream;
-    // the device clock is read by k_ghost, which set_state below launches:
-    // give it a defined value before any kernel runs
+    // the device clock has a defined value before any kernel runs
     {
-        Clock c0{};
-        c0.s1_cycle_ok = 1;
-        if (cudaMemcpy(s->clk, &c0, sizeof(c0), cudaMemcpyHostToDevice) != cudaSuccess) {
+        Clock c0[2] = {};
+        c0[0].s1_cycle_ok = c0[1].s1_cycle_ok = 1;
+        if (cudaMemcpy(s->clk, c0, sizeof(c0), cudaMemcpyHostToDevice) != cudaSuccess) {
             delete s;
             return fail(LQT_ERR_CUDA, "lqt_sim_create: clock upload failed");
         }
@@ -693,6 +737,15 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
     // per-voxel control bytes and maps
     s->ctl_host.resize(n);
     for (int64_t k = 0; k < n; ++k) s->ctl_host[k] = geom->cell_type[s->tm.cells[k]] & kCtlType;
+    std::vector<int32_t> gref, glist;
+    if (s->nbnd) {
+        build_ghost_refs(s->tm, s->ctl_host, gref, glist);
+        if (s->mem.alloc((void **)&s->gref, n * 4) | s->mem.alloc((void **)&s->glist, glist.size() * 4)) {
+            std::string m = g_err;
+            delete s;
+            return fail(LQT_ERR_NOMEM, "lqt_sim_create: " + m);
+        }
+    }
     std::vector<int32_t> gi32(dim > 1 ? n : 0), bd(s->nbnd), bs(s->nbnd);
     for (int64_t k = 0; k < (int64_t)gi32.size(); ++k) gi32[k] = (int32_t)s->tm.cells[k];
     for (int64_t j = 0; j < s->nbnd; ++j) {
@@ -708,6 +761,9 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
     if (e == cudaSuccess && dim > 1) e = cudaMemcpyAsync(s->gidx, gi32.data(), n * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && s->nbnd) e = cudaMemcpyAsync(s->bnd_dst, bd.data(), s->nbnd * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && s->nbnd) e = cudaMemcpyAsync(s->bnd_src, bs.data(), s->nbnd * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && s->gref) e = cudaMemcpyAsync(s->gref, gref.data(), n * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !glist.empty())
+        e = cudaMemcpyAsync(s->glist, glist.data(), glist.size() * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         delete s;
@@ -767,7 +823,7 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
     if (!rc) {
         Clock c{};
         c.s1_cycle_ok = 1;
-        cudaError_t e2 = cudaMemcpyAsync(s->clk, &c, sizeof(c), cudaMemcpyHostToDevice, st);
+        cudaError_t e2 = cudaMemcpyAsync(s->clk + s->cur, &c, sizeof(c), cudaMemcpyHostToDevice, st);
         std::vector<float4> d0(s->det ? n : 0, make_float4(0.f, 0.f, -1.f, 0.f));
         if (e2 == cudaSuccess && s->det) e2 = cudaMemcpyAsync(s->det, d0.data(), n * sizeof(float4), cudaMemcpyHostToDevice, st);
         if (e2 == cudaSuccess && s->apd90) e2 = cudaMemsetAsync(s->apd90, 0xff, n * 4, st);
@@ -806,7 +862,7 @@ int lqt_sim_set_protocol(lqt_sim *s, const lqt_protocol *q)
     std::vector<float> on;
     for (int64_t k = 0; k < n; ++k) {
         const int64_t g = s->tm.cells[k];
-        c[k] = (uint8_t)((c[k] & kCtlType) | (q->s1_mask[g] ? kCtlS1 : 0) | (q->s2_mask && q->s2_mask[g] ? kCtlS2 : 0));
+        c[k] = (uint8_t)((c[k] & (kCtlType | kCtlGhost)) | (q->s1_mask[g] ? kCtlS1 : 0) | (q->s2_mask && q->s2_mask[g] ? kCtlS2 : 0));
     }
     if (q->s1_onset) {
         on.resize(n);
@@ -1028,13 +1084,12 @@ int lqt_sim_set_state(lqt_sim *s, const double *state_host)
     if (s->fp64()) {
         if (e == cudaSuccess) e = launch_pack<double>(s->aos, SoA<double>{(double *)vtmp, s->conc, (double *)s->gate, s->ld}, n, s->stream);
         if (e == cudaSuccess) e = launch_scatter_v<double>((double *)vtmp, gi, (double *)s->vg[s->cur], n, s->stream);
-        if (e == cudaSuccess) e = launch_ghost<double>(s->dev<double>(), s->cur, s->stream);
+        if (e == cudaSuccess) e = launch_ghost<double>(s->dev<double>(), s->cur ^ 1, 0, s->stream);
     } else {
         if (e == cudaSuccess) e = launch_pack<float>(s->aos, SoA<float>{(float *)vtmp, s->conc, (float *)s->gate, s->ld}, n, s->stream);
         if (e == cudaSuccess) e = launch_scatter_v<float>((float *)vtmp, gi, (float *)s->vg[s->cur], n, s->stream);
-        if (e == cudaSuccess) e = launch_ghost<float>(s->dev<float>(), s->cur, s->stream);
+        if (e == cudaSuccess) e = launch_ghost<float>(s->dev<float>(), s->cur ^ 1, 0, s->stream);
     }
-    // launch_ghost also advanced the device clock: restore it
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return fail(LQT_ERR_CUDA, std::string("lqt_sim_set_state: ") + cudaGetErrorString(e));
     // a new state ends any macro step in progress: every voxel runs the plain
@@ -1048,7 +1103,7 @@ int lqt_sim_set_state(lqt_sim *s, const double *state_host)
     c.time_f = (float)s->time;
     c.s1_cycle_ok = 1;
     CK(cudaStreamSynchronize(s->stream));    // steps enqueued without waiting read the clock
-    CK(cudaMemcpy(s->clk, &c, sizeof(c), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(s->clk + s->cur, &c, sizeof(c), cudaMemcpyHostToDevice));
     return LQT_OK;
 }
 
@@ -1132,10 +1187,12 @@ int lqt_sim_tune(lqt_sim *s, int32_t variant, int32_t *chosen, float *ms_per_var
         for (int c = 0; c < ncand; ++c) ok |= cand[c] == variant;
         if (!ok) return fail(LQT_ERR_INVALID, "lqt_sim_tune: variant must be 2, 3 or 4 (mixed) or 1, 2 (FP64)");
         s->minb = variant;
+        s->step_forced = true;
         s->tuned = true;
         s->graph_valid = false;
     } else {
         int64_t used = 0;
+        s->step_forced = false;
         int rc = autotune(s, 5, &used);
         if (rc) return rc;
         CK(cudaStreamSynchronize(s->stream));
@@ -1191,6 +1248,7 @@ int lqt_sim_profile(lqt_sim *s, int64_t nsteps, double *ms_step, double *ms_ghos
         float a = 0, b = 0;
         if (e == cudaSuccess) e = cudaEventElapsedTime(&a, ev[0], ev[1]);
         if (e == cudaSuccess) e = cudaEventElapsedTime(&b, ev[1], ev[2]);
+        if (s->folds()) b = 0;
         if (e != cudaSuccess) rc = fail(LQT_ERR_CUDA, std::string("lqt_sim_profile: ") + cudaGetErrorString(e));
         t_step += a;
         t_ghost += b;

@@ -11,10 +11,12 @@ namespace lqt {
 constexpr uint8_t kCtlType = 7;    // bits 0-2: LQT_* cell type (0..4)
 constexpr uint8_t kCtlS1 = 8;      // receives S1
 constexpr uint8_t kCtlS2 = 16;     // receives S2
+constexpr uint8_t kCtlGhost = 32;  // mirrored by empty voxels next to it (GridDev::gref)
 constexpr int kMaxElectrodes = 8;
 
-// Per-step control, advanced on the device by k_ghost so that a run of steps
-// can be captured in one CUDA graph.
+// Per-step control, advanced on the device so that a run of steps can be
+// captured in one CUDA graph.  Two copies alternate with the V grids: a step
+// from grid cur reads clk[cur] while one thread of it writes clk[cur ^ 1].
 struct Clock {
     int64_t step;
     double time;        // accumulated as `time += dt` (OneD.cc:317)
@@ -42,7 +44,7 @@ template <typename R> struct GridDev {
     const float *xpos;
     double dt;
     ModelT<R> model;
-    Clock *clk;
+    Clock *clk;                    // [2]
     const Win *win;                // S1 windows
     int32_t nwin;
     int32_t s1_beats;
@@ -51,6 +53,11 @@ template <typename R> struct GridDev {
     R s1_strength, s2_strength;
     const float *onset;            // per tissue voxel onset delay, or null
     const int32_t *bnd_dst, *bnd_src;
+    // the same map from the source's side, for the tissue voxels with kCtlGhost:
+    // gref[k] >= 0 is the one empty voxel that mirrors voxel k, else ~gref[k] is
+    // where its list starts in glist, whose last entry has the sign bit set
+    const int32_t *gref, *glist;
+    int32_t fold;                  // 1: a step's one launch writes mirror voxels and clock (small grids)
     float4 *det;                   // {vrest, vpeak, t_act, bits}, or null
     float *apd90;
     float act_thr;
@@ -105,7 +112,13 @@ template <typename R>
 cudaError_t launch_grid_step(const GridDev<R> &gd, const StepK &k, int cur, int dim, int minb, cudaStream_t st);
 template <typename R>
 cudaError_t launch_grid_step_minb(const GridDev<R> &gd, const StepT<R> &k, int cur, int dim, int minb, cudaStream_t st);
-template <typename R> cudaError_t launch_ghost(const GridDev<R> &gd, int nxt, cudaStream_t st);
+template <typename R> cudaError_t launch_ghost(const GridDev<R> &gd, int cur, int clock, cudaStream_t st);
+// Grids of at most this many voxels per SM step in one launch (mixed form):
+// narrow CTAs over all SMs with all the registers the step can use, because
+// the time is then one thread's chain of loads and arithmetic (four warps per
+// SM partition at the most), and no second launch.
+constexpr int kSmallPerSM = 512;
+cudaError_t launch_sur_step_small(const GridDev<float> &gd, const StepK &k, int cur, int dim, cudaStream_t st);
 // Variants of the V-only substep: minimum CTAs/SM of 256 threads of
 // k_sur_substep (5, 6, 8: one thread per voxel, direct loads), of
 // k_sur_substep_tile (100 + CTAs/SM: persistent CTAs, each tile's streamed

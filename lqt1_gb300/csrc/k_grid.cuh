@@ -2,15 +2,21 @@
 //
 // Replaces the reference's per-step kernel chain calc_du -> init_Istim ->
 // set_Istim -> Itot -> new_u_v (GPU3D.cu:370-425,1222-1230; new_11.cu:352-455,
-// 1241-1255) with one kernel per step plus a small ghost-fill kernel.
+// 1241-1255) with one kernel per step, plus a mirror-boundary kernel on larger
+// grids.
 //
 // Layout: V lives in a dense grid (x-major, z fastest, as GPU3D.cu:29-33),
 // double-buffered; the other 39 states live in structure-of-arrays order over
 // the tissue voxels (common.cuh).  One thread per tissue voxel: it reads its V
 // stencil from the dense grid (neighbour rows are shared through L1/L2), its
 // state with streaming loads, and writes V into the other grid.  Empty voxels
-// next to tissue hold the V of their mirror source (GPU3D.cu:1487-1604),
-// refreshed after every step by k_ghost, so the stencil needs no branches.
+// next to tissue hold the V of their mirror source (GPU3D.cu:1487-1604), so the
+// stencil needs no branches.  On small grids (kSmallPerSM) the source's thread
+// writes them together with its own V and a step is one launch; on larger ones
+// k_ghost refreshes them after the step, because there the scattered stores in
+// the step kernels cost more than the launch (50 steps: sheet of 97 x 64
+// 1.01 -> 0.57 ms folded; 320 x 320 x 420 ventricle 10.36 ms with k_ghost,
+// 10.94 ms folded).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -146,18 +152,66 @@ template <typename R> __device__ __forceinline__ void grid_count_bad(const GridD
     if (m && (threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(gd.nbad, (unsigned long long)__popc(m));
 }
 
+// Voxel k's entry of the mirror map; loaded with the V stencil, so that it is
+// there when the new V is.
+template <typename R> __device__ __forceinline__ int32_t ghost_ref(const GridDev<R> &gd, int64_t k, uint8_t ctl)
+{
+    return (ctl & kCtlGhost) ? gd.gref[k] : 0;
+}
+
+// The new V of a tissue voxel (dense index g), there and in the empty voxels
+// that mirror it (e = ghost_ref).
+template <typename R>
+__device__ __forceinline__ void put_v(const GridDev<R> &gd, R *__restrict__ Vn, int64_t g, uint8_t ctl, int32_t e, R v)
+{
+    Vn[g] = v;
+    if (ctl & kCtlGhost) {
+        if (e >= 0) {
+            Vn[e] = v;
+        } else {
+            for (int32_t j = ~e;; ++j) {
+                const int32_t d = gd.glist[j];
+                Vn[d & 0x7fffffff] = v;
+                if (d < 0) break;
+            }
+        }
+    }
+}
+
+// The clock of the step after the one from grid cur (one thread of the launch).
+template <typename R> __device__ __forceinline__ void advance_clock(const GridDev<R> &gd, int cur)
+{
+    Clock ck = gd.clk[cur];
+    ck.step += 1;
+    ck.time += gd.dt;
+    ck.time_f = (float)ck.time;
+    int32_t w = ck.widx < 0 ? 0 : ck.widx;
+    const int32_t nwin = gd.win ? gd.nwin : 0;
+    while (w < nwin && ck.step >= gd.win[w].off) ++w;
+    ck.widx = w;
+    ck.s1_on = w < nwin && ck.step >= gd.win[w].on;
+    ck.opened = w < nwin && ck.step == gd.win[w].on;
+    ck.s2_on = ck.step >= gd.s2_win.on && ck.step < gd.s2_win.off;
+    if (gd.onset) {
+        ck.tb = ck.time - floor(ck.time / gd.bcl) * gd.bcl;
+        ck.s1_cycle_ok = gd.s1_beats <= 0 || floor(ck.time / gd.bcl) < gd.s1_beats;
+    }
+    gd.clk[cur ^ 1] = ck;
+}
+
 // One plain step of tissue voxel k: diffusion, stimulus, the TPORd update,
 // the new V, the detector and the blow-up count.
-template <typename R, int DIM>
+template <typename R, int DIM, bool FOLD>
 __device__ __forceinline__ void grid_step_voxel(const GridDev<R> &gd, const StepT<R> &kst, int cur, int64_t k,
                                                 const Clock &ck)
 {
     const R *__restrict__ V = gd.vg[cur];
     R *__restrict__ Vn = gd.vg[cur ^ 1];
     const int64_t g = DIM == 1 ? k : (int64_t)gd.gidx[k];
-    const R vc = V[g];
-    const R du = grid_du<R, DIM>(gd, V, g, k, vc);
     const uint8_t ctl = gd.ctl[k];
+    const R vc = V[g];
+    const int32_t gref = FOLD ? ghost_ref(gd, k, ctl) : 0;
+    const R du = grid_du<R, DIM>(gd, V, g, k, vc);
     const R ist = grid_stim(gd, ck, ctl, k);
 
     CellState<R> c;
@@ -166,7 +220,8 @@ __device__ __forceinline__ void grid_step_voxel(const GridDev<R> &gd, const Step
     StepOut<R> o{};
     tpord_update(c, ctl & kCtlType, gd.model, kst, ist, du, &o);
     store_cell(c, gd.s, k);
-    Vn[g] = c.v;
+    if (FOLD) put_v(gd, Vn, g, ctl, gref, c.v);
+    else Vn[g] = c.v;
     if (gd.det) grid_detect(gd, ck, k, (float)vc, (float)c.v, (float)o.dvdt);
     grid_count_bad(gd, c.v);
 }
@@ -177,19 +232,40 @@ template <typename R, int DIM>
 __device__ __noinline__ void grid_step_voxel_call(const GridDev<R> &gd, const StepT<R> &kst, int cur, int64_t k,
                                                   const Clock &ck)
 {
-    grid_step_voxel<R, DIM>(gd, kst, cur, k, ck);
+    grid_step_voxel<R, DIM, false>(gd, kst, cur, k, ck);
 }
 
-// MINB = minimum resident CTAs per SM the register allocation must allow
-// (occupancy variants picked at run time by the autotuner in api_sim.cu; they
-// differ only in register allocation, not in arithmetic).  One thread per
-// tissue voxel.
-template <typename R, int DIM, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_grid_step(GridDev<R> gd, StepT<R> kst, int cur)
+// BS = CTA width, MINB = minimum resident CTAs per SM the register allocation
+// must allow (occupancy variants; they differ only in register allocation, not
+// in arithmetic).  One thread per tissue voxel.  FOLD: mirror voxels and clock
+// (by one more block, so that no voxel waits for it) belong to this launch.
+template <typename R, int DIM, int MINB, int BS, bool FOLD>
+__global__ void __launch_bounds__(BS, MINB) k_grid_step(GridDev<R> gd, StepT<R> kst, int cur)
 {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (FOLD && blockIdx.x == 0) {
+        if (threadIdx.x == 0) advance_clock(gd, cur);
+        return;
+    }
+    const int64_t k = (blockIdx.x - (FOLD ? 1 : 0)) * (int64_t)BS + threadIdx.x;
     if (k >= gd.ntissue) return;
-    grid_step_voxel<R, DIM>(gd, kst, cur, k, *gd.clk);
+    grid_step_voxel<R, DIM, FOLD>(gd, kst, cur, k, gd.clk[cur]);
+}
+
+// A launch of k_grid_step with CTAs of BS threads.
+template <typename R, int DIM, int MINB, int BS, bool FOLD = false>
+cudaError_t grid_step_launch(const GridDev<R> &gd, const StepT<R> &kk, int cur, cudaStream_t st)
+{
+    const int64_t nb = (gd.ntissue + BS - 1) / BS + (FOLD ? 1 : 0);
+    k_grid_step<R, DIM, MINB, BS, FOLD><<<(unsigned)nb, BS, 0, st>>>(gd, kk, cur);
+    return cudaGetLastError();
+}
+
+inline int grid_sms()
+{
+    int dev = 0, nsm = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
 }
 
 // With the learned surrogate attached: the plain step of the voxels listed in
@@ -204,7 +280,7 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_list(GridDev<R> gd, StepT<
     const int64_t n = *gd.plist_n;
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const Clock ck = *gd.clk;
+    const Clock ck = gd.clk[cur];
     for (; i < n; i += (int64_t)gridDim.x * blockDim.x) grid_step_voxel_call<R, DIM>(gd, kst, cur, gd.plist[i], ck);
 }
 
@@ -212,11 +288,8 @@ __global__ void __launch_bounds__(256, 2) k_grid_step_list(GridDev<R> gd, StepT<
 // thread per tissue voxel.
 inline unsigned grid_list_blocks(int64_t ntissue)
 {
-    int dev = 0, nsm = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int64_t full = (ntissue + 255) / 256;
-    const int64_t cap = (int64_t)nsm * 2 * 4;
+    const int64_t cap = (int64_t)grid_sms() * 2 * 4;
     return (unsigned)(full < cap ? (full < 1 ? 1 : full) : cap);
 }
 
@@ -326,7 +399,7 @@ __global__ void __launch_bounds__(256, MINB) k_sur_substep(GridDev<float> gd, fl
         any |= on[u];
     }
     if (!any) return;
-    const Clock ck = *gd.clk;
+    const Clock ck = gd.clk[cur];
     const float *__restrict__ V = gd.vg[cur];
     float *__restrict__ Vn = gd.vg[cur ^ 1];
 #pragma unroll
@@ -345,32 +418,14 @@ __global__ void __launch_bounds__(256, MINB) k_sur_substep(GridDev<float> gd, fl
     }
 }
 
-// Mirror-boundary refresh of the new grid, then the clock advance for the
-// next step (block 0, thread 0).
-template <typename R>
-__global__ void __launch_bounds__(256) k_ghost(GridDev<R> gd, int nxt)
+// Mirror-boundary refresh of grid cur ^ 1, which a step from grid cur has
+// written, and the clock's advance (clock = 0: the refresh alone).
+template <typename R> __global__ void __launch_bounds__(256) k_ghost(GridDev<R> gd, int cur, int clock)
 {
-    R *V = gd.vg[nxt];
+    R *V = gd.vg[cur ^ 1];
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < gd.nbnd; j += (int64_t)gridDim.x * blockDim.x)
         V[gd.bnd_dst[j]] = V[gd.bnd_src[j]];
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        Clock ck = *gd.clk;
-        ck.step += 1;
-        ck.time += gd.dt;
-        ck.time_f = (float)ck.time;
-        int32_t w = ck.widx < 0 ? 0 : ck.widx;
-        const int32_t nwin = gd.win ? gd.nwin : 0;
-        while (w < nwin && ck.step >= gd.win[w].off) ++w;
-        ck.widx = w;
-        ck.s1_on = w < nwin && ck.step >= gd.win[w].on;
-        ck.opened = w < nwin && ck.step == gd.win[w].on;
-        ck.s2_on = ck.step >= gd.s2_win.on && ck.step < gd.s2_win.off;
-        if (gd.onset) {
-            ck.tb = ck.time - floor(ck.time / gd.bcl) * gd.bcl;
-            ck.s1_cycle_ok = gd.s1_beats <= 0 || floor(ck.time / gd.bcl) < gd.s1_beats;
-        }
-        *gd.clk = ck;
-    }
+    if (clock && blockIdx.x == 0 && threadIdx.x == 0) advance_clock(gd, cur);
 }
 
 // Compensated FP32 sum (hi, lo) += x: TwoSum of hi and x, error folded into lo.

@@ -14,12 +14,12 @@ template <> cudaError_t launch_grid_step<float>(const GridDev<float> &gd, const 
     return launch_grid_step_minb<float>(gd, step_as<float>(k), cur, dim, minb, st);
 }
 
-template <> cudaError_t launch_ghost<float>(const GridDev<float> &gd, int nxt, cudaStream_t st)
+template <> cudaError_t launch_ghost<float>(const GridDev<float> &gd, int cur, int clock, cudaStream_t st)
 {
     int64_t nb = (gd.nbnd + 255) / 256;
     if (nb < 1) nb = 1;
     if (nb > 152 * 16) nb = 152 * 16;
-    k_ghost<float><<<(unsigned)nb, 256, 0, st>>>(gd, nxt);
+    k_ghost<float><<<(unsigned)nb, 256, 0, st>>>(gd, cur, clock);
     return cudaGetLastError();
 }
 
@@ -31,7 +31,7 @@ cudaError_t launch_ecg<float>(const GridDev<float> &gd, int cur, const float4 *e
     if (dim == 1) k_ecg_partial<float, 1><<<(unsigned)nb, 256, 0, st>>>(gd, gd.vg[cur], el, nel, partial);
     else if (dim == 2) k_ecg_partial<float, 2><<<(unsigned)nb, 256, 0, st>>>(gd, gd.vg[cur], el, nel, partial);
     else k_ecg_partial<float, 3><<<(unsigned)nb, 256, 0, st>>>(gd, gd.vg[cur], el, nel, partial);
-    k_ecg_final<<<nel, 256, 0, st>>>(partial, nb, nel, out, t_out, counter, cap, gd.clk);
+    k_ecg_final<<<nel, 256, 0, st>>>(partial, nb, nel, out, t_out, counter, cap, gd.clk + cur);
     return cudaGetLastError();
 }
 

@@ -15,9 +15,8 @@ template <> cudaError_t launch_grid_step_minb<float>(const GridDev<float> &gd, c
         k_grid_step_list<float, 1><<<grid_list_blocks(gd.ntissue), 256, 0, st>>>(gd, kk, cur);
         return cudaGetLastError();
     }
-    const unsigned nb = (unsigned)((gd.ntissue + 255) / 256);
-    k_grid_step<float, 1, 2><<<nb, 256, 0, st>>>(gd, kk, cur);
-    return cudaGetLastError();
+    if (gd.fold) return grid_step_launch<float, 1, 4, 64, true>(gd, kk, cur, st);
+    return grid_step_launch<float, 1, 2, 256>(gd, kk, cur, st);
 }
 
 }  // namespace lqt

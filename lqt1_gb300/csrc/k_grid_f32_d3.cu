@@ -10,11 +10,10 @@ cudaError_t launch_f32_d3(const GridDev<float> &gd, const StepT<float> &kk, int 
         k_grid_step_list<float, 3><<<grid_list_blocks(gd.ntissue), 256, 0, st>>>(gd, kk, cur);
         return cudaGetLastError();
     }
-    const unsigned nb = (unsigned)((gd.ntissue + 255) / 256);
-    if (minb >= 4) k_grid_step<float, 3, 4><<<nb, 256, 0, st>>>(gd, kk, cur);
-    else if (minb == 3) k_grid_step<float, 3, 3><<<nb, 256, 0, st>>>(gd, kk, cur);
-    else k_grid_step<float, 3, 2><<<nb, 256, 0, st>>>(gd, kk, cur);
-    return cudaGetLastError();
+    if (gd.fold) return grid_step_launch<float, 3, 4, 64, true>(gd, kk, cur, st);
+    if (minb >= 4) return grid_step_launch<float, 3, 4, 256>(gd, kk, cur, st);
+    if (minb == 3) return grid_step_launch<float, 3, 3, 256>(gd, kk, cur, st);
+    return grid_step_launch<float, 3, 2, 256>(gd, kk, cur, st);
 }
 
 }  // namespace lqt

@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
     uint32_t phase = 0;
     bool net_ok = true;
 
-    const Clock ck = *gd.clk;
+    const Clock ck = gd.clk[cur];
     const float *__restrict__ V = gd.vg[cur];
     const float *__restrict__ Vp = gd.vg[cur ^ 1];
     const float inv_dt = sg.inv_dt, inv_mac = sg.inv_mac;

@@ -156,8 +156,9 @@ class Sim:
 
     def profile(self, nsteps: int = 20):
         """Mean device ms per launch of the fused step kernel, of the ghost
-        kernel and (with a surrogate attached) of the surrogate macro-step
-        kernel, 0 when none ran (CUDA events on the simulation's stream)."""
+        kernel (0 on small grids, whose step kernel does its work) and (with a
+        surrogate attached) of the surrogate macro-step kernel, 0 when none ran
+        (CUDA events on the simulation's stream)."""
         L = N.lib()
         L.lqt_sim_profile.argtypes = [C.c_void_p, C.c_int64] + [C.POINTER(C.c_double)] * 3
         a, b, c = C.c_double(), C.c_double(), C.c_double()

@@ -357,13 +357,17 @@ int lqt_sim_get_ecg(lqt_sim *s, int64_t max_samples, double *phi_host,
 int lqt_sim_get_detect(lqt_sim *s, float *t_act_host, float *apd90_host,
                        uint8_t *ead_host);
 
-/* Occupancy variant of the fused step kernel: the minimum resident CTAs/SM its
- * register allocation allows (mixed form 2, 3, 4; FP64 1, 2).  variant >= 0
- * forces one; variant < 0 runs the autotuner now (15 real steps, the variants
- * in turn, each timed with CUDA events, the fastest kept; with a surrogate
- * attached, 15 more steps pick the variant of the V-only substep kernel).  The
- * first lqt_sim_step call with nsteps >= 64 autotunes by itself unless a
- * variant was forced.  All variants give bit-identical results.
+/* Variant of the fused step kernel: the minimum resident CTAs/SM its register
+ * allocation allows (mixed form 2, 3, 4; FP64 1, 2), or 100: persistent warps
+ * that copy the next tile's state into shared memory while they step one (mixed
+ * form, 2D and 3D).  variant >= 0 forces one; variant < 0 runs the autotuner
+ * now (real steps, the variants in turn, five rounds, each timed with CUDA
+ * events, the fastest kept; with a surrogate attached, five more rounds pick
+ * the variant of the V-only substep kernel).  The first lqt_sim_step call of at
+ * least 64 steps, and of no fewer than the rounds take, autotunes by itself
+ * unless a variant was forced.  Small grids (at most 512 voxels per SM) in the
+ * mixed form use a kernel of their own unless a variant is forced.  All variants
+ * give bit-identical results.
  * ms_per_variant: up to 4 timings (or NULL). */
 int lqt_sim_tune(lqt_sim *s, int32_t variant, int32_t *chosen, float *ms_per_variant);
 

@@ -436,12 +436,12 @@ int step_once(lqt_sim *s)
 // The variants take turns step by step, so each sees the same phases of the
 // simulation (with a surrogate attached, the share of plain voxels changes
 // from one macro step to the next); the first round only loads the modules.
-// The variants differ only in register allocation, so the steps are valid
-// simulation steps whichever variant runs them.  Returns the steps consumed.
+// The variants give the same bits, so the steps are valid simulation steps
+// whichever variant runs them.  Returns the steps consumed.
 int autotune(lqt_sim *s, int per, int64_t *consumed)
 {
     const int *cand = s->fp64() ? kGridVariantsF64 : kGridVariantsF32;
-    const int ncand = s->dim == 1 ? 1 : (s->fp64() ? 2 : 3);
+    const int ncand = s->dim == 1 ? 1 : (s->fp64() ? 2 : kGridNVariantsF32);
     cudaEvent_t a, b;
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
@@ -895,7 +895,9 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
         if (rc) return rc;
     }
     int64_t left = nsteps;
-    if (!s->tuned && left >= 64) {
+    // (a call shorter than the autotuner's steps does not start it)
+    const int64_t tune_steps = 5 * ((s->fp64() ? 2 : kGridNVariantsF32) + (s->sur ? kSubNVariants : 0));
+    if (!s->tuned && left >= std::max<int64_t>(64, tune_steps)) {
         int64_t used = 0;
         int rc = autotune(s, 5, &used);
         if (rc) return rc;
@@ -1182,10 +1184,10 @@ int lqt_sim_tune(lqt_sim *s, int32_t variant, int32_t *chosen, float *ms_per_var
     if (!s) return fail(LQT_ERR_INVALID, "lqt_sim_tune: NULL handle");
     if (variant >= 0) {
         const int *cand = s->fp64() ? kGridVariantsF64 : kGridVariantsF32;
-        const int ncand = s->fp64() ? 2 : 3;
+        const int ncand = s->fp64() ? 2 : kGridNVariantsF32;
         bool ok = false;
         for (int c = 0; c < ncand; ++c) ok |= cand[c] == variant;
-        if (!ok) return fail(LQT_ERR_INVALID, "lqt_sim_tune: variant must be 2, 3 or 4 (mixed) or 1, 2 (FP64)");
+        if (!ok) return fail(LQT_ERR_INVALID, "lqt_sim_tune: variant must be 2, 3, 4 or 100 (mixed) or 1, 2 (FP64)");
         s->minb = variant;
         s->step_forced = true;
         s->tuned = true;

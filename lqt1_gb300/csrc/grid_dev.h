@@ -104,8 +104,11 @@ constexpr int kVBoxMaxCols = 64;
 constexpr int kSubTile = 256;
 inline int64_t pad_tiles(int64_t n) { return (n + kSubTile - 1) / kSubTile * kSubTile; }
 
-// Occupancy variants of k_grid_step: minimum CTAs/SM of 256 threads.
-constexpr int kGridVariantsF32[3] = {2, 3, 4};
+// Variants of the plain step: minimum CTAs/SM of 256 threads of k_grid_step,
+// and (mixed form, 2D and 3D) the pipelined k_grid_step_pipe.
+constexpr int kGridPipe = 100;
+constexpr int kGridNVariantsF32 = 4;
+constexpr int kGridVariantsF32[kGridNVariantsF32] = {2, 3, 4, kGridPipe};
 constexpr int kGridVariantsF64[2] = {1, 2};
 
 template <typename R>

@@ -23,8 +23,47 @@
 
 #include "common.cuh"
 #include "grid_dev.h"
+#include "tc.cuh"
 
 namespace lqt {
+
+// FP32 products that enter a sum, rounded by themselves, and explicit FMAs: the
+// diffusion term has one rounding whatever kernel it is inlined into (as the
+// cell step, tpord_f32.cuh).
+template <typename R> __device__ __forceinline__ R du_mul(R a, R b)
+{
+    if constexpr (sizeof(R) == 4) return __fmul_rn(a, b);
+    else return a * b;
+}
+template <typename R> __device__ __forceinline__ R du_fma(R a, R b, R c)
+{
+    if constexpr (sizeof(R) == 4) return fmaf(a, b, c);
+    else return a * b + c;
+}
+
+// The anisotropic stencil with the tensor (xx yy zz xy xz yz) and its
+// divergence at hand, on any x-major array of V with strides sx, sy (z stride
+// 1): the dense grid, or a tile's box of it staged in shared memory.
+template <int DIM>
+__device__ __forceinline__ float sub_du_at(const GridDev<float> &gd, const float *__restrict__ V, int64_t g,
+                                           int64_t sx, int64_t sy, float vc, const float *Dt, const float *Bt)
+{
+    const float vxp = V[g + sx], vxm = V[g - sx], vyp = V[g + sy], vym = V[g - sy];
+    const float c2 = gd.inv_dx2, c4 = gd.inv_4dx2, c1 = gd.inv_2dx;
+    const float lxx = (vxp + vxm - 2.f * vc) * c2;
+    const float lyy = (vyp + vym - 2.f * vc) * c2;
+    const float lxy = (V[g + sx + sy] + V[g - sx - sy] - V[g - sx + sy] - V[g + sx - sy]) * c4;
+    float du = fmaf(Dt[0], lxx, fmaf(Dt[1], lyy, __fmul_rn(2.f * Dt[3], lxy)));
+    du = fmaf(Bt[0], (vxp - vxm) * c1, fmaf(Bt[1], (vyp - vym) * c1, du));
+    if constexpr (DIM == 3) {
+        const float vzp = V[g + 1], vzm = V[g - 1];
+        const float lzz = (vzp + vzm - 2.f * vc) * c2;
+        const float lxz = (V[g + sx + 1] + V[g - sx - 1] - V[g - sx + 1] - V[g + sx - 1]) * c4;
+        const float lyz = (V[g + sy + 1] + V[g - sy - 1] - V[g - sy + 1] - V[g + sy - 1]) * c4;
+        du = fmaf(Dt[2], lzz, fmaf(2.f, fmaf(Dt[4], lxz, __fmul_rn(Dt[5], lyz)), fmaf(Bt[2], (vzp - vzm) * c1, du)));
+    }
+    return du;
+}
 
 // du = sum_i D_ii V_ii + 2 sum_{i<j} D_ij V_ij + sum_j b_j V_j
 // (new_11.cu:352-417 in 2D; 7-point D*lap(V) when isotropic, GPU3D.cu:370-385).
@@ -49,18 +88,21 @@ __device__ __forceinline__ R grid_du(const GridDev<R> &gd, const R *__restrict__
             fo = (vp - vm) * gd.inv_2dx;
             so = (vp + vm - (R)2 * vc) * gd.inv_dx2;
         }
-        return (R)gd.dcoeff[k] * fo + (R)gd.coeff[k] * so;
+        return du_fma((R)gd.dcoeff[k], fo, du_mul((R)gd.coeff[k], so));
     } else {
         const int64_t sx = gd.sx, sy = gd.sy;
+        if constexpr (sizeof(R) == 4) {
+            if (gd.d6) return sub_du_at<DIM>(gd, V, g, sx, sy, vc, gd.d6 + 6 * k, gd.b3 + 3 * k);
+        }
         const R vxp = V[g + sx], vxm = V[g - sx], vyp = V[g + sy], vym = V[g - sy];
         const R c2 = gd.inv_dx2;
-        const R lxx = (vxp + vxm - (R)2 * vc) * c2;
-        const R lyy = (vyp + vym - (R)2 * vc) * c2;
+        const R lxx = du_mul(vxp + vxm - (R)2 * vc, c2);
+        const R lyy = du_mul(vyp + vym - (R)2 * vc, c2);
         R lzz = 0, vzp = 0, vzm = 0;
         if constexpr (DIM == 3) {
             vzp = V[g + 1];
             vzm = V[g - 1];
-            lzz = (vzp + vzm - (R)2 * vc) * c2;
+            lzz = du_mul(vzp + vzm - (R)2 * vc, c2);
         }
         if (!gd.d6) return gd.diso * (lxx + lyy + lzz);
         const R *D = gd.d6 + 6 * k;
@@ -268,6 +310,146 @@ inline int grid_sms()
     return nsm;
 }
 
+// ---- the plain step with its state staged ahead (mixed form, 2D and 3D) -----
+// One thread per voxel loads 45 state values, waits for them, computes and
+// stores: at the 64 to 80 registers that fit enough warps the step spills, and
+// with 128 too few loads are in flight.  Here persistent warps take tiles of 32
+// voxels and copy the next tile's state and tensor rows into shared memory
+// (16-byte cp.async past L1, which stays with the V rows) while they step the
+// current one: the loads in flight need no registers, the step gets 128 of them
+// and reads a value where it uses it.  A warp's stages are its own, so a tile
+// needs no barrier beyond the warp's.  Measured per step (GB300) against the
+// best of the 2, 3 and 4 CTAs/SM variants of k_grid_step: 1.12 M-voxel shell
+// 107 -> 90 us, 6.3 M 547 -> 472 us (5.8 TB/s), 600 x 600 sheet 32.7 -> 27.7 us;
+// at 90,000 voxels (one or two tiles per warp) 12.4 and 12.8 us.
+constexpr int kPipeRows = 16 + 29;                       // concentrations (hi, lo), evolving gates
+constexpr int kPipeWarps = 8, kPipeCtas = 2;             // per CTA, CTAs per SM
+struct __align__(16) PipeStage {
+    float st[kPipeRows][32];
+    float d6[32 * 6];
+    float b3[32 * 3];
+};
+constexpr uint32_t kPipeSmem = 2 * kPipeWarps * sizeof(PipeStage);
+static_assert(kPipeCtas * (kPipeSmem + 1024) <= 228 * 1024, "stages of the CTAs of an SM");
+
+__device__ __forceinline__ void pipe_cp16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// This lane's share of the copies of tile k0 (a multiple of 32): rows of 128
+// bytes, four rows per instruction.  The state arrays hold whole groups of 128
+// voxels and the tensor whole tiles of 256, so every copy is in bounds.
+__device__ __forceinline__ void pipe_issue(PipeStage &s, const GridDev<float> &gd, int64_t k0, int lane)
+{
+    const int64_t ld = gd.s.ld;
+    const int row = lane >> 3, part = (lane & 7) * 4;
+    const float *c = reinterpret_cast<const float *>(gd.s.conc) + row * ld + k0 + part;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pipe_cp16(&s.st[4 * i + row][part], c + 4 * i * ld);
+    // gate slots 3 and 4 (hsp, jp) never change: rows 0..2, then 5..30
+    const float *g = gd.s.gate + row * ld + k0 + part;
+    pipe_cp16(&s.st[16 + row][part], g + (row == 3 ? 2 * ld : 0));
+#pragma unroll
+    for (int i = 1; i < 7; ++i) pipe_cp16(&s.st[16 + 4 * i + row][part], g + (4 * i + 2) * ld);
+    if (lane < 8) pipe_cp16(&s.st[44][part], g + 30 * ld);
+    if (gd.d6) {
+        const float *d = gd.d6 + 6 * k0, *b = gd.b3 + 3 * k0;
+        pipe_cp16(&s.d6[4 * lane], d + 4 * lane);
+        if (lane < 16) pipe_cp16(&s.d6[128 + 4 * lane], d + 128 + 4 * lane);
+        else if (lane < 24) pipe_cp16(&s.b3[64 + 4 * (lane - 16)], b + 64 + 4 * (lane - 16));
+        else pipe_cp16(&s.b3[4 * (lane - 24)], b + 4 * (lane - 24));
+        if (lane < 8) pipe_cp16(&s.b3[32 + 4 * lane], b + 32 + 4 * lane);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ void pipe_load(CellState<float> &c, const PipeStage &s, int lane)
+{
+    float2 *cp[8] = {&c.nai, &c.nass, &c.ki, &c.kss, &c.cai, &c.cass, &c.cansr, &c.cajsr};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) *cp[j] = make_float2(s.st[j][lane], s.st[8 + j][lane]);
+    float *gp[29] = {&c.sm, &c.sh, &c.sj, &c.mL, &c.hL, &c.hLp, &c.a, &c.iF, &c.iS, &c.ap, &c.iFp, &c.iSp, &c.d, &c.ff, &c.fs,
+                     &c.fcaf, &c.fcas, &c.jca, &c.nca, &c.ffp, &c.fcafp, &c.xrf, &c.xrs, &c.xs1, &c.xs2, &c.xk1,
+                     &c.Jrelnp, &c.Jrelp, &c.CaMKt};
+#pragma unroll
+    for (int j = 0; j < 29; ++j) *gp[j] = s.st[16 + j][lane];
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kPipeWarps * 32, kPipeCtas) k_grid_step_pipe(GridDev<float> gd, StepT<float> kst, int cur)
+{
+    extern __shared__ __align__(16) uint8_t pipe_sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    PipeStage *stg = reinterpret_cast<PipeStage *>(pipe_sm) + 2 * warp;
+    const int64_t n = gd.ntissue, stride = (int64_t)gridDim.x * kPipeWarps * 32;
+    int64_t k0 = ((int64_t)blockIdx.x * kPipeWarps + warp) * 32;
+    if (k0 >= n) return;
+    const Clock ck = gd.clk[cur];
+    const float *__restrict__ V = gd.vg[cur];
+    float *__restrict__ Vn = gd.vg[cur ^ 1];
+    pipe_issue(stg[0], gd, k0, lane);
+    int64_t k = k0 + lane;
+    int32_t g = k < n ? gd.gidx[k] : 0;
+    uint8_t ctl = k < n ? gd.ctl[k] : 0;
+    for (int s = 0; k0 < n; k0 += stride, s ^= 1) {
+        const int64_t kn = k0 + stride + lane;
+        int32_t g_next = 0;
+        uint8_t ctl_next = 0;
+        if (k0 + stride < n) {
+            pipe_issue(stg[s ^ 1], gd, k0 + stride, lane);
+            if (kn < n) {
+                g_next = gd.gidx[kn];
+                ctl_next = gd.ctl[kn];
+            }
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();                      // every lane's copies of this stage have landed
+        k = k0 + lane;
+        if (k < n) {
+            const PipeStage &st = stg[s];
+            const float vc = V[g];
+            const float4 det = gd.det ? gd.det[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+            float du;
+            if (gd.d6) {
+                float Dt[6], Bt[3];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) Dt[i] = st.d6[6 * lane + i];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) Bt[i] = st.b3[3 * lane + i];
+                du = sub_du_at<DIM>(gd, V, g, gd.sx, gd.sy, vc, Dt, Bt);
+            } else {
+                du = grid_du<float, DIM>(gd, V, g, k, vc);
+            }
+            const float ist = grid_stim(gd, ck, ctl, k);
+            CellState<float> c;
+            pipe_load(c, st, lane);
+            c.v = vc;
+            StepOut<float> o{};
+            tpord_update(c, ctl & kCtlType, gd.model, kst, ist, du, &o);
+            store_cell(c, gd.s, k);
+            Vn[g] = c.v;
+            if (gd.det) grid_detect_rec(gd, ck, k, det, vc, c.v, o.dvdt);
+            grid_count_bad(gd, c.v);
+        }
+        __syncwarp();                      // the stage is read before the next copies into it
+        g = g_next;
+        ctl = ctl_next;
+    }
+}
+
+template <int DIM> cudaError_t grid_step_pipe_launch(const GridDev<float> &gd, const StepT<float> &kk, int cur, cudaStream_t st)
+{
+    static std::atomic<uint64_t> done{0};
+    cudaError_t e = tc::smem_attr_once(k_grid_step_pipe<DIM>, kPipeSmem, done);
+    if (e != cudaSuccess) return e;
+    const int64_t need = (gd.ntissue + kPipeWarps * 32 - 1) / (kPipeWarps * 32), cap = (int64_t)grid_sms() * kPipeCtas;
+    k_grid_step_pipe<DIM><<<(unsigned)(need < cap ? need : cap), kPipeWarps * 32, kPipeSmem, st>>>(gd, kk, cur);
+    return cudaGetLastError();
+}
+
 // With the learned surrogate attached: the plain step of the voxels listed in
 // plist (plist_n of them, written by the macro-step kernel), grid-stride over
 // a launch of a few waves of CTAs, so that a short list costs its own voxels
@@ -329,30 +511,6 @@ __device__ __forceinline__ void sub_tensor_unpack(const float2 (&q)[3], float dt
     Bt[2] = DIM == 3 ? q[2].y : 0.f;
 }
 
-// The anisotropic stencil of grid_du with the tensor already loaded, on any
-// x-major array of V with strides sx, sy (z stride 1): the dense grid, or a
-// tile's box of it staged in shared memory (the same values in the same
-// order of operations, so the same bits).
-template <int DIM>
-__device__ __forceinline__ float sub_du_at(const GridDev<float> &gd, const float *__restrict__ V, int64_t g,
-                                           int64_t sx, int64_t sy, float vc, const float *Dt, const float *Bt)
-{
-    const float vxp = V[g + sx], vxm = V[g - sx], vyp = V[g + sy], vym = V[g - sy];
-    const float c2 = gd.inv_dx2, c4 = gd.inv_4dx2, c1 = gd.inv_2dx;
-    const float lxx = (vxp + vxm - 2.f * vc) * c2;
-    const float lyy = (vyp + vym - 2.f * vc) * c2;
-    const float lxy = (V[g + sx + sy] + V[g - sx - sy] - V[g - sx + sy] - V[g + sx - sy]) * c4;
-    float du = Dt[0] * lxx + Dt[1] * lyy + 2.f * Dt[3] * lxy + Bt[0] * ((vxp - vxm) * c1) + Bt[1] * ((vyp - vym) * c1);
-    if constexpr (DIM == 3) {
-        const float vzp = V[g + 1], vzm = V[g - 1];
-        const float lzz = (vzp + vzm - 2.f * vc) * c2;
-        const float lxz = (V[g + sx + 1] + V[g - sx - 1] - V[g - sx + 1] - V[g + sx - 1]) * c4;
-        const float lyz = (V[g + sy + 1] + V[g - sy - 1] - V[g - sy + 1] - V[g + sy - 1]) * c4;
-        du += Dt[2] * lzz + 2.f * (Dt[4] * lxz + Dt[5] * lyz) + Bt[2] * ((vzp - vzm) * c1);
-    }
-    return du;
-}
-
 template <int DIM>
 __device__ __forceinline__ float sub_du(const GridDev<float> &gd, const float *__restrict__ V, int64_t g, int64_t k,
                                         float vc, const float *Dt, const float *Bt)
@@ -410,7 +568,7 @@ __global__ void __launch_bounds__(256, MINB) k_sur_substep(GridDev<float> gd, fl
         const float du = sub_du<DIM>(gd, V, g[u], k, vc, Dt[u], Bt[u]);
         const float ist = grid_stim(gd, ck, ctl[u], k);
         const float dvdt = r[u] - ist;
-        const float vn = vc + (dvdt + du) * dt;
+        const float vn = fmaf(dvdt + du, dt, vc);
         Vn[g[u]] = vn;
         if (fl[u]) grid_detect(gd, ck, k, vc, vn, dvdt);
         const bool bad = !(vn == vn) || vn < gd.vmin_ok || vn > gd.vmax_ok;

@@ -11,6 +11,7 @@ cudaError_t launch_f32_d3(const GridDev<float> &gd, const StepT<float> &kk, int 
         return cudaGetLastError();
     }
     if (gd.fold) return grid_step_launch<float, 3, 4, 64, true>(gd, kk, cur, st);
+    if (minb >= kGridPipe) return grid_step_pipe_launch<3>(gd, kk, cur, st);
     if (minb >= 4) return grid_step_launch<float, 3, 4, 256>(gd, kk, cur, st);
     if (minb == 3) return grid_step_launch<float, 3, 3, 256>(gd, kk, cur, st);
     return grid_step_launch<float, 3, 2, 256>(gd, kk, cur, st);

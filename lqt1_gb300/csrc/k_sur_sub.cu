@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kSubTile, MINB) k_sur_substep_tile(GridDev<flo
             const float du = sub_du<DIM>(gd, V, g, k, vc, Dt, Bt);
             const float ist = grid_stim(gd, ck, sg.ctl[t], k);
             const float dvdt = r - ist;
-            const float vn = vc + (dvdt + du) * dt;
+            const float vn = fmaf(dvdt + du, dt, vc);
             Vn[g] = vn;
             if (det && sg.flag[t]) grid_detect(gd, ck, k, vc, vn, dvdt);
             const bool bad = !(vn == vn) || vn < gd.vmin_ok || vn > gd.vmax_ok;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kSubTile + 32, MINB) k_sur_substep_vbox(GridDe
             }
             const float ist = grid_stim(gd, ck, sg.ctl[t], k);
             const float dvdt = r - ist;
-            const float vn = vc + (dvdt + du) * dt;
+            const float vn = fmaf(dvdt + du, dt, vc);
             Vn[g] = vn;
             if (det && sg.flag[t]) grid_detect(gd, ck, k, vc, vn, dvdt);
             const bool bad = !(vn == vn) || vn < gd.vmin_ok || vn > gd.vmax_ok;
@@ -353,7 +353,7 @@ template <int DIM> __global__ void __launch_bounds__(64, 4) k_sur_step_small(Gri
     const float du = sub_du<DIM>(gd, V, g, k, vc, Dt, Bt);
     const float ist = grid_stim(gd, ck, ctl, k);
     const float dvdt = r - ist;
-    const float vn = vc + (dvdt + du) * kst.dt;
+    const float vn = fmaf(dvdt + du, kst.dt, vc);
     put_v(gd, gd.vg[cur ^ 1], g, ctl, gref, vn);
     if (fl) grid_detect(gd, ck, k, vc, vn, dvdt);
     if (!(vn == vn) || vn < gd.vmin_ok || vn > gd.vmax_ok) atomicAdd(gd.nbad, 1ull);

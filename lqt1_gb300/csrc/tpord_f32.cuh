@@ -52,6 +52,12 @@ __device__ __forceinline__ float rcpf_(float x)
 
 constexpr double kLog2e = 1.4426950408889634;
 
+// A product that enters a sum, rounded by itself: with every other sum of
+// products written as an FMA the step has one rounding whatever kernel it is
+// inlined into (left to the compiler, which of two products is fused changes
+// from kernel to kernel, and with it last bits).
+__device__ __forceinline__ float mulp(float a, float b) { return __fmul_rn(a, b); }
+
 // exp((v + a) / k): the offset is formed from the rounded slope, so that the
 // slope's rounding acts on v + a and not on v.
 __device__ __forceinline__ float exva(float v, double a, double k)
@@ -66,7 +72,7 @@ __device__ __forceinline__ float sigva(float v, double a, double k) { return rcp
 // x -> inf - (inf - x) exp(-rate dt), ndtl = -dt log2(e)
 __device__ __forceinline__ float relaxf(float x, float inf, float rate, float ndtl)
 {
-    return inf - (inf - x) * ex2f_(ndtl * rate);
+    return fmaf(x - inf, ex2f_(ndtl * rate), inf);
 }
 
 __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, const ModelT<float> &m,
@@ -116,7 +122,7 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
     // TP06 fast INa, TPORd.cc:465-504
     {
         // 1/(AM BM), AM = 1/(1+a), BM = 0.1/(1+b) + 0.1/(1+e); a b = exp(-5)
-        const float a = 6.14421235332821e-6f * I5;               // exp((-60 - v)/5)
+        const float a = mulp(6.14421235332821e-6f, I5);               // exp((-60 - v)/5)
         const float b = fminf(1096.6331584284585f * E5, 1e18f);  // exp((v + 35)/5)
         const float e = exva(v, -50, 200);
         const float rate_m = 10.0f * ((1.0067379469990854f + a) + b) * (1.0f + e) * rcpf_((2.0f + b) + e);
@@ -125,19 +131,19 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         float rate_h, rate_j;   // 1/tau
         if (v >= -40.0f) {
             const float x = 1.0f + exva(v, 10.66, -11.1);
-            const float y = 1.0f + 0.04076220397836621f * I10;   // 1 + exp(-0.1 (v + 32))
+            const float y = fmaf(0.04076220397836621f, I10, 1.0f);   // 1 + exp(-0.1 (v + 32))
             const float r = rcpf_(x * y);
             rate_h = (float)(0.77 / 0.13) * (y * r);
             rate_j = 0.6f * ex2f_(v * (float)(0.057 * kLog2e)) * (x * r);
         } else {
-            rate_h = 0.057f * exva(v, 80, -6.8) +
-                     (2.7f * ex2f_(v * (float)(0.079 * kLog2e)) + 3.1e5f * ex2f_(v * (float)(0.3485 * kLog2e)));
-            const float n1 = (-2.5428e4f * ex2f_(v * (float)(0.2444 * kLog2e)) -
-                              6.948e-6f * ex2f_(v * (float)(-0.04391 * kLog2e))) * (v + 37.78f);
+            rate_h = fmaf(0.057f, exva(v, 80, -6.8), fmaf(2.7f, ex2f_(v * (float)(0.079 * kLog2e)),
+                                                          3.1e5f * ex2f_(v * (float)(0.3485 * kLog2e))));
+            const float n1 = fmaf(-2.5428e4f, ex2f_(v * (float)(0.2444 * kLog2e)),
+                                  -6.948e-6f * ex2f_(v * (float)(-0.04391 * kLog2e))) * (v + 37.78f);
             const float n2 = 0.02424f * ex2f_(v * (float)(-0.01052 * kLog2e));
             const float x = 1.0f + exva(v, 79.23, 1.0 / 0.311);
             const float y = 1.0f + fminf(exva(v, 40.14, -1.0 / 0.1378), 1e18f);
-            rate_j = (n1 * y + n2 * x) * rcpf_(x * y);
+            rate_j = fmaf(n1, y, n2 * x) * rcpf_(x * y);
         }
         const float eh = 1.0f + exva(v, 71.55, 7.43);
         const float H_INF = rcpf_(eh * eh);
@@ -145,40 +151,41 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         c.sh = relaxf(c.sh, H_INF, rate_h, ndtl);
         c.sj = relaxf(c.sj, H_INF, rate_j, ndtl);
     }
-    const float INa = 14.838f * c.sm * c.sm * c.sm * c.sh * c.sj * (v - ENa);
+    const float INa = mulp(14.838f * c.sm * c.sm * c.sm * c.sh * c.sj, v - ENa);
 
     // INaL, TPORd.cc:509-528
     const float mLss = sigva(v, 42.85, -5.264);
-    const float rate_mL = 6.765f * exva(v, 11.64, 34.77) + 8.552f * exva(v, 77.42, -5.955);
+    const float rate_mL = fmaf(6.765f, exva(v, 11.64, 34.77), 8.552f * exva(v, 77.42, -5.955));
     c.mL = relaxf(c.mL, mLss, rate_mL, ndtl);
     {
         const float x = fminf(exva(v, 87.61, 7.488), 1e18f);
-        const float p = 1.0f + x, q = 1.0f + 2.288717124596482f * x;   // exp((v + 93.81)/7.488)
+        const float p = 1.0f + x, q = fmaf(2.288717124596482f, x, 1.0f);   // exp((v + 93.81)/7.488)
         const float r = rcpf_(p * q);
-        c.hL = q * r - (q * r - c.hL) * k.e_hl;
-        c.hLp = p * r - (p * r - c.hLp) * k.e_hlp;
+        const float hLss = mulp(q, r), hLssp = mulp(p, r);
+        c.hL = fmaf(c.hL - hLss, k.e_hl, hLss);
+        c.hLp = fmaf(c.hLp - hLssp, k.e_hlp, hLssp);
     }
     const float GNaL = epi ? (float)(0.0075 * 0.6) : 0.0075f;
-    const float INaL = GNaL * (v - ENa) * c.mL * ((1.0f - fP) * c.hL + fP * c.hLp);
+    const float INaL = mulp(GNaL * (v - ENa) * c.mL, fmaf(1.0f - fP, c.hL, fP * c.hLp));
 
     // Ito, TPORd.cc:530-571
     {
         const float x = exva(v, -14.34, -14.82);
-        const float p = 1.0f + x, q = 1.0f + 1.9635691902911017f * x;   // exp(-(v - 24.34)/14.82)
+        const float p = 1.0f + x, q = fmaf(1.9635691902911017f, x, 1.0f);   // exp(-(v - 24.34)/14.82)
         const float r = rcpf_(p * q);
-        const float ass = q * r, assp = p * r;
+        const float ass = mulp(q, r), assp = mulp(p, r);
         // 1/ta from its two terms over one denominator
         const float y = 1.0f + exva(v, -18.4099, -29.3814), z = 1.0f + exva(v, 100, 29.3814);
-        const float rate_a = ((float)(1.0 / (1.2089 * 1.0515)) * z + (float)(3.5 / 1.0515) * y) * rcpf_(y * z);
+        const float rate_a = fmaf((float)(1.0 / (1.2089 * 1.0515)), z, (float)(3.5 / 1.0515) * y) * rcpf_(y * z);
         const float e_ta = ex2f_(ndtl * rate_a);
-        c.a = ass - (ass - c.a) * e_ta;
-        c.ap = assp - (assp - c.ap) * e_ta;
+        c.a = fmaf(c.a - ass, e_ta, ass);
+        c.ap = fmaf(c.ap - assp, e_ta, assp);
     }
     const float iss = sigva(v, 43.94, 5.711);
     {
         // tiF = (4.562 + 1/sF) delta, tiS = (23.62 + 1/sS) delta
-        const float sF = fminf(0.3933f * exva(v, 100, -100) + 0.08004f * exva(v, 50, 16.59), 1e12f);
-        const float sS = fminf(0.001416f * exva(v, 96.52, -59.05) + 1.780e-8f * exva(v, 114.1, 8.079), 1e12f);
+        const float sF = fminf(fmaf(0.3933f, exva(v, 100, -100), 0.08004f * exva(v, 50, 16.59)), 1e12f);
+        const float sS = fminf(fmaf(0.001416f, exva(v, 96.52, -59.05), 1.780e-8f * exva(v, 114.1, 8.079)), 1e12f);
         const float dF = fmaf(4.562f, sF, 1.0f), dS = fmaf(23.62f, sS, 1.0f);
         // delta = 1 - 0.95/(1 + z) in the epicardium, else 1
         const float z = fminf(1202604.2841647768f * E5, 1e10f);   // exp((v + 70)/5)
@@ -195,22 +202,22 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         c.iSp = relaxf(c.iSp, iss, rS * f, ndtl);
     }
     const float AiF = sigva(v, -213.6, 151.2);
-    const float ii = AiF * c.iF + (1.0f - AiF) * c.iS;
-    const float ip = AiF * c.iFp + (1.0f - AiF) * c.iSp;
+    const float ii = fmaf(AiF, c.iF, (1.0f - AiF) * c.iS);
+    const float ip = fmaf(AiF, c.iFp, (1.0f - AiF) * c.iSp);
     const float Gto = (epi || mid) ? (float)(0.02 * 4.0) : 0.02f;
-    const float Ito = Gto * (v - EK) * ((1.0f - fP) * c.a * ii + fP * c.ap * ip);
+    const float Ito = mulp(Gto * (v - EK), fmaf((1.0f - fP) * c.a, ii, fP * c.ap * ip));
 
     // ICaL, ICaNa, ICaK, TPORd.cc:573-652
     {
         const float dss = rcpf_(1.0f + ex2f_((v + (3.940f + m.dss_shift)) * (float)(-kLog2e / 4.230)));
-        const float s = fminf(0.7408182206817179f * I20 + exva(v, 14, 1.0 / 0.09), 1e12f);   // exp(-0.05 (v + 6))
+        const float s = fminf(fmaf(0.7408182206817179f, I20, exva(v, 14, 1.0 / 0.09)), 1e12f);   // exp(-0.05 (v + 6))
         c.d = relaxf(c.d, dss, s * rcpf_(fmaf(0.6f, s, 1.0f)), ndtl);
     }
     const float fss = rcpf_(1.0f + ex2f_((v + (19.58f + m.fss_shift)) * (float)(kLog2e / 3.696)));   // = fcass
     const float E7 = ex2f_(v * (float)(kLog2e / 7.0)), I7 = ex2f_(v * (float)(-kLog2e / 7.0));
     {
         // tff = 7 + 1/sf, tfs = 1000 + 1/ss
-        const float sf = fminf((float)(0.0045 * 0.1353352832366127) * I10 + (float)(0.0045 * 7.38905609893065) * E10, 1e12f);
+        const float sf = fminf(fmaf((float)(0.0045 * 0.1353352832366127), I10, (float)(0.0045 * 7.38905609893065) * E10), 1e12f);
         const float ss = fminf(0.000035f * (exva(v, 5, -4) + exva(v, 5, 6)), 1e12f);
         const float df = fmaf(7.0f, sf, 1.0f), ds = fmaf(1000.0f, ss, 1.0f);
         const float r = rcpf_(df * ds);
@@ -221,7 +228,7 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
     }
     {
         // tfcaf = 7 + 1/sf, tfcas = 100 + 1/ss
-        const float sf = fminf((float)(0.04 * 1.770794952435155) * I7 + (float)(0.04 * 0.5647181220077593) * E7, 1e12f);
+        const float sf = fminf(fmaf((float)(0.04 * 1.770794952435155), I7, (float)(0.04 * 0.5647181220077593) * E7), 1e12f);
         const float ss = fminf(0.00012f * (ex2f_(v * (float)(-kLog2e / 3.0)) + E7), 1e12f);
         const float df = fmaf(7.0f, sf, 1.0f), ds = fmaf(100.0f, ss, 1.0f);
         const float r = rcpf_(df * ds);
@@ -232,14 +239,15 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
     }
     const float Afcaf = fmaf(0.6f, rcpf_(fmaf(0.36787944117144233f, E10, 1.0f)), 0.3f);   // exp((v - 10)/10)
     const float Afcas = 1.0f - Afcaf;
-    c.jca = fss - (fss - c.jca) * k.e_jca;
+    c.jca = fmaf(c.jca - fss, k.e_jca, fss);
     {
         const float q = fmaf(0.002f, rcass, 1.0f), q2 = q * q;
         const float nss = rcpf_(fmaf(1.0e-3f * c.jca, q2 * q2, 1.0f));   // anca k2n / km2n
         c.nca = relaxf(c.nca, nss, c.jca, ndtl);
     }
-    const float f = 0.6f * c.ff + 0.4f * c.fs, fp = 0.6f * c.ffp + 0.4f * c.fs;
-    const float fca = Afcaf * c.fcaf + Afcas * c.fcas, fcap = Afcaf * c.fcafp + Afcas * c.fcas;
+    const float fs4 = mulp(0.4f, c.fs), fcs = mulp(Afcas, c.fcas);
+    const float f = fmaf(0.6f, c.ff, fs4), fp = fmaf(0.6f, c.ffp, fs4);
+    const float fca = fmaf(Afcaf, c.fcaf, fcs), fcap = fmaf(Afcaf, c.fcafp, fcs);
     float PhiCaL, PhiCaNa, PhiCaK, INab_phi, ICab_phi;
     {
         // em1 = e^x - 1, x = v F / RT
@@ -253,32 +261,33 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         p = fmaf(x * x, p, x);
         const float em1 = fabsf(x) < 0.5f ? p : ex2f_(x * (float)kLog2e) - 1.0f;
         const float e1 = em1 + 1.0f, e1p = e1 + 1.0f;
-        const float e2m1 = em1 * e1p, e2 = e2m1 + 1.0f;
+        const float e2m1 = mulp(em1, e1p), e2 = e2m1 + 1.0f;
         // vffrt/(e1 - 1) = F x/(e^x - 1) and vffrt/(e2 - 1), 1 - x/2 near 0
         const float r = rcpf_(e2m1) * x;
         const bool tiny = fabsf(x) < 1e-4f;
-        const float g1 = (float)F_ * (tiny ? 1.0f - 0.5f * x : r * e1p);
-        const float g2 = (float)F_ * (tiny ? 0.5f - 0.5f * x : r);
-        PhiCaL = 4.0f * g2 * (cass * e2 - (float)(0.341 * cao));
-        PhiCaNa = g1 * (0.75f * nass * e1 - (float)(0.75 * nao));
-        PhiCaK = g1 * (0.75f * kss * e1 - (float)(0.75 * ko));
-        INab_phi = g1 * (nai * e1 - (float)nao);
-        ICab_phi = 4.0f * g2 * (cai * e2 - (float)(0.341 * cao));
+        const float g1 = (float)F_ * (tiny ? fmaf(-0.5f, x, 1.0f) : r * e1p);
+        const float g2 = (float)F_ * (tiny ? fmaf(-0.5f, x, 0.5f) : r);
+        PhiCaL = 4.0f * g2 * fmaf(cass, e2, (float)(-0.341 * cao));
+        PhiCaNa = g1 * fmaf(0.75f * nass, e1, (float)(-0.75 * nao));
+        PhiCaK = g1 * fmaf(0.75f * kss, e1, (float)(-0.75 * ko));
+        INab_phi = g1 * fmaf(nai, e1, (float)-nao);
+        ICab_phi = 4.0f * g2 * fmaf(cai, e2, (float)(-0.341 * cao));
     }
     const float PCa = epi ? m.pca[1] : (mid ? m.pca[2] : m.pca[0]);
-    const float gate_np = c.d * (f * (1.0f - c.nca) + c.jca * fca * c.nca);
-    const float gate_p = c.d * (fp * (1.0f - c.nca) + c.jca * fcap * c.nca);
+    const float jn = c.jca * c.nca;
+    const float gate_np = c.d * fmaf(f, 1.0f - c.nca, fca * jn);
+    const float gate_p = c.d * fmaf(fp, 1.0f - c.nca, fcap * jn);
     // (1 - fP) PCa gate_np + fP (1.1 PCa) gate_p, shared by the three fluxes
-    const float G = PCa * ((1.0f - fP) * gate_np + 1.1f * fP * gate_p);
-    const float ICaL = G * PhiCaL;
-    const float ICaNa = 0.00125f * G * PhiCaNa;
-    const float ICaK = 3.574e-4f * G * PhiCaK;
+    const float G = PCa * fmaf(1.0f - fP, gate_np, 1.1f * fP * gate_p);
+    const float ICaL = mulp(G, PhiCaL);
+    const float ICaNa = mulp(0.00125f * G, PhiCaNa);
+    const float ICaK = mulp(3.574e-4f * G, PhiCaK);
 
     // IKr, TPORd.cc:654-678 (sqrt(ko/5.4) = 1)
     const float xrss = sigva(v, 8.337, -6.789);
     {
-        const float sf = fminf(0.3652f * exva(v, -31.66, 3.869) + 4.123e-5f * exva(v, -47.78, -20.38), 1e12f);
-        const float ss = fminf(0.06629f * exva(v, -34.70, 7.355) + 1.128e-5f * exva(v, -29.74, -25.94), 1e12f);
+        const float sf = fminf(fmaf(0.3652f, exva(v, -31.66, 3.869), 4.123e-5f * exva(v, -47.78, -20.38)), 1e12f);
+        const float ss = fminf(fmaf(0.06629f, exva(v, -34.70, 7.355), 1.128e-5f * exva(v, -29.74, -25.94)), 1e12f);
         const float df = fmaf(12.98f, sf, 1.0f), ds = fmaf(1.865f, ss, 1.0f);
         const float r = rcpf_(df * ds);
         c.xrf = relaxf(c.xrf, xrss, sf * ds * r, ndtl);
@@ -289,25 +298,25 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         const float p = 1.0f + exva(v, 54.81, 38.21);
         const float q = (1.0f + exva(v, 55, 75)) * (1.0f + exva(v, -10, 30));
         const float r = rcpf_(p * q);
-        const float Axrf = q * r, rkr = p * r;
-        const float xr = Axrf * c.xrf + (1.0f - Axrf) * c.xrs;
+        const float Axrf = mulp(q, r), rkr = p * r;
+        const float xr = fmaf(Axrf, c.xrf, (1.0f - Axrf) * c.xrs);
         const float GKr = epi ? (float)(0.046 * 1.3) : (mid ? (float)(0.046 * 0.8) : 0.046f);
-        IKr = GKr * xr * rkr * (v - EK);
+        IKr = mulp(GKr * xr * rkr, v - EK);
     }
 
     // IKs, TPORd.cc:680-735
     const float xs1ss = sigva(v, 11.60, -8.932);
     {
-        const float s = fminf(2.326e-4f * exva(v, 48.28, 17.80) + 0.001292f * exva(v, 210, -230), 1e12f);
+        const float s = fminf(fmaf(2.326e-4f, exva(v, 48.28, 17.80), 0.001292f * exva(v, 210, -230)), 1e12f);
         c.xs1 = relaxf(c.xs1, xs1ss, s * rcpf_(fmaf(817.3f, s, 1.0f)), ndtl);
-        const float rate2 = (float)(0.01 * 0.0820849986238988) * E20 + 0.0193f * exva(v, 66.54, -31);
+        const float rate2 = fmaf((float)(0.01 * 0.0820849986238988), E20, 0.0193f * exva(v, 66.54, -31));
         c.xs2 = relaxf(c.xs2, xs1ss, rate2, ndtl);
     }
     // 1 + 0.6/(1 + (3.8e-5/cai)^1.4)
     constexpr double lg_ks = -14.683641055880589;   // log2(3.8e-5)
     const float KsCa = fmaf(0.6f, rcpf_(1.0f + ex2f_(1.4f * ((float)lg_ks - lg2f_(cai)))), 1.0f);
     const float GKs = epi ? m.gks[1] : (mid ? m.gks[2] : m.gks[0]);
-    const float IKs = GKs * KsCa * c.xs1 * c.xs2 * (v - EKs);
+    const float IKs = mulp(GKs * KsCa * c.xs1 * c.xs2, v - EKs);
 
     // IK1, TPORd.cc:738-751 (sqrt(ko) constant)
     float rk1;
@@ -317,10 +326,10 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         const float r = rcpf_(x * y);
         rk1 = x * r;
         const float rate = (float)(1.0 / 122.2) * (exva(v, 127.2, -20.36) + exva(v, 236.8, 69.33));
-        c.xk1 = relaxf(c.xk1, y * r, rate, ndtl);
+        c.xk1 = relaxf(c.xk1, mulp(y, r), rate, ndtl);
     }
     const float GK1 = epi ? (float)(0.1908 * 1.2) : (mid ? (float)(0.1908 * 1.3) : 0.1908f);
-    const float IK1 = GK1 * 2.32379000772445f /* sqrt(ko) */ * rk1 * c.xk1 * (v - EK);
+    const float IK1 = mulp(GK1 * 2.32379000772445f /* sqrt(ko) */ * rk1 * c.xk1, v - EK);
 
     // INaCa_i and INaCa_ss, TPORd.cc:753-852
     constexpr double kna1 = 15.0, kna2 = 5.0, kna3 = 88.12, kasymm = 12.5;
@@ -334,9 +343,9 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
     // h8 = nao/(kna3 hna h7), h9 = 1/h7 with h7 = 1 + nao/kna3 (1 + 1/hna)
     const float r7 = rcpf_(fmaf(hna, (float)(kna3 + nao), (float)nao));
     const float h8 = (float)nao * r7;
-    const float k3pp = h8 * (float)wnaca;
-    const float k3 = (float)(kna3 * wca) * hna * r7 + k3pp;
-    const float k8 = h8 * (float)(h11 * wna);
+    const float k3pp = mulp(h8, (float)wnaca);
+    const float k3 = fmaf((float)(kna3 * wca) * hna, r7, k3pp);
+    const float k8 = mulp(h8, (float)(h11 * wna));
     const float Gncx = epi ? (float)(0.0008 * 1.1) : (mid ? (float)(0.0008 * 1.4) : 0.0008f);
     const float hna1 = (1.0f + hna) * (float)(1.0 / kna3);
     float INaCa_i, INaCa_ss;
@@ -350,22 +359,23 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         const float h3 = h4 * r14, h6 = h1 * r14;      // 1/h1, 1/h4
         const float h2 = na * hna * (float)(1.0 / kna3) * h3;
         const float h5 = na * na * (float)(1.0 / (kna1 * kna2)) * h6;
-        const float k4pp = h2 * (float)wnaca;
-        const float k4 = h3 * (float)wca * ihca + k4pp;
-        const float k6 = h6 * ca * (float)kcaon;
-        const float k7 = h5 * h2 * (float)wna;
+        const float k4pp = mulp(h2, (float)wnaca);
+        const float k4 = fmaf(h3 * (float)wca, ihca, k4pp);
+        const float k6 = mulp(h6 * ca, (float)kcaon);
+        const float k7 = mulp(h5 * h2, (float)wna);
         const float k67 = k6 + k7, k23 = k2 + k3, k45 = k4 + k2, k18 = (float)k1 + k8;
-        const float x1 = k2 * (k4 * k67 + k7 * k23);
-        const float x2 = (float)k1 * k7 * k45 + k4 * k6 * k18;
-        const float x3 = (float)k1 * k3 * k67 + k8 * k6 * k23;
-        const float x4 = k2 * (k8 * k45 + k3 * k18);
+        const float x1 = mulp(k2, fmaf(k4, k67, k7 * k23));
+        const float x2 = fmaf((float)k1 * k7, k45, k4 * k6 * k18);
+        const float x3 = fmaf((float)k1 * k3, k67, k8 * k6 * k23);
+        const float x4 = mulp(k2, fmaf(k8, k45, k3 * k18));
         const float xs = (x1 + x2) + (x3 + x4);
         // J = (3 (x4 k7 - x1 k8) + x3 k4pp - x2 k3pp + 2 (x2 k2 - x1 k1)) / xs; allo = ca^2/(ca^2 + KmCaAct^2)
-        const float num = 3.0f * (x4 * k7 - x1 * k8) + x3 * k4pp - x2 * k3pp + 2.0f * (x2 * k2 - x1 * (float)k1);
-        const float ca2 = ca * ca;
+        const float a = fmaf(x4, k7, -mulp(x1, k8)), b = fmaf(x2, k2, -mulp(x1, (float)k1));
+        const float num = fmaf(2.0f, b, fmaf(3.0f, a, fmaf(x3, k4pp, -mulp(x2, k3pp))));
+        const float ca2 = mulp(ca, ca);
         const float val = Gncx * num * ca2 * rcpf_(xs * (ca2 + (float)(150.0e-6 * 150.0e-6)));
-        if (pass == 0) INaCa_i = 0.8f * val;
-        else INaCa_ss = 0.2f * val;
+        if (pass == 0) INaCa_i = mulp(0.8f, val);
+        else INaCa_ss = mulp(0.2f, val);
     }
     const float INaCa = INaCa_i + INaCa_ss;
 
@@ -378,53 +388,54 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         constexpr double Kki = 0.5, Kko = 0.3582, MgADP = 0.05, MgATP = 9.8, Kmgatp = 1.698e-7;
         constexpr double H = 1.0e-7, eP = 4.2, Khp = 1.698e-7, Knap = 224.0, Kxkur = 292.0;
         constexpr double rko = ko / Kko;
-        const float rnai = nai * (float)(1.0 / Knai0) * ex2f_(v * (float)(-delta / 3.0 * FRT * kLog2e));
-        const float rnao = (float)(nao / Knao0) * ex2f_(v * (float)(-(1.0 - delta) / 3.0 * FRT * kLog2e));
-        const float rki = ki * (float)(1.0 / Kki);
-        const float pP = (float)(1.0 + H / Khp) + nai * (float)(1.0 / Knap) + ki * (float)(1.0 / Kxkur);   // eP/P
+        const float rnai = mulp(nai * (float)(1.0 / Knai0), ex2f_(v * (float)(-delta / 3.0 * FRT * kLog2e)));
+        const float rnao = mulp((float)(nao / Knao0), ex2f_(v * (float)(-(1.0 - delta) / 3.0 * FRT * kLog2e)));
+        const float rki = mulp(ki, (float)(1.0 / Kki));
+        const float pP = fmaf(ki, (float)(1.0 / Kxkur), fmaf(nai, (float)(1.0 / Knap), (float)(1.0 + H / Khp)));   // eP/P
         const float pnai = 1.0f + rnai, pnao = 1.0f + rnao, pki = 1.0f + rki;
-        const float den_i = pnai * pnai * pnai + (pki * pki - 1.0f);
-        const float den_o = pnao * pnao * pnao + (float)((1.0 + rko) * (1.0 + rko) - 1.0);
+        const float den_i = fmaf(pnai * pnai, pnai, fmaf(pki, pki, -1.0f));
+        const float den_o = fmaf(pnao * pnao, pnao, (float)((1.0 + rko) * (1.0 + rko) - 1.0));
         const float rio = rcpf_(den_i * den_o);
         const float ri = den_o * rio, ro = den_i * rio;
-        const float a1 = (float)k1p * (rnai * rnai * rnai) * ri;
-        const float b4 = (float)k4m * (rki * rki) * ri;
-        const float b2 = (float)k2m * (rnao * rnao * rnao) * ro;
-        const float a3 = (float)(k3p_ * rko * rko) * ro;
-        const float b3 = (float)(k3m * H / (1.0 + MgATP / Kmgatp) * eP) * rcpf_(pP);
+        const float a1 = mulp((float)k1p * (rnai * rnai * rnai), ri);
+        const float b4 = mulp((float)k4m * (rki * rki), ri);
+        const float b2 = mulp((float)k2m * (rnao * rnao * rnao), ro);
+        const float a3 = mulp((float)(k3p_ * rko * rko), ro);
+        const float b3 = mulp((float)(k3m * H / (1.0 + MgATP / Kmgatp) * eP), rcpf_(pP));
         constexpr float b1 = (float)(k1m * MgADP), a2 = (float)k2p;
         constexpr float a4 = (float)((k4p_ * MgATP / Kmgatp) / (1.0 + MgATP / Kmgatp));
-        const float y1 = a2 * (a1 * (a4 + b3) + b4 * b3) + b2 * b4 * b3;
-        const float y2 = b1 * b4 * (b2 + a3) + a2 * a3 * (a1 + b4);
-        const float y3 = a3 * a4 * (a2 + b1) + b1 * b2 * (b3 + a4);
-        const float y4 = b2 * b3 * (b4 + a1) + a4 * a1 * (a3 + b2);
-        const float J = 3.0f * (y1 * a3 - y2 * b3) + 2.0f * (y4 * b1 - y3 * a1);
+        const float b43 = mulp(b4, b3), b23 = mulp(b2, b3);
+        const float y1 = fmaf(a2, fmaf(a1, a4 + b3, b43), b2 * b43);
+        const float y2 = fmaf(b1 * b4, b2 + a3, a2 * a3 * (a1 + b4));
+        const float y3 = fmaf(a3 * a4, a2 + b1, b1 * b2 * (b3 + a4));
+        const float y4 = fmaf(b23, b4 + a1, a4 * a1 * (a3 + b2));
+        const float J = fmaf(3.0f, fmaf(y1, a3, -mulp(y2, b3)), 2.0f * fmaf(y4, b1, -mulp(y3, a1)));
         const float Pnak = epi ? (float)(30 * 0.9) : (mid ? (float)(30 * 0.7) : 30.0f);
-        INaK = Pnak * J * rcpf_((y1 + y2) + (y3 + y4));
+        INaK = mulp(Pnak * J, rcpf_((y1 + y2) + (y3 + y4)));
     }
 
     // background currents and pump, TPORd.cc:908-923
     const float GKb = epi ? (float)(0.003 * 0.6) : 0.003f;
-    const float IKb = GKb * sigva(v, -14.48, -18.34) * (v - EK);
-    const float INab = 3.75e-10f * INab_phi;
-    const float ICab = 2.5e-8f * ICab_phi;
+    const float IKb = mulp(GKb * sigva(v, -14.48, -18.34), v - EK);
+    const float INab = mulp(3.75e-10f, INab_phi);
+    const float ICab = mulp(2.5e-8f, ICab_phi);
     // cytosolic buffer and pump: Bcai = 1/(1 + cm/qc^2 + ct/qt^2), IpCa = 0.0005 cai/qt (qt = 0.0005 + cai)
     constexpr double cmdnmax = 0.05, kmcmdn = 0.00238, trpnmax = 0.07, kmtrpn = 0.0005;
     float IpCa, Bcai;
     {
         const float qc = (float)kmcmdn + cai, qt = (float)kmtrpn + cai;
-        const float qc2 = qc * qc, qt2 = qt * qt, qq = qc2 * qt2;
+        const float qc2 = mulp(qc, qc), qt2 = mulp(qt, qt), qq = mulp(qc2, qt2);
         const float cm = epi ? (float)(1.3 * cmdnmax * kmcmdn) : (float)(cmdnmax * kmcmdn);
-        const float D = qq + cm * qt2 + (float)(trpnmax * kmtrpn) * qc2;
+        const float D = fmaf((float)(trpnmax * kmtrpn), qc2, fmaf(cm, qt2, qq));
         const float r = rcpf_(D * qt);
         Bcai = qq * (r * qt);
-        IpCa = 0.0005f * cai * (r * D);
+        IpCa = mulp(0.0005f * cai, r * D);
     }
 
     // membrane potential, TPORd.cc:927-935
     const float Iion = INa + INaL + Ito + ICaL + ICaNa + ICaK + IKr + IKs + IK1 + INaCa + INaK + INab + IKb + IpCa + ICab;
     const float dV_dt = -(Iion + Ist);
-    c.v = v + (dV_dt + dVgap_dt) * dt;
+    c.v = fmaf(dV_dt + dVgap_dt, dt, v);
     if (out) {
         out->dvdt = dV_dt;
         out->ical = ICaL;
@@ -435,52 +446,51 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
     }
 
     // CaMK and fluxes, TPORd.cc:939-995
-    c.CaMKt += dt * (0.05f * CaMKb * CaMKa - 0.00068f * c.CaMKt);
+    c.CaMKt = fmaf(dt, fmaf(0.05f * CaMKb, CaMKa, -mulp(0.00068f, c.CaMKt)), c.CaMKt);
     // concentration differences from the full-precision values (file comment of tpord.cuh)
-    const float JdiffNa = cdiff(c.nass, c.nai) * 0.5f;
-    const float JdiffK = cdiff(c.kss, c.ki) * 0.5f;
-    const float Jdiff = cdiff(c.cass, c.cai) * 5.0f;
-    const float Jtr = cdiff(c.cansr, c.cajsr) * 0.01f;
+    const float JdiffNa = mulp(cdiff(c.nass, c.nai), 0.5f);
+    const float JdiffK = mulp(cdiff(c.kss, c.ki), 0.5f);
+    const float Jdiff = mulp(cdiff(c.cass, c.cai), 5.0f);
+    const float Jtr = mulp(cdiff(c.cansr, c.cajsr), 0.01f);
     {
         // 1/(1 + (1.5/cajsr)^8) and 1/cajsr from one reciprocal
-        const float j2 = cajsr * cajsr, j4 = j2 * j2, j8 = j4 * j4;
+        const float j2 = cajsr * cajsr, j4 = j2 * j2, j8 = mulp(j4, j4);
         const float dj = j8 + 25.62890625f;
         const float r = rcpf_(dj * cajsr);
         const float rel = (mid ? 1.7f : 1.0f) * -ICaL * j8 * (r * cajsr);
         const float rate = fmaf((float)(0.0123 / 4.75), r * dj, (float)(1.0 / 4.75));   // 1/tau_rel, tau_rel >= 0.005
-        const float Jrel_inf = (float)(0.5 * 4.75) * rel, Jrel_infp = (float)(0.5 * 1.25 * 4.75) * rel;
+        const float Jrel_inf = mulp((float)(0.5 * 4.75), rel), Jrel_infp = mulp((float)(0.5 * 1.25 * 4.75), rel);
         c.Jrelnp = relaxf(c.Jrelnp, Jrel_inf, fminf(rate, 200.0f), ndtl);
         c.Jrelp = relaxf(c.Jrelp, Jrel_infp, fminf(0.8f * rate, 200.0f), ndtl);
     }
-    const float Jrel = (1.0f - fP) * c.Jrelnp + fP * c.Jrelp;
+    const float Jrel = fmaf(1.0f - fP, c.Jrelnp, fP * c.Jrelp);
     float Jup;
     {
         const float p = cai + 0.00092f, q = cai + (float)(0.00092 - 0.00017);
         const float s = (epi ? 1.3f : 1.0f) * cai * rcpf_(p * q);
-        Jup = s * ((1.0f - fP) * 0.004375f * q + fP * (float)(2.75 * 0.004375) * p) - (float)(0.0039375 / 15.0) * cansr;
+        const float u = fmaf((1.0f - fP) * 0.004375f, q, fP * (float)(2.75 * 0.004375) * p);
+        Jup = fmaf(s, u, -mulp((float)(0.0039375 / 15.0), cansr));
     }
 
     // concentrations, forward Euler, TPORd.cc:997-1020
-    const float dnai = -(INa + INaL + 3.0f * INaCa_i + 3.0f * INaK + INab) * (float)(Acap / (F_ * vmyo)) +
-                       JdiffNa * (float)(vss / vmyo);
-    const float dnass = -(ICaNa + 3.0f * INaCa_ss) * (float)(Acap / (F_ * vss)) - JdiffNa;
-    const float dki = -(Ito + IKr + IKs + IK1 + IKb + Ist - 2.0f * INaK) * (float)(Acap / (F_ * vmyo)) +
-                      JdiffK * (float)(vss / vmyo);
-    const float dkss = -ICaK * (float)(Acap / (F_ * vss)) - JdiffK;
-    const float dcai = Bcai * (-(IpCa + ICab - 2.0f * INaCa_i) * (float)(Acap / (2.0 * F_ * vmyo)) -
-                               Jup * (float)(vnsr / vmyo) + Jdiff * (float)(vss / vmyo));
+    constexpr float cm = (float)(Acap / (F_ * vmyo)), cs = (float)(Acap / (F_ * vss));
+    const float dnai = fmaf(-fmaf(3.0f, INaCa_i + INaK, INa + INaL + INab), cm, JdiffNa * (float)(vss / vmyo));
+    const float dnass = fmaf(-fmaf(3.0f, INaCa_ss, ICaNa), cs, -JdiffNa);
+    const float dki = fmaf(-fmaf(-2.0f, INaK, Ito + IKr + IKs + IK1 + IKb + Ist), cm, JdiffK * (float)(vss / vmyo));
+    const float dkss = fmaf(-ICaK, cs, -JdiffK);
+    const float dcai = Bcai * fmaf(-fmaf(-2.0f, INaCa_i, IpCa + ICab), 0.5f * cm,
+                                   fmaf(-Jup, (float)(vnsr / vmyo), Jdiff * (float)(vss / vmyo)));
     // Bcass and Bcajsr from one reciprocal
     constexpr double BSRmax = 0.047, KmBSR = 0.00087, BSLmax = 1.124, KmBSL = 0.0087;
     constexpr double csqnmax = 10.0, kmcsqn = 0.8;
     const float qsr = (float)KmBSR + cass, qsl = (float)KmBSL + cass, qj = (float)kmcsqn + cajsr;
-    const float qsr2 = qsr * qsr, qsl2 = qsl * qsl, qs = qsr2 * qsl2, qj2 = qj * qj;
-    const float Ds = qs + (float)(BSRmax * KmBSR) * qsl2 + (float)(BSLmax * KmBSL) * qsr2;
+    const float qsr2 = mulp(qsr, qsr), qsl2 = mulp(qsl, qsl), qs = mulp(qsr2, qsl2), qj2 = mulp(qj, qj);
+    const float Ds = fmaf((float)(BSLmax * KmBSL), qsr2, fmaf((float)(BSRmax * KmBSR), qsl2, qs));
     const float Dj = qj2 + (float)(csqnmax * kmcsqn);
     const float rsj = rcpf_(Ds * Dj);
     const float Bcass = qs * (Dj * rsj), Bcajsr = qj2 * (Ds * rsj);
-    const float dcass = Bcass * (-(ICaL - 2.0f * INaCa_ss) * (float)(Acap / (2.0 * F_ * vss)) +
-                                 Jrel * (float)(vjsr / vss) - Jdiff);
-    const float dcansr = Jup - Jtr * (float)(vjsr / vnsr);
+    const float dcass = Bcass * fmaf(-fmaf(-2.0f, INaCa_ss, ICaL), 0.5f * cs, fmaf(Jrel, (float)(vjsr / vss), -Jdiff));
+    const float dcansr = fmaf(-Jtr, (float)(vjsr / vnsr), Jup);
     const float dcajsr = Bcajsr * (Jtr - Jrel);
     cadd(c.nai, dt * dnai);
     cadd(c.nass, dt * dnass);

@@ -458,10 +458,13 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
         const float dj = j8 + 25.62890625f;
         const float r = rcpf_(dj * cajsr);
         const float rel = (mid ? 1.7f : 1.0f) * -ICaL * j8 * (r * cajsr);
-        const float rate = fmaf((float)(0.0123 / 4.75), r * dj, (float)(1.0 / 4.75));   // 1/tau_rel, tau_rel >= 0.005
+        // 1/tau_rel; tau_rel below 0.005, negative ones too (cajsr < 0), is 0.005: the
+        // sign bit makes a negative rate the larger unsigned number
+        const float rate = fmaf((float)(0.0123 / 4.75), r * dj, (float)(1.0 / 4.75));
+        auto bound = [](float x) { return __float_as_uint(x) < 0x43480000u ? x : 200.0f; };
         const float Jrel_inf = mulp((float)(0.5 * 4.75), rel), Jrel_infp = mulp((float)(0.5 * 1.25 * 4.75), rel);
-        c.Jrelnp = relaxf(c.Jrelnp, Jrel_inf, fminf(rate, 200.0f), ndtl);
-        c.Jrelp = relaxf(c.Jrelp, Jrel_infp, fminf(0.8f * rate, 200.0f), ndtl);
+        c.Jrelnp = relaxf(c.Jrelnp, Jrel_inf, bound(rate), ndtl);
+        c.Jrelp = relaxf(c.Jrelp, Jrel_infp, bound(0.8f * rate), ndtl);
     }
     const float Jrel = fmaf(1.0f - fP, c.Jrelnp, fP * c.Jrelp);
     float Jup;

@@ -52,3 +52,25 @@ def test_step_against_oracle(n, vrange, dt):
         total = np.abs(cur[:, :5]).sum(1) + np.abs(cur[:, 5]) + np.abs(v)
         dv = np.abs(got[:, 0] - ref[:, 0])
         assert np.all(dv <= 1e-5 * (np.abs(ref[:, 0] - s0[:, 0]) + dt * 4 * total + np.abs(v)) + 2e-5)
+
+
+@pytest.mark.parametrize("precision", [lq.MIXED, lq.FP64])
+@pytest.mark.parametrize("cajsr", [-0.05, -0.0124, -0.0122, -0.005, -1e-4, 1e-4, 0.005, 1.2])
+def test_release_time_constant_at_any_jsr_calcium(cajsr, precision):
+    """tau_rel = 4.75 / (1 + 0.0123 / cajsr) below 0.005 is 0.005, also where it
+    is negative (TPORd.cc:962-969); the release gates against the oracle, to a
+    few roundings of a relaxation that is complete within the step (1e-5 of the
+    steady state in FP32, 1e-12 in FP64)."""
+    s0 = orc.random_states(64, seed=9)
+    s0[:, 8] = np.float32(cajsr)
+    types = np.arange(64).astype(np.uint8) % 5
+    ref = orc.cells_update(s0.copy(), types, orc.model("default"), nsteps=1)
+    c = lq.TPORdCells(types, precision=precision, model="default")
+    c.set_state(s0)
+    c.update(1)
+    got = c.get_state()
+    c.close()
+    tol = 1e-5 if precision == lq.MIXED else 1e-12
+    for j in (37, 38):
+        scale = np.maximum(np.abs(ref[:, j]), np.abs(s0[:, j]))
+        assert np.all(np.abs(got[:, j] - ref[:, j]) <= tol * np.maximum(scale, 1e-9) * (1 if precision == lq.FP64 else 4))

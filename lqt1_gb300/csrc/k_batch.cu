@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(BatchDev<R> b, StepT<R> k)
                     ++beat;
                 }
                 StepOut<R> o{};
-                tpord_step<R>(c, ct, m, k, ist, dvgap, &o);
+                tpord_batch_update(c, ct, m, k, ist, dvgap, &o);
                 vbuf[cur ^ 1][t] = c.v;
                 if (st >= seg.vmax_from && c.v >= vmax) vmax = c.v;
 

@@ -1,13 +1,9 @@
 // tpord.cuh -- device implementation of one TPORd step (the reference's
 // TPORd::update(), SingleCell/TPORd.cc:379-1021; GPU copies GPU3D.cu:425-1220,
-// new_11.cu:459-1239) for the sm_103a kernels.
+// new_11.cu:459-1239) for the sm_103a kernels: the state types and their
+// arithmetic.
 //
-// One source serves two arithmetic forms through a precision policy (the mixed
-// form has a second, faster writing, tpord_f32.cuh):
-//   R = double : the plain FP64 form.  Divisions, exp and log follow the
-//                reference expression by expression; integer powers are
-//                multiplications and constant-tau decays are precomputed on
-//                the host (same glibc values the reference computes).
+//   R = double : the plain FP64 form (tpord_f64.cuh).
 //   R = float  : the mixed form.  Gates, currents and fluxes in FP32 with the
 //                hardware exp2/log2/rcp approximations; the eight
 //                concentrations are Kahan-compensated FP32 pairs (hi + lo,
@@ -17,6 +13,8 @@
 //                FP32 ulp of 1.5e-5 mM at 145 mM.  No FP64 instruction is left
 //                on this path: GB300 issues FP64 at about 1/64 of the FP32 rate.
 //                GHK terms use x/expm1(x), finite at V = 0.
+//                Two writings: tpord_f32.cuh for the cell, grid and surrogate
+//                kernels, and term by term below for the batch kernel.
 //
 // States hsp and jp are carried in the state vector but never change (their
 // ORd INa is commented out in SingleCell/TPORd.cc:436-460), so the step does
@@ -86,23 +84,8 @@ __device__ __forceinline__ void cadd(float2 &c, float inc)
     c.x = h;
 }
 
-// ---- math policy ----------------------------------------------------------
-template <typename R> struct Mth;
-
-template <> struct Mth<double> {
-    static __device__ __forceinline__ double ex(double x) { return exp(x); }
-    static __device__ __forceinline__ double lg(double x) { return log(x); }
-    static __device__ __forceinline__ double pw(double x, double y) { return pow(x, y); }
-    static __device__ __forceinline__ double dv(double a, double b) { return a / b; }
-    // divide by a literal: kept a true division in FP64 (reference rounding)
-    static __device__ __forceinline__ double dk(double a, double k) { return a / k; }
-    // GHK factor vffrt*(A e^z - B)/(e^z - 1) written as in TPORd.cc:618-620
-    static __device__ __forceinline__ double ghk(double vffrt, double ez, double A, double B) {
-        return vffrt * (A * ez - B) / (ez - 1.0);
-    }
-};
-
-template <> struct Mth<float> {
+// ---- FP32 math of the term-by-term writing ---------------------------------
+struct Mth {
     static __device__ __forceinline__ float ex(float x) { return __expf(x); }
     static __device__ __forceinline__ float lg(float x) { return __logf(x); }
     static __device__ __forceinline__ float pw(float x, float y) { return __powf(x, y); }
@@ -110,7 +93,7 @@ template <> struct Mth<float> {
     static __device__ __forceinline__ float dk(float a, double k) { return a * (float)(1.0 / k); }
 };
 
-// x / (e^x - 1), finite and accurate near x = 0 (FP32 form only).
+// x / (e^x - 1), finite and accurate near x = 0.
 __device__ __forceinline__ float x_over_expm1(float x, float em1)
 {
     return fabsf(x) < 1e-4f ? 1.0f - 0.5f * x : __fdividef(x, em1);
@@ -132,13 +115,14 @@ template <typename R> struct StepOut {
     R ina, ikr, ik1;   // INa, IKr, IK1 of the step (TPORd::getINa / getIKr / getIK1, TPORd.cc:365-370)
 };
 
-// One TPORd update.  ctype: 2 = EPI, 4 = MCELL, other = endocardial
+// One TPORd update, mixed form, term by term (see the note on the batch kernel
+// in tpord_f32.cuh).  ctype: 2 = EPI, 4 = MCELL, other = endocardial
 // (SingleCell/Cell.cc:20; only EPI and MCELL change parameters).
-template <typename R>
-__device__ __forceinline__ void tpord_step(CellState<R> &c, int ctype, const ModelT<R> &m, const StepT<R> &k,
-                                           R Ist, R dVgap_dt, StepOut<R> *out)
+__device__ __forceinline__ void tpord_step_terms(CellState<float> &c, int ctype, const ModelT<float> &m,
+                                                 const StepT<float> &k, float Ist, float dVgap_dt, StepOut<float> *out)
 {
-    using M = Mth<R>;
+    using R = float;
+    using M = Mth;
     const bool epi = (ctype == 2);
     const bool mid = (ctype == 4);
     const R dt = k.dt;
@@ -197,13 +181,8 @@ __device__ __forceinline__ void tpord_step(CellState<R> &c, int ctype, const Mod
         const R H_INF = M::dv((R)1, eh * eh);
         c.sm = M_INF - (M_INF - c.sm) * M::ex(M::dv(-dt, TAU_M));
         // exp(-dt/TAU) with TAU = 1/rate (TPORd.cc:475,481,488,496)
-        if constexpr (sizeof(R) == 8) {
-            c.sh = H_INF - (H_INF - c.sh) * M::ex(-dt / ((R)1 / rate_h));
-            c.sj = H_INF - (H_INF - c.sj) * M::ex(-dt / ((R)1 / rate_j));
-        } else {
-            c.sh = H_INF - (H_INF - c.sh) * M::ex(-dt * rate_h);
-            c.sj = H_INF - (H_INF - c.sj) * M::ex(-dt * rate_j);
-        }
+        c.sh = H_INF - (H_INF - c.sh) * M::ex(-dt * rate_h);
+        c.sj = H_INF - (H_INF - c.sj) * M::ex(-dt * rate_j);
     }
     const R INa = (R)14.838 * c.sm * c.sm * c.sm * c.sh * c.sj * (v - ENa);
 
@@ -287,14 +266,7 @@ __device__ __forceinline__ void tpord_step(CellState<R> &c, int ctype, const Mod
         c.nca = nss - (nss - c.nca) * M::ex(-km2n * dt);
     }
     R PhiCaL, PhiCaNa, PhiCaK, INab_phi, ICab_phi;
-    if constexpr (sizeof(R) == 8) {
-        const R e1 = exp(1.0 * vfrt), e2 = exp(2.0 * vfrt);
-        PhiCaL = 4.0 * vffrt * (cass * e2 - 0.341 * cao) / (e2 - 1.0);
-        PhiCaNa = 1.0 * vffrt * (0.75 * nass * e1 - 0.75 * nao) / (e1 - 1.0);
-        PhiCaK = 1.0 * vffrt * (0.75 * kss * e1 - 0.75 * ko) / (e1 - 1.0);
-        INab_phi = vffrt * (nai * e1 - nao) / (e1 - 1.0);
-        ICab_phi = 4.0 * vffrt * (cai * e2 - 0.341 * cao) / (e2 - 1.0);
-    } else {
+    {
         // vffrt/(e^z - 1) = (F/z_) * (z/(e^z - 1)) / z_-scaled: vffrt = F*vfrt
         const float em1 = expm1f(vfrt);
         const float e1 = em1 + 1.0f;
@@ -338,10 +310,7 @@ __device__ __forceinline__ void tpord_step(CellState<R> &c, int ctype, const Mod
                                           (R)0.001292 * M::ex(M::dk(-(v + (R)210), 230.)));
     c.xs1 = xs1ss - (xs1ss - c.xs1) * M::ex(M::dv(-dt, txs1));
     const R rate_xs2 = (R)0.01 * M::ex(M::dk(v - (R)50, 20.)) + (R)0.0193 * M::ex(M::dk(-(v + (R)66.54), 31.));
-    if constexpr (sizeof(R) == 8)
-        c.xs2 = xs1ss - (xs1ss - c.xs2) * exp(-dt / (1.0 / rate_xs2));
-    else
-        c.xs2 = xs1ss - (xs1ss - c.xs2) * M::ex(-dt * rate_xs2);
+    c.xs2 = xs1ss - (xs1ss - c.xs2) * M::ex(-dt * rate_xs2);
     const R KsCa = (R)1 + M::dv((R)0.6, (R)1 + M::pw(M::dv((R)3.8e-5, cai), (R)1.4));
     const R IKs = m.gks[cls] * KsCa * c.xs1 * c.xs2 * (v - EKs);
 
@@ -526,3 +495,4 @@ __device__ __forceinline__ void tpord_step(CellState<R> &c, int ctype, const Mod
 }  // namespace lqt
 
 #include "tpord_f32.cuh"
+#include "tpord_f64.cuh"

@@ -506,11 +506,6 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
 }
 
 // The step of the cell, grid and surrogate kernels in each form.
-__device__ __forceinline__ void tpord_update(CellState<double> &c, int ctype, const ModelT<double> &m,
-                                             const StepT<double> &k, double Ist, double dVgap_dt, StepOut<double> *out)
-{
-    tpord_step<double>(c, ctype, m, k, Ist, dVgap_dt, out);
-}
 __device__ __forceinline__ void tpord_update(CellState<float> &c, int ctype, const ModelT<float> &m,
                                              const StepT<float> &k, float Ist, float dVgap_dt, StepOut<float> *out)
 {

@@ -193,7 +193,21 @@ static int tune_batch(lqt_batch *b)
     for (auto &v : all)
         if (v.first >= b->max_strand && (b->p.threads == 0 || v.first == b->p.threads)) cand.push_back(v);
     if (cand.empty()) return fail(LQT_ERR_INVALID, "no kernel variant fits the longest strand");
-    if (cand.size() == 1) return set_items(b, cand[0].first, cand[0].second);
+    // As many SMs as items: each item has one to itself, the narrowest CTA that
+    // holds the longest strand puts the fewest cells on it, and one CTA per SM
+    // may use all the registers -- nothing to try (1000 steps of a 100-cell
+    // strand take 2.06 ms at width 128 with one CTA, 3.01 ms at the widths of
+    // more CTAs per SM; 300 cells, where only 512 fits, 3.99 ms).
+    {
+        std::pair<int, int> narrow{1 << 30, 0};
+        for (auto &v : cand)
+            if (v.first < narrow.first || (v.first == narrow.first && v.second < narrow.second)) narrow = v;
+        int dev = 0, nsm = 152;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (cand.size() == 1 || (int)make_items(b, narrow.first).size() <= nsm)
+            return set_items(b, narrow.first, narrow.second);
+    }
     const size_t rsz = b->p.precision == LQT_FP64 ? 8 : 4;
     const size_t bytes_v = b->ld * rsz, bytes_g = b->ld * rsz * kNGate, bytes_c = b->ld * 8 * kNConc;
     void *snap = nullptr;

@@ -191,13 +191,30 @@ int lqt_initial_state(double v0, double *state40_host)
 
 // ===========================================================================
 // Cells (Cell interface for N cells)
+// Up to kMappedCells cells keep what the interface sets and reads per cell
+// (inputs, V, dV/dt, currents: 10 doubles) in page-locked host memory that the
+// update kernel addresses: setting and reading are then plain memory accesses,
+// and the loop set inputs / update / read V / read currents costs its one
+// launch.  The kernel touches them once per update, over the link to the host:
+// 21 us an iteration against 56 with device arrays at 1 cell, 44 against 69 at
+// 4096, 66 against 80 at 8192, 109 against 97 at 16384.
+namespace {
+constexpr int64_t kMappedCells = 8192;
+}
+
 struct lqt_cells {
     int precision = LQT_MIXED;
     int64_t n = 0, ld = 0;
     cudaStream_t stream = nullptr;
     DevMem mem;
     uint8_t *ctype = nullptr;
-    double *ist = nullptr, *dvgap = nullptr, *dvdt = nullptr, *aos = nullptr, *cur = nullptr;
+    double *ist = nullptr, *dvgap = nullptr, *dvdt = nullptr, *aos = nullptr, *cur = nullptr;   // device addresses
+    double *vout = nullptr;
+    double *hio = nullptr;          // mapped: ist[n], dvgap[n], V[n], dV/dt[n], currents[6n]
+    ~lqt_cells()
+    {
+        if (hio) cudaFreeHost(hio);
+    }
     void *v = nullptr, *gate = nullptr;
     double *conc = nullptr;
     ModelK *modelk = nullptr;
@@ -226,10 +243,25 @@ int lqt_cells_create(int64_t n, const uint8_t *types_host, int precision, const 
     c->stream = (cudaStream_t)stream;
     c->stepk = make_stepk(dt);
     const size_t rsz = precision == LQT_FP64 ? 8 : 4;
-    rc = c->mem.alloc((void **)&c->ctype, n) | c->mem.alloc((void **)&c->ist, n * 8) |
-         c->mem.alloc((void **)&c->dvgap, n * 8) | c->mem.alloc((void **)&c->dvdt, n * 8) |
-         c->mem.alloc((void **)&c->cur, n * 6 * 8) |
-         c->mem.alloc((void **)&c->aos, n * 40 * 8) | c->mem.alloc(&c->v, c->ld * rsz) |
+    rc = 0;
+    double *io = nullptr;           // the same ten doubles per cell as the device addresses them
+    if (n <= kMappedCells) {
+        if (cudaHostAlloc((void **)&c->hio, n * 10 * 8, cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer((void **)&io, c->hio, 0) != cudaSuccess) {
+            delete c;
+            return fail(LQT_ERR_NOMEM, "lqt_cells_create: page-locked host memory");
+        }
+        std::memset(c->hio, 0, n * 10 * 8);
+        for (int64_t i = 0; i < n; ++i) c->hio[2 * n + i] = -87.5;
+    } else {
+        rc = c->mem.alloc((void **)&io, n * 10 * 8);
+    }
+    c->ist = io;
+    c->dvgap = io + n;
+    c->vout = io + 2 * n;
+    c->dvdt = io + 3 * n;
+    c->cur = io + 4 * n;
+    rc = rc | c->mem.alloc((void **)&c->ctype, n) | c->mem.alloc((void **)&c->aos, n * 40 * 8) | c->mem.alloc(&c->v, c->ld * rsz) |
          c->mem.alloc(&c->gate, c->ld * rsz * kNGate) | c->mem.alloc((void **)&c->conc, c->ld * 8 * kNConc) |
          c->mem.alloc((void **)&c->modelk, sizeof(ModelK));
     if (rc) {
@@ -241,10 +273,7 @@ int lqt_cells_create(int64_t n, const uint8_t *types_host, int precision, const 
     for (int64_t i = 0; i < n; ++i) initial_state(-87.5, &init[i * 40]);
     cudaError_t e = cudaMemcpyAsync(c->ctype, types_host, n, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->modelk, &mk, sizeof(mk), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->ist, 0, n * 8, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->dvgap, 0, n * 8, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->dvdt, 0, n * 8, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->cur, 0, n * 6 * 8, c->stream);
+    if (e == cudaSuccess && !c->hio) e = cudaMemsetAsync(io, 0, n * 10 * 8, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->aos, init.data(), n * 320, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
         e = precision == LQT_FP64 ? launch_pack<double>(c->aos, c->soa<double>(), n, c->stream)
@@ -269,6 +298,9 @@ int lqt_cells_set_state(lqt_cells *c, const double *state_host)
     CK(c->precision == LQT_FP64 ? launch_pack<double>(c->aos, c->soa<double>(), c->n, c->stream)
                                 : launch_pack<float>(c->aos, c->soa<float>(), c->n, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (c->hio)
+        for (int64_t i = 0; i < c->n; ++i)
+            c->hio[2 * c->n + i] = c->precision == LQT_FP64 ? state_host[40 * i] : (double)(float)state_host[40 * i];
     return LQT_OK;
 }
 
@@ -285,6 +317,15 @@ int lqt_cells_get_state(lqt_cells *c, double *state_host)
 int lqt_cells_set_inputs(lqt_cells *c, const double *istim_host, const double *dvgap_host)
 {
     if (!c) return fail(LQT_ERR_INVALID, "lqt_cells_set_inputs: NULL handle");
+    if (c->hio) {
+        // (no update is in flight: lqt_cells_update waits for its kernel)
+        const size_t bytes = c->n * 8;
+        if (istim_host) std::memcpy(c->hio, istim_host, bytes);
+        else std::memset(c->hio, 0, bytes);
+        if (dvgap_host) std::memcpy(c->hio + c->n, dvgap_host, bytes);
+        else std::memset(c->hio + c->n, 0, bytes);
+        return LQT_OK;
+    }
     if (istim_host) CK(cudaMemcpyAsync(c->ist, istim_host, c->n * 8, cudaMemcpyHostToDevice, c->stream));
     else CK(cudaMemsetAsync(c->ist, 0, c->n * 8, c->stream));
     if (dvgap_host) CK(cudaMemcpyAsync(c->dvgap, dvgap_host, c->n * 8, cudaMemcpyHostToDevice, c->stream));
@@ -298,10 +339,10 @@ int lqt_cells_update(lqt_cells *c, int64_t nsteps)
     if (!c || nsteps < 0) return fail(LQT_ERR_INVALID, "lqt_cells_update: NULL handle or nsteps < 0");
     if (nsteps == 0) return LQT_OK;
     CK(c->precision == LQT_FP64
-           ? launch_cells_update<double>(c->soa<double>(), c->ctype, c->ist, c->dvgap, c->dvdt, c->cur, c->modelk,
-                                         nullptr, c->stepk, c->n, nsteps, c->stream)
-           : launch_cells_update<float>(c->soa<float>(), c->ctype, c->ist, c->dvgap, c->dvdt, c->cur, c->modelk,
-                                        nullptr, c->stepk, c->n, nsteps, c->stream));
+           ? launch_cells_update<double>(c->soa<double>(), c->ctype, c->ist, c->dvgap, c->dvdt, c->cur, c->vout,
+                                         c->modelk, nullptr, c->stepk, c->n, nsteps, c->stream)
+           : launch_cells_update<float>(c->soa<float>(), c->ctype, c->ist, c->dvgap, c->dvdt, c->cur, c->vout,
+                                        c->modelk, nullptr, c->stepk, c->n, nsteps, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return LQT_OK;
 }
@@ -309,16 +350,24 @@ int lqt_cells_update(lqt_cells *c, int64_t nsteps)
 int lqt_cells_get_v(lqt_cells *c, double *v_host)
 {
     if (!c || !v_host) return fail(LQT_ERR_INVALID, "lqt_cells_get_v: NULL");
-    std::vector<double> aos((size_t)c->n * 40);
-    int rc = lqt_cells_get_state(c, aos.data());
-    if (rc) return rc;
-    for (int64_t i = 0; i < c->n; ++i) v_host[i] = aos[i * 40];
+    if (c->hio) {
+        std::memcpy(v_host, c->hio + 2 * c->n, c->n * 8);
+        return LQT_OK;
+    }
+    if (c->precision == LQT_FP64) CK((launch_gather_v<double, double>((double *)c->v, nullptr, c->vout, c->n, c->stream)));
+    else CK((launch_gather_v<float, double>((float *)c->v, nullptr, c->vout, c->n, c->stream)));
+    CK(cudaMemcpyAsync(v_host, c->vout, c->n * 8, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     return LQT_OK;
 }
 
 int lqt_cells_get_dvdt(lqt_cells *c, double *dvdt_host)
 {
     if (!c || !dvdt_host) return fail(LQT_ERR_INVALID, "lqt_cells_get_dvdt: NULL");
+    if (c->hio) {
+        std::memcpy(dvdt_host, c->hio + 3 * c->n, c->n * 8);
+        return LQT_OK;
+    }
     CK(cudaMemcpyAsync(dvdt_host, c->dvdt, c->n * 8, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return LQT_OK;
@@ -327,6 +376,10 @@ int lqt_cells_get_dvdt(lqt_cells *c, double *dvdt_host)
 int lqt_cells_get_currents(lqt_cells *c, double *currents_host)
 {
     if (!c || !currents_host) return fail(LQT_ERR_INVALID, "lqt_cells_get_currents: NULL");
+    if (c->hio) {
+        std::memcpy(currents_host, c->hio + 4 * c->n, c->n * 6 * 8);
+        return LQT_OK;
+    }
     CK(cudaMemcpyAsync(currents_host, c->cur, c->n * 6 * 8, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return LQT_OK;

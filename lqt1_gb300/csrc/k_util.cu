@@ -9,11 +9,12 @@
 
 namespace lqt {
 
+// perm (or NULL): row of the per-cell order that holds cell i.
 template <typename R>
-__global__ void k_pack(const double *__restrict__ aos, SoA<R> s, int64_t n)
+__global__ void k_pack(const double *__restrict__ aos, SoA<R> s, int64_t n, const int32_t *__restrict__ perm)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double *a = aos + i * 40;
+        const double *a = aos + (perm ? (int64_t)perm[i] : i) * 40;
         if (s.v) s.v[i] = (R)a[0];
         if (sizeof(R) == 8) {
             for (int j = 0; j < kNConc; ++j) s.conc[j * s.ld + i] = a[1 + j];
@@ -30,10 +31,10 @@ __global__ void k_pack(const double *__restrict__ aos, SoA<R> s, int64_t n)
 }
 
 template <typename R>
-__global__ void k_unpack(SoA<R> s, double *__restrict__ aos, int64_t n)
+__global__ void k_unpack(SoA<R> s, double *__restrict__ aos, int64_t n, const int32_t *__restrict__ perm)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double *a = aos + i * 40;
+        double *a = aos + (perm ? (int64_t)perm[i] : i) * 40;
         a[0] = s.v ? (double)s.v[i] : 0.0;
         if (sizeof(R) == 8) {
             for (int j = 0; j < kNConc; ++j) a[1 + j] = s.conc[j * s.ld + i];
@@ -51,22 +52,41 @@ static unsigned grid_for(int64_t n, int bs)
     return (unsigned)(nb < 1 ? 1 : (nb > 152 * 32 ? 152 * 32 : nb));
 }
 
-template <typename R> cudaError_t launch_pack(const double *aos, const SoA<R> &s, int64_t n, cudaStream_t st)
+template <typename R>
+cudaError_t launch_pack(const double *aos, const SoA<R> &s, int64_t n, cudaStream_t st, const int32_t *perm)
 {
     if (n <= 0) return cudaSuccess;
-    k_pack<R><<<grid_for(n, 256), 256, 0, st>>>(aos, s, n);
+    k_pack<R><<<grid_for(n, 256), 256, 0, st>>>(aos, s, n, perm);
     return cudaGetLastError();
 }
-template <typename R> cudaError_t launch_unpack(const SoA<R> &s, double *aos, int64_t n, cudaStream_t st)
+template <typename R>
+cudaError_t launch_unpack(const SoA<R> &s, double *aos, int64_t n, cudaStream_t st, const int32_t *perm)
 {
     if (n <= 0) return cudaSuccess;
-    k_unpack<R><<<grid_for(n, 256), 256, 0, st>>>(s, aos, n);
+    k_unpack<R><<<grid_for(n, 256), 256, 0, st>>>(s, aos, n, perm);
     return cudaGetLastError();
 }
-template cudaError_t launch_pack<double>(const double *, const SoA<double> &, int64_t, cudaStream_t);
-template cudaError_t launch_pack<float>(const double *, const SoA<float> &, int64_t, cudaStream_t);
-template cudaError_t launch_unpack<double>(const SoA<double> &, double *, int64_t, cudaStream_t);
-template cudaError_t launch_unpack<float>(const SoA<float> &, double *, int64_t, cudaStream_t);
+template cudaError_t launch_pack<double>(const double *, const SoA<double> &, int64_t, cudaStream_t, const int32_t *);
+template cudaError_t launch_pack<float>(const double *, const SoA<float> &, int64_t, cudaStream_t, const int32_t *);
+template cudaError_t launch_unpack<double>(const SoA<double> &, double *, int64_t, cudaStream_t, const int32_t *);
+template cudaError_t launch_unpack<float>(const SoA<float> &, double *, int64_t, cudaStream_t, const int32_t *);
+
+// out[perm[i]][k] = in[i][k], NaN (nothing recorded) as -1.
+__global__ void k_permute_rows(const float *__restrict__ in, const int32_t *__restrict__ perm, int64_t n, int32_t w,
+                               float *__restrict__ out)
+{
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n * w; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = e / w, k = e - i * w;
+        const float x = in[e];
+        out[(int64_t)perm[i] * w + k] = x == x ? x : -1.f;
+    }
+}
+cudaError_t launch_permute_rows(const float *in, const int32_t *perm, int64_t n, int32_t w, float *out, cudaStream_t st)
+{
+    if (n <= 0 || w <= 0) return cudaSuccess;
+    k_permute_rows<<<grid_for(n * w, 256), 256, 0, st>>>(in, perm, n, w, out);
+    return cudaGetLastError();
+}
 
 }  // namespace lqt
 

@@ -85,16 +85,19 @@ template <typename R> struct BatchDev {
 
 template <typename R>
 cudaError_t launch_cells_update(const SoA<R> &s, const uint8_t *ctype, const double *ist, const double *dvgap,
-                                double *dvdt, double *cur, const ModelK *models, const uint16_t *model_of,
-                                const StepK &k, int64_t n, int64_t nsteps, cudaStream_t stream);
+                                double *dvdt, double *cur, double *vout, const ModelK *models,
+                                const uint16_t *model_of, const StepK &k, int64_t n, int64_t nsteps, cudaStream_t stream);
 template <typename R>
 cudaError_t launch_batch(const BatchDev<R> &b, const StepK &k, int threads, int minb, int ctas, cudaStream_t stream);
 
 // AoS (reference order, double) <-> SoA conversion
+// (perm: the row of aos that holds cell i, or NULL = i)
 template <typename R>
-cudaError_t launch_pack(const double *aos, const SoA<R> &s, int64_t n, cudaStream_t st);
+cudaError_t launch_pack(const double *aos, const SoA<R> &s, int64_t n, cudaStream_t st, const int32_t *perm = nullptr);
 template <typename R>
-cudaError_t launch_unpack(const SoA<R> &s, double *aos, int64_t n, cudaStream_t st);
+cudaError_t launch_unpack(const SoA<R> &s, double *aos, int64_t n, cudaStream_t st, const int32_t *perm = nullptr);
+// out[perm[i]][w] = in[i][w], NaN as -1
+cudaError_t launch_permute_rows(const float *in, const int32_t *perm, int64_t n, int32_t w, float *out, cudaStream_t st);
 
 }  // namespace lqt
 

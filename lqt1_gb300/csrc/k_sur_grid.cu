@@ -8,17 +8,18 @@
 // may take macro steps, with the detector run at every substep so that the
 // running peak that sets the APD90 level is kept).  For the offered voxels of
 // a tile
-//   1. each thread writes its voxel's normalised BF16 features into shared
-//      memory (row = thread, tcgen05 K-major core-matrix layout);
+//   1. each thread takes its voxel's state from the tile's rows in shared
+//      memory into registers and writes its normalised BF16 features (row =
+//      thread, tcgen05 K-major core-matrix layout);
 //   2. one elected thread runs the 48 -> 128 -> 128 -> 48 network with
 //      tcgen05.mma into TMEM (three layers, each bias added by one more MMA
 //      k-step against a constant ones tile; the threads read the hidden
 //      accumulators back with tcgen05.ld, apply SiLU and write the next FP16
 //      operand into shared memory);
-//   3. each thread reloads its state, advances it by one coarse TPORd step of
-//      the macro length (dt = nsub * dt, no diffusion) and adds the
-//      network's output, the correction to the state after nsub plain
-//      steps, read from TMEM.
+//   3. each thread advances its state by one coarse TPORd step of the macro
+//      length (dt = nsub * dt, no diffusion) while the first layer runs, and
+//      adds the network's output, the correction to the state after nsub
+//      plain steps, read from TMEM.
 // Residual check: every normalised correction within +-kappa times its bound
 // (the largest correction of the training set: the network is not
 // extrapolating), gates within [0, 1] up to a small tolerance (then clamped),
@@ -29,13 +30,24 @@
 // voxel gets rate = NaN and joins the list of voxels that k_grid_step
 // advances with the plain step.
 //
-// Layout: one CTA of four warpgroups per SM.  The weights (BF16, 56 KB), the
-// bias tiles and the normalisation are staged once per CTA; each warpgroup owns a
-// 32 KB operand buffer (the 128 x 48 feature tile, then the 128 x 128 hidden
-// tile in the same bytes) and 128 TMEM columns (hidden accumulator; the
-// 48-column output reuses them once the hidden values are read), so the four
-// warpgroups work on four tiles independently, synchronised by named
-// barriers.
+// Layout: one CTA of four warpgroups per SM.  The weights (56 KB), the bias
+// tiles and the normalisation are staged once per CTA; each warpgroup owns a
+// 35 KB buffer (the 128 x 48 feature tile and the tile's state rows, then the
+// 128 x 128 hidden tile over both) and 128 TMEM columns (hidden accumulator;
+// the 48-column output reuses them once the hidden values are read), so the
+// four warpgroups work on four tiles independently, synchronised by named
+// barriers.  The next tile's rows are copied (cp.async) from the last layer's
+// end on, its voxel index, V and detector before that, so that no tile starts
+// with a chain of loads from HBM.
+//
+// What bounds it: four warps a scheduler, the most that 128 registers of state
+// and step allow, share the special-function unit (tanh.f16x2 takes 16 cycles
+// a warp, 128 of them a tile and warp), the issue slots and shared memory, each
+// 40..57% used; a warp's own chain of phases (state 15%, coarse step 19%,
+// network 47%, correction and stores 19% of 21,500 cycles a tile) fills the
+// rest.  7.5 million voxels: 1.22 -> 1.11 ms with the copies ahead; the HBM
+// floor is 0.38 ms.  Running a third of the coarse step beside each layer's
+// MMAs instead spilled and gained nothing.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -64,7 +76,13 @@ constexpr uint32_t kOffW1 = 0;                                      // 128 x 48 
 constexpr uint32_t kOffW2 = kOffW1 + kMlpHid * kMlpIn * 2;          // 128 x 128 FP16
 constexpr uint32_t kOffW3 = kOffW2 + kMlpHid * kMlpHid * 2;         // 48 x 128 FP16
 constexpr uint32_t kOffXH = kOffW3 + kMlpOut * kMlpHid * 2;         // per group: BF16 features, then FP16 hidden
-constexpr uint32_t kXHBytes = kTile * kMlpHid * 2;
+// per group: the feature tile and, behind it, the 45 state rows and control
+// bytes of a tile as they lie in memory; the hidden tile overlays both
+constexpr int kRows = 45;                                           // 8 concentrations hi, lo; 29 gates
+constexpr uint32_t kRowBytes = kTile * 4;
+constexpr uint32_t kStateOff = kTile * kMlpIn * 2;
+constexpr uint32_t kCtlOff = kStateOff + kRows * kRowBytes;
+constexpr uint32_t kXHBytes = kCtlOff + kTile;
 // bias k-step operands (K = 16 core-matrix tiles): A = ones in columns 0, 1;
 // B = the bias split into hi + lo parts in columns 0, 1
 constexpr uint32_t kBiasK = 16;
@@ -74,9 +92,13 @@ constexpr uint32_t kOffB1 = kOffOnesH + kTile * kBiasK * 2;         // 128 x 16 
 constexpr uint32_t kOffB2 = kOffB1 + kMlpHid * kBiasK * 2;          // 128 x 16 (b2 / 2, FP16)
 constexpr uint32_t kOffB3 = kOffB2 + kMlpHid * kBiasK * 2;          // 48 x 16 (b3, FP16)
 constexpr uint32_t kOffNorm = kOffB3 + kMlpOut * kBiasK * 2;        // 4 x 48 floats
-constexpr uint32_t kOffBar = kOffNorm + 4 * kMlpIn * 4;             // per group mbarrier; tmem slot
-constexpr uint32_t kSmemBytes = kOffBar + 8 * kGroups + 16;
-static_assert(kOffXH % 1024 == 0 && kXHBytes % 1024 == 0, "operand tiles 1 KB aligned");
+constexpr uint32_t kOffDet = kOffNorm + 4 * kMlpIn * 4;             // per thread: next tile's detector,
+constexpr uint32_t kOffNext = kOffDet + kThreads * 16;              // index, V, previous V
+constexpr uint32_t kOffBar = kOffNext + 3 * kThreads * 4;           // per group two mbarriers; tmem slot
+constexpr uint32_t kSmemBytes = kOffBar + 16 * kGroups + 16;
+static_assert(kOffXH % 128 == 0 && kXHBytes % 128 == 0 && kStateOff % 16 == 0, "operand tiles, bulk copies aligned");
+static_assert(kTile * kMlpHid * 2 <= kXHBytes, "hidden tile inside the group's buffer");
+static_assert(kOffDet % 16 == 0 && kOffBar % 8 == 0, "alignment");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 static_assert(kOffNorm % 16 == 0, "normalisation pairs read as float4");
 
@@ -153,18 +175,17 @@ __device__ __forceinline__ uint32_t silu2_f16(float h0, float h1)
 
 // D[128 x N] = A[128 x K] * B[N x K]^T + ones * bias^T: K / 16 MMAs over the
 // operands, then one k-step of the constant ones tile against the bias tile;
-// every operand of the call is BF16 (f16 = false) or every one FP16.
-__device__ __forceinline__ void gemm(uint32_t tmem_d, const uint8_t *A, const uint8_t *B, int K, int N,
-                                     const uint8_t *ones, const uint8_t *bias, bool f16)
+// every operand of the call is BF16 (F16 = false) or every one FP16.
+template <int K, int N, bool F16>
+__device__ __forceinline__ void gemm(uint32_t tmem_d, const uint8_t *A, const uint8_t *B, const uint8_t *ones,
+                                     const uint8_t *bias)
 {
-    const uint32_t lbo = 128, sbo = (uint32_t)(K / 8) * 128;
-    const uint32_t id = f16 ? tc::idesc_f16_f32(128, N) : tc::idesc_bf16_f32(128, N);
-    const uint32_t a0 = tc::smem_u32(A), b0 = tc::smem_u32(B);
-    for (int kk = 0; kk < K / 16; ++kk) {
-        const uint32_t step = (uint32_t)kk * 256;     // two core matrices along K
-        tc::mma_bf16(tmem_d, tc::smem_desc(a0 + step, lbo, sbo), tc::smem_desc(b0 + step, lbo, sbo), id, kk > 0);
-    }
-    const uint32_t sb = (kBiasK / 8) * 128;
+    constexpr uint32_t lbo = 128, sbo = (K / 8) * 128, sb = (kBiasK / 8) * 128;
+    const uint32_t id = F16 ? tc::idesc_f16_f32(128, N) : tc::idesc_bf16_f32(128, N);
+    const uint64_t da = tc::smem_desc(tc::smem_u32(A), lbo, sbo), db = tc::smem_desc(tc::smem_u32(B), lbo, sbo);
+#pragma unroll
+    for (int kk = 0; kk < K / 16; ++kk)      // two core matrices along K: 256 bytes, 16 in a descriptor's address
+        tc::mma_bf16(tmem_d, da + 16 * kk, db + 16 * kk, id, kk > 0);
     tc::mma_bf16(tmem_d, tc::smem_desc(tc::smem_u32(ones), lbo, sb), tc::smem_desc(tc::smem_u32(bias), lbo, sb), id,
                  1u);
 }
@@ -192,21 +213,68 @@ __device__ __forceinline__ int wg_and(int id, int v)
     return r;
 }
 
-// 32 consecutive FP32 columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v)
+// 16 consecutive FP32 columns of this thread's TMEM lane: start the load, and
+// wait for it (and any other) before its registers are used.
+__device__ __forceinline__ void tmem_start16(uint32_t taddr, uint32_t (&r)[16])
 {
-    uint32_t r[32];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ready16(uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                   "+r"(r[15])::"memory");
+}
+// 16 hidden values of row t, columns c .. c + 15: SiLU, FP16 operand.
+__device__ __forceinline__ void silu16(const uint32_t (&r)[16], uint8_t *xh, int t, int c)
+{
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+    for (int q = 0; q < 2; ++q) {
+        uint32_t p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            p[i] = silu2_f16(__uint_as_float(r[8 * q + 2 * i]), __uint_as_float(r[8 * q + 2 * i + 1]));
+        *reinterpret_cast<uint4 *>(xh + tc::kmaj_off(t, c + q * 8, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
+    }
+}
+
+// 4 or 16 bytes global -> shared, asynchronous (per thread, no barrier needed: the
+// thread that waits is the one that reads).
+__device__ __forceinline__ void cp4(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// A warpgroup starts the copies of a tile's state rows and control bytes into
+// its buffer: one row per warp instruction (16 bytes a lane; a bulk copy per
+// row cost its issuing thread 90 cycles).  Every thread's arrival on bar
+// follows its own copies, those of V and the detector included.  Rows are
+// padded to whole tiles and a tile starts at a multiple of 128 voxels, so
+// every copy is aligned and in bounds.
+__device__ __forceinline__ void fetch_state(uint8_t *xh, uint64_t *bar, const GridDev<float> &gd, int64_t k0, int t)
+{
+    const int w = t >> 5, lane = t & 31;
+    const float *cb = reinterpret_cast<const float *>(gd.s.conc) + k0 + 4 * lane, *gb = gd.s.gate + k0 + 4 * lane;
+    uint8_t *dst = xh + kStateOff + 16 * lane;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cp16(dst + (w + 4 * i) * kRowBytes, cb + (w + 4 * i) * gd.s.ld);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = w + 4 * i;                       // gate rows 0..28: slots 0, 1, 2, 5..30
+        if (r < 29) cp16(dst + (16 + r) * kRowBytes, gb + (r < 3 ? r : r + 2) * gd.s.ld);
+    }
+    if (w == 3 && lane < kTile / 16) cp16(xh + kCtlOff + 16 * lane, gd.ctl + k0 + 16 * lane);
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
 }
 
 // Per-voxel onsets: could the S1 stimulus of a voxel with this onset start
@@ -242,11 +310,38 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = tid >> 7, t = tid & 127;          // warpgroup, row within its tile
     const int bar_id = 1 + grp;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kOffBar) + grp;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kOffBar + 8 * kGroups);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kOffBar) + grp;          // network
+    uint64_t *sbar = bar + kGroups;                                             // state rows
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kOffBar + 16 * kGroups);
     float *nrm = reinterpret_cast<float *>(smem + kOffNorm);
     uint8_t *xh = smem + kOffXH + grp * kXHBytes;
     const bool use_net = sg.use_net != 0;
+    const float *__restrict__ V = gd.vg[cur];
+    const float *__restrict__ Vp = gd.vg[cur ^ 1];
+    const int64_t nt = gd.ntissue;
+    const int64_t ntiles = (nt + kTile - 1) / kTile;
+    const int64_t tstride = (int64_t)gridDim.x * kGroups;
+    int64_t tile = (int64_t)blockIdx.x * kGroups + grp;
+    if (t == 0) {
+        tc::mbar_init(bar, 1);
+        tc::mbar_init(sbar, kTile);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    wg_sync(bar_id);
+    // the group's first tile, under way while the weights are staged
+    float4 *nx_d = reinterpret_cast<float4 *>(smem + kOffDet) + tid;
+    int32_t *nx_g = reinterpret_cast<int32_t *>(smem + kOffNext) + tid;
+    float *nx_v = reinterpret_cast<float *>(nx_g) + kThreads, *nx_p = nx_v + kThreads;
+    if (tile < ntiles) {
+        const int64_t k = tile * kTile + t;
+        if (k < nt) {
+            const int64_t g = dim == 1 ? k : (int64_t)gd.gidx[k];
+            cp4(nx_v, V + g);
+            cp4(nx_p, Vp + g);
+            if (gd.det) cp16(nx_d, gd.det + k);
+        }
+        fetch_state(xh, sbar, gd, tile * kTile, t);
+    }
 
     // normalisation, rearranged once per CTA: (scale, -mean * scale) per
     // input (one FMA per feature), the output scales, and kappa times the
@@ -255,8 +350,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
         const float mu = sg.norm[j], sc = sg.norm[kMlpIn + j];
         nrm[2 * j] = sc;
         nrm[2 * j + 1] = -mu * sc;
-        nrm[2 * kMlpIn + j] = sg.norm[2 * kMlpIn + j];
-        nrm[3 * kMlpIn + j] = sg.kappa * sg.norm[3 * kMlpIn + j];
+        nrm[2 * kMlpIn + 2 * j] = sg.norm[2 * kMlpIn + j];
+        nrm[2 * kMlpIn + 2 * j + 1] = sg.kappa * sg.norm[3 * kMlpIn + j];
     }
     if (use_net) {
         // hidden layers halved (see silu2_bf16); biases as an extra k-step
@@ -274,10 +369,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
             *reinterpret_cast<uint4 *>(smem + kOffOnes + tc::kmaj_off(r, kg * 8, kBiasK)) = vb;
             *reinterpret_cast<uint4 *>(smem + kOffOnesH + tc::kmaj_off(r, kg * 8, kBiasK)) = vh;
         }
-        if (t == 0) {
-            tc::mbar_init(bar, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
         if (warp == 0) tc::tmem_alloc(tslot, kTmemCols);
     }
     tc::fence_before();
@@ -287,17 +378,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
     // warp w of the CTA may access TMEM lanes 32 * (w % 4) .. + 31
     const uint32_t t_acc = tmem + grp * kColsPerGroup + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t t_acc_mma = tmem + grp * kColsPerGroup;
-    uint32_t phase = 0;
-    bool net_ok = true;
+    uint32_t phase = 0, sphase = 0;
+    bool net_ok = true;                 // the same in all threads of a warpgroup at the top of the loop
 
     const Clock ck = gd.clk[cur];
-    const float *__restrict__ V = gd.vg[cur];
-    const float *__restrict__ Vp = gd.vg[cur ^ 1];
     const float inv_dt = sg.inv_dt, inv_mac = sg.inv_mac;
-    const int64_t nt = gd.ntissue;
-    const int64_t ntiles = (nt + kTile - 1) / kTile;
     unsigned long long n_offer = 0, n_acc = 0;
-    const int64_t tstride = (int64_t)gridDim.x * kGroups;
     // an S1 window opens during this macro step: every detector records its rest
     bool opens = false;
     {
@@ -309,25 +395,39 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
 
     // the warpgroups are independent (own tiles, barrier, TMEM columns and
     // operand buffer); the loop is uniform within a warpgroup
-    for (int64_t tile = (int64_t)blockIdx.x * kGroups + grp; tile < ntiles; tile += tstride) {
-        const int64_t k = tile * kTile + t;
+    for (; tile < ntiles; tile += tstride) {
+        const int64_t k = tile * kTile + t, kn = k + tstride * kTile;
+        const bool more = kn < nt;
         bool elig = false, need_det = false;
         float vc = 0.f;
         int ct = 0;
-        // 1. the state, loaded once (its loads need only k, so they are in
-        //    flight while the index, V and detector loads resolve): the
-        //    features are built from it and the coarse step advances it in
-        //    registers while the first layer's MMAs run
+        // 1. the tile's state, V and detectors, copied during the previous
+        //    tile's epilogue: the features are built from it and the coarse
+        //    step advances it in registers while the first layer's MMAs run
         CellState<float> c;
-        if (k < nt) {
-            load_cell(c, gd.s, k);
-            const int64_t g = dim == 1 ? k : (int64_t)gd.gidx[k];
-            vc = V[g];
-            const float dv = (vc - Vp[g]) * inv_dt;
-            const uint8_t ctl = gd.ctl[k];
+        bool my_ok = net_ok;            // a wait of this thread ran out in this tile: false
+        if (net_ok) {
+            my_ok = tc::mbar_wait(sbar, sphase, kWaitLimit) || tc::mbar_wait(sbar, sphase, kWaitLimit);
+            sphase ^= 1;
+        }
+        if (k < nt && my_ok) {
+            {
+                const float *st = reinterpret_cast<const float *>(xh + kStateOff) + t;
+                float2 *cp[8];
+                float *gp[29];
+                conc_ptrs(c, cp);
+                gate_ptrs(c, gp);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) *cp[j] = make_float2(st[j * kTile], st[(8 + j) * kTile]);
+#pragma unroll
+                for (int j = 0; j < 29; ++j) *gp[j] = st[(16 + j) * kTile];
+            }
+            vc = *nx_v;
+            const float dv = (vc - *nx_p) * inv_dt;
+            const uint8_t ctl = xh[kCtlOff + t];
             ct = ctl & kCtlType;
             if (gd.det) {
-                const float4 d = gd.det[k];
+                const float4 d = *nx_d;
                 const uint32_t ph = __float_as_uint(d.w) & 7u;
                 // does the detector need this voxel's substeps?  A cycle that
                 // opens; an activation crossing within reach; a slow rise
@@ -340,10 +440,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
             }
             // (a NaN dV/dt fails the first test; the foot test keeps a rising
             // voxel below the foot voltage on the plain step)
-            elig = net_ok && fabsf(dv) <= sg.dvdt_max && !(vc < sg.foot_v && dv > sg.foot_dvdt) &&
+            elig = fabsf(dv) <= sg.dvdt_max && !(vc < sg.foot_v && dv > sg.foot_dvdt) &&
                    !stim_ahead(gd, ck, ctl, k, sg.nsub);
         }
         c.v = vc;
+        // the next tile: its index now, its V once that is here
+        if (more && dim != 1) cp4(nx_g, gd.gidx + kn);
         if (use_net) {
             // features (the previous tile's MMAs have all completed)
             uint4 *row[kMlpIn / 8];
@@ -384,7 +486,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
         const bool run_net = use_net && any && net_ok;
         if (run_net && t == 0) {
             tc::fence_after();
-            gemm(t_acc_mma, xh, smem + kOffW1, kMlpIn, kMlpHid, smem + kOffOnes, smem + kOffB1, false);
+            gemm<kMlpIn, kMlpHid, false>(t_acc_mma, xh, smem + kOffW1, smem + kOffOnes, smem + kOffB1);
             tc::mma_commit(bar);
         }
         // 2. coarse TPORd step of the macro length, overlapping layer 1
@@ -392,60 +494,67 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
             StepOut<float> o;
             tpord_update(c, ct, gd.model, sg.kmac, 0.f, 0.f, &o);
         }
+        if (more) {
+            cp_wait();
+            const int64_t g = dim == 1 ? kn : (int64_t)*nx_g;
+            cp4(nx_v, V + g);
+            cp4(nx_p, Vp + g);
+            if (gd.det) cp16(nx_d, gd.det + kn);
+        }
         // 3. the rest of the network
-        bool have_net = false;
         if (run_net) {
+#pragma unroll 1
             for (int layer = 0; layer < 3; ++layer) {
-                if (layer > 0 && t == 0) {
+                if (layer > 0 && t == 0 && my_ok) {
                     tc::fence_after();
                     if (layer == 1)
-                        gemm(t_acc_mma, xh, smem + kOffW2, kMlpHid, kMlpHid, smem + kOffOnesH, smem + kOffB2, true);
-                    else gemm(t_acc_mma, xh, smem + kOffW3, kMlpHid, kMlpOut, smem + kOffOnesH, smem + kOffB3, true);
+                        gemm<kMlpHid, kMlpHid, true>(t_acc_mma, xh, smem + kOffW2, smem + kOffOnesH, smem + kOffB2);
+                    else gemm<kMlpHid, kMlpOut, true>(t_acc_mma, xh, smem + kOffW3, smem + kOffOnesH, smem + kOffB3);
                     tc::mma_commit(bar);
                 }
-                // every thread of the group takes the same branch: a wait that
-                // ran out anywhere ends the network for this kernel
-                const bool w_ok = tc::mbar_wait(bar, phase, kWaitLimit);
-                if (!wg_and(bar_id, w_ok ? 1 : 0)) {
-                    if (!w_ok) tc::mbar_wait(bar, phase, kWaitLimit);
-                    if (t == 0) atomicExch(sg.err, 1);
-                    net_ok = false;
-                    break;
-                }
+                // a thread whose wait ran out (twice the bound) waits no more:
+                // its row is not used, and the group leaves the network after
+                // this tile
+                if (my_ok) my_ok = tc::mbar_wait(bar, phase, kWaitLimit) || tc::mbar_wait(bar, phase, kWaitLimit);
                 phase ^= 1;
                 tc::fence_after();
                 if (layer == 2) break;
                 // hidden layer: TMEM -> SiLU -> FP16 operand (over the feature
-                // tile, which the finished MMA no longer needs)
+                // and state tiles, which nothing reads any more); the next 16
+                // columns are under way while 16 are computed
+                uint32_t ra[16], rb[16];
+                tmem_start16(t_acc, ra);
 #pragma unroll 1
                 for (int cc = 0; cc < kMlpHid; cc += 32) {
-                    float v[32];
-                    tmem_ld32(t_acc + cc, v);
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t packed[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) packed[i] = silu2_f16(v[q * 8 + 2 * i], v[q * 8 + 2 * i + 1]);
-                        *reinterpret_cast<uint4 *>(xh + tc::kmaj_off(t, cc + q * 8, kMlpHid)) =
-                            make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    }
+                    tmem_ready16(ra);
+                    tmem_start16(t_acc + cc + 16, rb);
+                    silu16(ra, xh, t, cc);
+                    tmem_ready16(rb);
+                    if (cc + 32 < kMlpHid) tmem_start16(t_acc + cc + 32, ra);
+                    silu16(rb, xh, t, cc + 16);
                 }
                 tc::fence_before();
                 tc::fence_proxy_async();
                 wg_sync(bar_id);
             }
-            have_net = net_ok;
         }
+        // every thread of the group takes the same branch: a wait that ran out
+        // anywhere ends the network, and the copies, for this kernel
+        if (net_ok && !wg_and(bar_id, my_ok ? 1 : 0)) {
+            if (t == 0) atomicExch(sg.err, 1);
+            net_ok = false;
+        }
+        if (net_ok && tile + tstride < ntiles) fetch_state(xh, sbar, gd, (tile + tstride) * kTile, t);
+        const bool have_net = run_net && net_ok;
         // 4. the correction
-        bool ok = elig && (net_ok || !use_net);
-        uint32_t why = 0;   // failed checks: 1 network bound, 2 gate range, 4 concentration, 8 ionic V step
+        bool ok = elig && net_ok;
+        // checks passed: network bound, gate range, concentration, ionic V step
+        bool ok_net = true, ok_gate = true, ok_conc = true, ok_v = true;
         if (have_net) {
             float2 *cp[8];
             float *gp[29];
             conc_ptrs(c, cp);
             gate_ptrs(c, gp);
-            const float *osc = nrm + 2 * kMlpIn;
-            const float *kbd = nrm + 3 * kMlpIn;     // kappa * bound
 #pragma unroll
             for (int cc = 0; cc < 48; cc += 16) {
                 float v[16];
@@ -455,9 +564,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
                     for (int i = 0; i < 16; ++i) {
                         const int j = cc + i;
                         if (j < kMlpNState) {
-                            const float z = v[i];
-                            if (!(fabsf(z) <= kbd[j])) why |= 1u;
-                            const float d = z * osc[j];
+                            // (output scale, kappa * bound)
+                            const float2 q = reinterpret_cast<const float2 *>(nrm + 2 * kMlpIn)[j];
+                            const float z = v[i], d = z * q.x;
+                            ok_net = ok_net && fabsf(z) <= q.y;
                             if (j == 0) c.v += d;
                             else if (j < 9) cadd(*cp[j - 1], d);
                             else *gp[j - 9] += d;
@@ -474,18 +584,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
 #pragma unroll
             for (int j = 0; j < kSurNProb; ++j) {
                 const float x = *gp[j];
-                if (!(x >= -1e-3f && x <= 1.001f)) why |= 2u;
+                ok_gate = ok_gate && x >= -1e-3f && x <= 1.001f;
                 *gp[j] = fminf(fmaxf(x, 0.f), 1.f);
             }
 #pragma unroll
             for (int j = kSurNProb; j < 29; ++j)
-                if (!(*gp[j] == *gp[j])) why |= 2u;
+                ok_gate = ok_gate && *gp[j] == *gp[j];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                if (!(cp[j]->x > 0.f)) why |= 4u;
+                ok_conc = ok_conc && cp[j]->x > 0.f;
             const float dvm = c.v - vc;
-            if (!(fabsf(dvm) <= sg.vstep_max)) why |= 8u;    // NaN fails as well
-            ok = ok && why == 0;
+            ok_v = fabsf(dvm) <= sg.vstep_max;               // NaN fails as well
+            ok = ok && ok_net && ok_gate && ok_conc && ok_v;
             if (ok) {
                 store_cell(c, gd.s, k);
                 sg.rate[k] = dvm * inv_mac;
@@ -503,10 +613,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
             if (plain) sg.plist[base + __popc(mp & ((1u << lane) - 1u))] = (int32_t)k;
         }
         // offered voxels that failed each check (one atomic per warp and reason)
+        if (__any_sync(0xffffffffu, elig && !(ok_net && ok_gate && ok_conc && ok_v))) {
+            const bool good[4] = {ok_net, ok_gate, ok_conc, ok_v};
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const unsigned mr = __ballot_sync(0xffffffffu, elig && ((why >> r) & 1u));
-            if (lane == 0 && mr) atomicAdd(sg.stats + 2 + r, (unsigned long long)__popc(mr));
+            for (int r = 0; r < 4; ++r) {
+                const unsigned mr = __ballot_sync(0xffffffffu, elig && !good[r]);
+                if (lane == 0 && mr) atomicAdd(sg.stats + 2 + r, (unsigned long long)__popc(mr));
+            }
         }
         const unsigned mo = __ballot_sync(0xffffffffu, elig), ma = __ballot_sync(0xffffffffu, ok);
         if (lane == 0) {

@@ -379,11 +379,13 @@ int lqt_sim_tune(lqt_sim *s, int32_t variant, int32_t *chosen, float *ms_per_var
  * elsewhere the direct kernel runs); 203, 204 = the same with each tile's
  * V halo (the box of the dense V grid its 19-point stencils reach, copied as
  * z-segments of its columns) staged in shared memory too, at 3, 4 CTAs/SM
- * (3D anisotropic grids with nz a multiple of 4; elsewhere 105 runs);
- * 304, 305, 306 = one producer warp streams each tile's rows into a two-stage
- * shared-memory ring (full/empty barriers) while eight warps compute, V read
- * from the grid, at 4, 5, 6 CTAs/SM (2D/3D anisotropic grids; elsewhere 105
- * runs).  variant >= 0 forces one (the autotuner then keeps it); variant < 0
+ * (3D anisotropic grids of less than 2^30 voxels with nz a multiple of 4;
+ * elsewhere 105 runs);
+ * 304, 305, 306 = two voxels per thread, V read from the grid; 304: one
+ * producer warp streams each tile's rows into a two-stage shared-memory ring
+ * (full/empty barriers) while four warps compute; 305, 306: each warp copies
+ * its own rows one unit of 64 voxels ahead, at two occupancies (2D/3D
+ * anisotropic grids of less than 2^30 voxels; elsewhere 105 runs).  variant >= 0 forces one (the autotuner then keeps it); variant < 0
  * only reports the current one.  All variants give bit-identical results.
  * ms_per_variant (or NULL): 11 mean milliseconds per step from the last
  * autotune, in the order 5, 6, 8, 105, 106, 108, 203, 204, 304, 305, 306

@@ -159,6 +159,7 @@ struct lqt_sim {
         g.ntissue = ntissue;
         g.nbnd = nbnd;
         g.sx = (int64_t)ny * nz;
+        g.ngrid = ngrid;
         g.sy = dim == 2 ? 1 : nz;
         g.pad = 0;
         g.dx = dx;

@@ -36,6 +36,7 @@ template <typename R> struct GridDev {
     R diso;                        // isotropic D
     int64_t ntissue, nbnd;
     int64_t sx, sy;                // dense strides of x and y (z stride 1)
+    int64_t ngrid;                 // voxels of the dense grid
     int64_t pad;                   // grid origin offset (0)
     double dx;
     R inv_dx, inv_2dx, inv_dx2, inv_4dx2;
@@ -129,9 +130,11 @@ cudaError_t launch_sur_step_small(const GridDev<float> &gd, const StepK &k, int 
 // anisotropic grids, the others fall back to the direct kernel) or of
 // k_sur_substep_vbox (200 + CTAs/SM: the same with each tile's V halo box
 // staged too; 3D anisotropic grids with nz a multiple of 4 and the boxes
-// built, the others fall back to k_sur_substep_tile at 5 CTAs/SM) or of the
-// same producer-warp kernel with the rows only (300 + CTAs/SM; 2D/3D
-// anisotropic grids, the others fall back as the 100s do).
+// built, the others fall back to k_sur_substep_tile at 5 CTAs/SM), or the
+// kernels with two voxels per thread (2D/3D anisotropic grids, the others fall
+// back as the 100s do): 304 k_sur_substep_pair, rows by a producer warp; 305,
+// 306 k_sur_substep_warp, rows by each warp itself, at 6 and 8 CTAs/SM (2D: 8
+// and 10).
 constexpr int kSubVariants[11] = {5, 6, 8, 105, 106, 108, 203, 204, 304, 305, 306};
 constexpr int kSubNVariants = 11;
 cudaError_t launch_sur_substep(const GridDev<float> &gd, double dt, int cur, int dim, int minb, cudaStream_t st);

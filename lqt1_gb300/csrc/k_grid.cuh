@@ -42,27 +42,53 @@ template <typename R> __device__ __forceinline__ R du_fma(R a, R b, R c)
 }
 
 // The anisotropic stencil with the tensor (xx yy zz xy xz yz) and its
-// divergence at hand, on any x-major array of V with strides sx, sy (z stride
-// 1): the dense grid, or a tile's box of it staged in shared memory.
+// divergence at hand; at(i, j, l) is V at the neighbour i, j, l voxels away
+// along x, y, z.
+template <int DIM, typename At>
+__device__ __forceinline__ float sub_du_of(const GridDev<float> &gd, At at, float vc, const float *Dt, const float *Bt)
+{
+    const float vxp = at(1, 0, 0), vxm = at(-1, 0, 0), vyp = at(0, 1, 0), vym = at(0, -1, 0);
+    const float c2 = gd.inv_dx2, c4 = gd.inv_4dx2, c1 = gd.inv_2dx;
+    const float lxx = (vxp + vxm - 2.f * vc) * c2;
+    const float lyy = (vyp + vym - 2.f * vc) * c2;
+    const float lxy = (at(1, 1, 0) + at(-1, -1, 0) - at(-1, 1, 0) - at(1, -1, 0)) * c4;
+    float du = fmaf(Dt[0], lxx, fmaf(Dt[1], lyy, __fmul_rn(2.f * Dt[3], lxy)));
+    du = fmaf(Bt[0], (vxp - vxm) * c1, fmaf(Bt[1], (vyp - vym) * c1, du));
+    if constexpr (DIM == 3) {
+        const float vzp = at(0, 0, 1), vzm = at(0, 0, -1);
+        const float lzz = (vzp + vzm - 2.f * vc) * c2;
+        const float lxz = (at(1, 0, 1) + at(-1, 0, -1) - at(-1, 0, 1) - at(1, 0, -1)) * c4;
+        const float lyz = (at(0, 1, 1) + at(0, -1, -1) - at(0, -1, 1) - at(0, 1, -1)) * c4;
+        du = fmaf(Dt[2], lzz, fmaf(2.f, fmaf(Dt[4], lxz, __fmul_rn(Dt[5], lyz)), fmaf(Bt[2], (vzp - vzm) * c1, du)));
+    }
+    return du;
+}
+
+// ... on any x-major array of V with strides sx, sy (z stride 1): the dense
+// grid, or a tile's box of it staged in shared memory.
 template <int DIM>
 __device__ __forceinline__ float sub_du_at(const GridDev<float> &gd, const float *__restrict__ V, int64_t g,
                                            int64_t sx, int64_t sy, float vc, const float *Dt, const float *Bt)
 {
-    const float vxp = V[g + sx], vxm = V[g - sx], vyp = V[g + sy], vym = V[g - sy];
-    const float c2 = gd.inv_dx2, c4 = gd.inv_4dx2, c1 = gd.inv_2dx;
-    const float lxx = (vxp + vxm - 2.f * vc) * c2;
-    const float lyy = (vyp + vym - 2.f * vc) * c2;
-    const float lxy = (V[g + sx + sy] + V[g - sx - sy] - V[g - sx + sy] - V[g + sx - sy]) * c4;
-    float du = fmaf(Dt[0], lxx, fmaf(Dt[1], lyy, __fmul_rn(2.f * Dt[3], lxy)));
-    du = fmaf(Bt[0], (vxp - vxm) * c1, fmaf(Bt[1], (vyp - vym) * c1, du));
-    if constexpr (DIM == 3) {
-        const float vzp = V[g + 1], vzm = V[g - 1];
-        const float lzz = (vzp + vzm - 2.f * vc) * c2;
-        const float lxz = (V[g + sx + 1] + V[g - sx - 1] - V[g - sx + 1] - V[g + sx - 1]) * c4;
-        const float lyz = (V[g + sy + 1] + V[g - sy - 1] - V[g - sy + 1] - V[g + sy - 1]) * c4;
-        du = fmaf(Dt[2], lzz, fmaf(2.f, fmaf(Dt[4], lxz, __fmul_rn(Dt[5], lyz)), fmaf(Bt[2], (vzp - vzm) * c1, du)));
-    }
-    return du;
+    return sub_du_of<DIM>(gd, [&](int i, int j, int l) { return V[g + i * sx + j * sy + l]; }, vc, Dt, Bt);
+}
+
+// ... on a grid of less than 2^30 voxels, o being the voxel's byte offset and
+// sx4, sy4 the strides in bytes: 32-bit arithmetic per neighbour column.
+template <int DIM>
+__device__ __forceinline__ float sub_du_32(const GridDev<float> &gd, const float *__restrict__ V, uint32_t o,
+                                           uint32_t sx4, uint32_t sy4, float vc, const float *Dt, const float *Bt)
+{
+    const char *Vb = reinterpret_cast<const char *>(V);
+    return sub_du_of<DIM>(gd, [&](int i, int j, int l) {
+        return *reinterpret_cast<const float *>(Vb + (o + (uint32_t)i * sx4 + (uint32_t)j * sy4) + 4 * l);
+    }, vc, Dt, Bt);
+}
+
+// The stimulus bits of a voxel's control byte that can act in this step.
+__device__ __forceinline__ uint32_t stim_mask(const GridDev<float> &gd, const Clock &ck)
+{
+    return ((gd.onset ? ck.s1_cycle_ok : ck.s1_on) ? (uint32_t)kCtlS1 : 0u) | (ck.s2_on ? (uint32_t)kCtlS2 : 0u);
 }
 
 // du = sum_i D_ii V_ii + 2 sum_{i<j} D_ij V_ij + sum_j b_j V_j

@@ -78,34 +78,6 @@ __device__ __forceinline__ float mlp_rcp(float x)
     return r;
 }
 
-// Two FP32 values in a register pair: one instruction for both (IEEE rounding
-// per value, as the scalar forms).
-__device__ __forceinline__ uint64_t pair2(float a, float b)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void split2(uint64_t p, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // SiLU of two values, x / (1 + exp(-x)), as a BF16 pair.  One reciprocal of
 // the product of the two denominators serves both; each quotient is corrected
 // once by its remainder, which an FMA gives exactly (Markstein's correction),
@@ -116,14 +88,14 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
 __device__ __forceinline__ uint32_t silu2_bf16(uint64_t x)
 {
     float a0, a1, d0, d1, q0, q1;
-    split2(mul2(x, pair2(-1.4426950408889634f, -1.4426950408889634f)), a0, a1);
-    const uint64_t d = add2(pair2(fminf(mlp_ex2(a0), 1e18f), fminf(mlp_ex2(a1), 1e18f)), pair2(1.0f, 1.0f));
-    split2(d, d0, d1);
+    tc::split2(tc::mul2(x, tc::pair2(-1.4426950408889634f, -1.4426950408889634f)), a0, a1);
+    const uint64_t d = tc::add2(tc::pair2(fminf(mlp_ex2(a0), 1e18f), fminf(mlp_ex2(a1), 1e18f)), tc::pair2(1.0f, 1.0f));
+    tc::split2(d, d0, d1);
     const float r = mlp_rcp(d0 * -d1);
-    const uint64_t nr = pair2(r * d1, r * d0);
-    uint64_t nq = mul2(x, nr);
-    nq = fma2(fma2(nq, d, x), nr, nq);
-    split2(nq, q0, q1);
+    const uint64_t nr = tc::pair2(r * d1, r * d0);
+    uint64_t nq = tc::mul2(x, nr);
+    nq = tc::fma2(tc::fma2(nq, d, x), nr, nq);
+    tc::split2(nq, q0, q1);
     const __nv_bfloat162 h = __floats2bfloat162_rn(-q0, -q1);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
@@ -248,8 +220,8 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_infer_tc(const __nv_bf
                     for (int i = 0; i < 2; ++i) {
                         const float4 b = bs[(c >> 2) + q * 2 + i];
                         const float *u = v + q * 8 + 4 * i;
-                        p[2 * i] = silu2_bf16(add2(pair2(u[0], u[1]), pair2(b.x, b.y)));
-                        p[2 * i + 1] = silu2_bf16(add2(pair2(u[2], u[3]), pair2(b.z, b.w)));
+                        p[2 * i] = silu2_bf16(tc::add2(tc::pair2(u[0], u[1]), tc::pair2(b.x, b.y)));
+                        p[2 * i + 1] = silu2_bf16(tc::add2(tc::pair2(u[2], u[3]), tc::pair2(b.z, b.w)));
                     }
                     *reinterpret_cast<uint4 *>(xh + tc::kmaj_off(t, c + q * 8, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
                 }

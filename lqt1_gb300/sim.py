@@ -143,8 +143,9 @@ class Sim:
 
     def substep_variant(self, variant: int = -1, timings: bool = False):
         """Force the V-only substep's kernel variant (5, 6, 8 direct; 105, 106,
-        108 staged by bulk copies; 203, 204 with the V halo staged too; 304,
-        305, 306 rows streamed by a producer warp) or,
+        108 staged by bulk copies; 203, 204 with the V halo staged too; 304
+        two voxels a thread, rows by a producer warp; 305, 306 rows by each
+        warp itself) or,
         with -1, report the current one; with timings, also the last
         autotune's ms per variant (same order)."""
         L = N.lib()

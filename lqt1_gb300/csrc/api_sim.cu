@@ -83,6 +83,11 @@ struct lqt_sim {
     int minb = 2;
     int sub_minb = 5;               // V-only substep variant (kSubVariants)
     int64_t small_n = 0;            // voxels up to which a grid is small (kSmallPerSM per SM)
+    // many steps in one launch: block dependencies (NULL: not for this grid),
+    // published steps, and the error word in mapped host memory
+    int2 *persist_dep = nullptr;
+    uint32_t *persist_flags = nullptr;
+    int32_t *persist_err = nullptr, *persist_err_dev = nullptr;
     bool step_forced = false;       // set by lqt_sim_tune with a variant
     bool sub_forced = false;        // set by lqt_sim_substep_variant: the autotuner keeps it
     int32_t sub_skip_copy = 0;      // failure-path test (lqt_sim_set_wait_test)
@@ -137,11 +142,17 @@ struct lqt_sim {
         for (cudaStream_t c : copy_stream)
             if (c) cudaStreamDestroy(c);
         if (graph) cudaGraphExecDestroy(graph);
+        if (persist_err) {
+            cudaStreamSynchronize(stream);
+            cudaFreeHost(persist_err);
+        }
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
     bool fp64() const { return p.precision == LQT_FP64; }
     // A step is one launch: small grids in the mixed form, unless a variant of
     // the step kernel, or of the substep in effect, was asked for.
+    // Several steps are one launch (k_grid_persist.cu).
+    bool persists() const { return persist_dep && !sur && folds(); }
     bool folds() const { return !fp64() && ntissue <= small_n && !step_forced && !(sub_forced && sur && plist_valid); }
 
     template <typename R> GridDev<R> dev() const
@@ -343,6 +354,46 @@ void build_ghost_refs(const TissueMap &tm, std::vector<uint8_t> &ctl, std::vecto
         for (int32_t j = first[k]; j >= 0; j = next[j]) glist.push_back((int32_t)tm.bnd_dst[j]);
         glist.back() |= INT32_MIN;
     }
+}
+
+// Per block of kPersistBlock voxels the range of blocks it exchanges V with: a
+// voxel's neighbours, or the voxels that those mirror; in both directions.
+std::vector<int2> persist_deps(const TissueMap &tm, int dim, int64_t ny, int64_t nz, int64_t n)
+{
+    const int64_t nb = (n + kPersistBlock - 1) / kPersistBlock;
+    std::vector<int2> dep(nb);
+    for (int64_t b = 0; b < nb; ++b) dep[b] = make_int2((int)b, (int)b);
+    auto meet = [&](int64_t k, int64_t j) {
+        const int p = (int)(k / kPersistBlock), q = (int)(j / kPersistBlock);
+        dep[p].x = std::min(dep[p].x, q);
+        dep[p].y = std::max(dep[p].y, q);
+        dep[q].x = std::min(dep[q].x, p);
+        dep[q].y = std::max(dep[q].y, p);
+    };
+    if (dim == 1) {
+        for (int64_t k = 0; k + 1 < n; ++k) meet(k, k + 1);
+        return dep;
+    }
+    std::vector<int32_t> owner = tm.tissue_of;
+    for (size_t j = 0; j < tm.bnd_dst.size(); ++j) owner[tm.bnd_dst[j]] = tm.tissue_of[tm.bnd_src[j]];
+    const int64_t sx = ny * nz, sy = dim == 2 ? 1 : nz;
+    const int lz = dim == 3 ? 1 : 0;
+    for (int64_t k = 0; k < n; ++k)
+        for (int i = -1; i <= 1; ++i)
+            for (int j = -1; j <= 1; ++j)
+                for (int l = -lz; l <= lz; ++l) {
+                    const int32_t o = owner[tm.cells[k] + i * sx + j * sy + l];
+                    if (o >= 0) meet(k, o);
+                }
+    return dep;
+}
+
+// Waits and device errors that a finished step left behind.
+int persist_status(const lqt_sim *s)
+{
+    if (s->persist_err && *(volatile int32_t *)s->persist_err)
+        return fail(LQT_ERR_CUDA, "lqt_sim: a wait between the blocks of a small grid's launch ran out; the run is not valid");
+    return LQT_OK;
 }
 
 // At a macro-step boundary with a surrogate attached: the macro-step kernel.
@@ -747,6 +798,22 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
             return fail(LQT_ERR_NOMEM, "lqt_sim_create: " + m);
         }
     }
+    if (!s->fp64() && (n + kPersistBlock - 1) / kPersistBlock <= grid_persist_capacity(dim)) {
+        const std::vector<int2> dep = persist_deps(s->tm, dim, ny, nz, n);
+        int2 *d = nullptr;
+        bool ok = !s->mem.alloc((void **)&d, dep.size() * sizeof(int2)) &&
+                  !s->mem.alloc((void **)&s->persist_flags, dep.size() * 4) &&
+                  cudaHostAlloc((void **)&s->persist_err, 4, cudaHostAllocMapped) == cudaSuccess &&
+                  cudaHostGetDevicePointer((void **)&s->persist_err_dev, s->persist_err, 0) == cudaSuccess &&
+                  cudaMemcpy(d, dep.data(), dep.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
+                  cudaMemset(s->persist_flags, 0, dep.size() * 4) == cudaSuccess;
+        if (!ok) {
+            delete s;
+            return fail(LQT_ERR_NOMEM, "lqt_sim_create: step flags");
+        }
+        *s->persist_err = 0;
+        s->persist_dep = d;
+    }
     std::vector<int32_t> gi32(dim > 1 ? n : 0), bd(s->nbnd), bs(s->nbnd);
     for (int64_t k = 0; k < (int64_t)gi32.size(); ++k) gi32[k] = (int32_t)s->tm.cells[k];
     for (int64_t j = 0; j < s->nbnd; ++j) {
@@ -897,14 +964,34 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
     }
     int64_t left = nsteps;
     // (a call shorter than the autotuner's steps does not start it)
+    // (with many steps in one launch the autotuner has nothing to choose)
+    const bool persist = s->persists();
     const int64_t tune_steps = 5 * ((s->fp64() ? 2 : kGridNVariantsF32) + (s->sur ? kSubNVariants : 0));
-    if (!s->tuned && left >= std::max<int64_t>(64, tune_steps)) {
+    if (!persist && !s->tuned && left >= std::max<int64_t>(64, tune_steps)) {
         int64_t used = 0;
         int rc = autotune(s, 5, &used);
         if (rc) return rc;
         left -= used;
     }
     while (left > 0) {
+        if (persist && left >= kPersistMin) {
+            const bool ecg = s->nel > 0 && s->ecg_every > 0;
+            int64_t m = std::min<int64_t>(left, kPersistMax);
+            if (ecg) m = std::min<int64_t>(m, s->ecg_every - s->step % s->ecg_every);
+            int rc = persist_status(s);
+            if (rc) return rc;
+            const PersistArgs a{s->persist_dep, s->persist_flags, s->persist_err_dev, (int)m};
+            CK(launch_grid_persist(devf<float>(s), make_stepk(s->p.dt), s->cur, s->dim, a, s->stream));
+            s->cur ^= (int)(m & 1);
+            s->step += m;
+            for (int64_t i = 0; i < m; ++i) s->time += s->p.dt;
+            left -= m;
+            if (ecg && s->step % s->ecg_every == 0) {
+                rc = launch_ecg_now(s);
+                if (rc) return rc;
+            }
+            continue;
+        }
         // graph replay for whole chunks starting on a chunk boundary
         if (left >= kGraphChunk && s->step % kGraphChunk == 0 &&
             (s->ecg_every <= 0 || kGraphChunk % s->ecg_every == 0)) {
@@ -935,7 +1022,7 @@ int lqt_sim_step(lqt_sim *s, int64_t nsteps)
     const int rc = sim_advance(s, nsteps);
     if (rc) return rc;
     CK(cudaStreamSynchronize(s->stream));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_step_async(lqt_sim *s, int64_t nsteps)
@@ -948,7 +1035,7 @@ int lqt_sim_sync(lqt_sim *s)
 {
     if (!s) return fail(LQT_ERR_INVALID, "lqt_sim_sync: NULL handle");
     CK(cudaStreamSynchronize(s->stream));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_get_v(lqt_sim *s, void *v_host, int as_double)
@@ -1284,6 +1371,7 @@ int lqt_sim_check(lqt_sim *s, int64_t *n_bad)
     CK(cudaMemcpy(&v, s->nbad, sizeof(v), cudaMemcpyDeviceToHost));
     CK(cudaMemset(s->nbad, 0, sizeof(v)));
     *n_bad = (int64_t)v;
+    if (persist_status(s)) return LQT_ERR_CUDA;
     if (s->sur_err) {
         int err = 0;
         CK(cudaMemcpy(&err, s->sur_err, sizeof(int), cudaMemcpyDeviceToHost));

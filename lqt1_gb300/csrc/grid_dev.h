@@ -122,6 +122,23 @@ template <typename R> cudaError_t launch_ghost(const GridDev<R> &gd, int cur, in
 // the time is then one thread's chain of loads and arithmetic (four warps per
 // SM partition at the most), and no second launch.
 constexpr int kSmallPerSM = 512;
+
+// Many steps in one launch (k_grid_persist.cu): grids of at most one block of
+// 128 voxels per SM in the mixed form, for runs of at least kPersistMin steps.
+// Up to there a step takes 2.6..3.0 us against 5.5 in a launch of its own; with
+// two blocks per SM 4.2..5.9 against 4.5..5.0, so larger grids stay with the
+// launch per step.
+constexpr int kPersistBlock = 128, kPersistPerSM = 1, kPersistMin = 3, kPersistMax = 500;
+struct PersistArgs {
+    const int2 *dep;               // per block: the blocks whose V it reads or that read its V, [x, y]
+    uint32_t *flags;               // per block: steps published, the same in all blocks between launches
+    int32_t *err;                  // set when a wait ran out
+    int nsteps;
+};
+// blocks that can be resident together on the current device
+int grid_persist_capacity(int dim);
+cudaError_t launch_grid_persist(const GridDev<float> &gd, const StepK &k, int cur, int dim, const PersistArgs &a,
+                                cudaStream_t st);
 cudaError_t launch_sur_step_small(const GridDev<float> &gd, const StepK &k, int cur, int dim, cudaStream_t st);
 // Variants of the V-only substep: minimum CTAs/SM of 256 threads of
 // k_sur_substep (5, 6, 8: one thread per voxel, direct loads), of

@@ -230,7 +230,7 @@ template <typename R> __device__ __forceinline__ int32_t ghost_ref(const GridDev
 // The new V of a tissue voxel (dense index g), there and in the empty voxels
 // that mirror it (e = ghost_ref).
 template <typename R>
-__device__ __forceinline__ void put_v(const GridDev<R> &gd, R *__restrict__ Vn, int64_t g, uint8_t ctl, int32_t e, R v)
+__device__ __forceinline__ void put_v(const GridDev<R> &gd, R *Vn, int64_t g, uint8_t ctl, int32_t e, R v)
 {
     Vn[g] = v;
     if (ctl & kCtlGhost) {
@@ -246,10 +246,9 @@ __device__ __forceinline__ void put_v(const GridDev<R> &gd, R *__restrict__ Vn, 
     }
 }
 
-// The clock of the step after the one from grid cur (one thread of the launch).
-template <typename R> __device__ __forceinline__ void advance_clock(const GridDev<R> &gd, int cur)
+// The clock of the step after ck's.
+template <typename R> __device__ __forceinline__ Clock next_clock(const GridDev<R> &gd, Clock ck)
 {
-    Clock ck = gd.clk[cur];
     ck.step += 1;
     ck.time += gd.dt;
     ck.time_f = (float)ck.time;
@@ -264,7 +263,13 @@ template <typename R> __device__ __forceinline__ void advance_clock(const GridDe
         ck.tb = ck.time - floor(ck.time / gd.bcl) * gd.bcl;
         ck.s1_cycle_ok = gd.s1_beats <= 0 || floor(ck.time / gd.bcl) < gd.s1_beats;
     }
-    gd.clk[cur ^ 1] = ck;
+    return ck;
+}
+
+// ... after the step from grid cur (one thread of the launch).
+template <typename R> __device__ __forceinline__ void advance_clock(const GridDev<R> &gd, int cur)
+{
+    gd.clk[cur ^ 1] = next_clock(gd, gd.clk[cur]);
 }
 
 // One plain step of tissue voxel k: diffusion, stimulus, the TPORd update,

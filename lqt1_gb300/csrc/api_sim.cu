@@ -51,6 +51,7 @@ struct lqt_sim {
     int32_t *vbox_hdr = nullptr, *vli = nullptr;   // V-halo boxes of the 3D substep (k_sur_substep_vbox)
     double *conc = nullptr, *aos = nullptr;
     int32_t *gidx = nullptr, *bnd_dst = nullptr, *bnd_src = nullptr;
+    int32_t *bnd_k = nullptr;       // with a surrogate: tissue index of each mirror voxel's source
     int32_t *gref = nullptr, *glist = nullptr;   // the mirror map by source voxel (GridDev::gref)
     float *xpos = nullptr;          // 2D/3D: (float)(i * dx), i < max(nx, ny, nz)
     uint8_t *ctl = nullptr;
@@ -82,6 +83,7 @@ struct lqt_sim {
     // occupancy variant of k_grid_step (minimum CTAs/SM) and the autotuner
     int minb = 2;
     int sub_minb = 5;               // V-only substep variant (kSubVariants)
+    int64_t merge_bnd = 0;          // mirror voxels up to which they share a launch with the list (kMergeBndPerSM)
     int64_t small_n = 0;            // voxels up to which a grid is small (kSmallPerSM per SM)
     // many steps in one launch: block dependencies (NULL: not for this grid),
     // published steps, and the error word in mapped host memory
@@ -194,6 +196,7 @@ struct lqt_sim {
         g.onset = onset;
         g.bnd_dst = bnd_dst;
         g.bnd_src = bnd_src;
+        g.bnd_k = bnd_k;
         g.gref = gref;
         g.glist = glist;
         g.fold = folds();
@@ -455,8 +458,14 @@ int launch_step(lqt_sim *s)
 {
     int rc = launch_sur_if_due(s);
     if (rc) return rc;
-    CK(launch_substep(s));
-    CK(launch_ghost_now(s));
+    if (s->sur && s->plist_valid && !s->folds() && s->nbnd <= s->merge_bnd) {
+        const GridDev<float> g = devf<float>(s);
+        CK(launch_sur_substep(g, s->p.dt, s->cur, s->dim, s->sub_minb, s->stream));
+        CK(launch_list_ghost(g, make_stepk(s->p.dt), s->cur, s->dim, s->stream));
+    } else {
+        CK(launch_substep(s));
+        CK(launch_ghost_now(s));
+    }
     s->cur ^= 1;
     return LQT_OK;
 }
@@ -736,6 +745,7 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         s->small_n = (int64_t)nsm * kSmallPerSM;
+        s->merge_bnd = (int64_t)nsm * kMergeBndPerSM;
     }
     s->nbnd = (int64_t)s->tm.bnd_dst.size();
     if (s->ntissue == 0) {
@@ -1434,7 +1444,14 @@ int lqt_sim_set_surrogate(lqt_sim *s, lqt_mlp *m, const lqt_sur_config *cfg)
                  s->mem.alloc((void **)&s->plist_n, sizeof(unsigned long long)) |
                  s->mem.alloc((void **)&s->sur_stats, kSurNStats * sizeof(unsigned long long)) |
                  s->mem.alloc((void **)&s->sur_err, sizeof(int));
+        rc = rc | s->mem.alloc((void **)&s->bnd_k, std::max<int64_t>(1, s->nbnd) * 4);
         if (rc) return LQT_ERR_NOMEM;
+        if (s->nbnd) {
+            std::vector<int32_t> bk(s->nbnd);
+            for (int64_t j = 0; j < s->nbnd; ++j) bk[j] = s->tm.tissue_of[s->tm.bnd_src[j]];
+            CK(cudaMemcpyAsync(s->bnd_k, bk.data(), s->nbnd * 4, cudaMemcpyHostToDevice, s->stream));
+            CK(cudaStreamSynchronize(s->stream));
+        }
         CK(cudaMemsetAsync(s->sur_stats, 0, kSurNStats * sizeof(unsigned long long), s->stream));
         CK(cudaMemsetAsync(s->sdflag, 0, pad_tiles(s->ntissue), s->stream));
         CK(cudaMemsetAsync(s->sur_err, 0, sizeof(int), s->stream));

@@ -54,6 +54,7 @@ template <typename R> struct GridDev {
     R s1_strength, s2_strength;
     const float *onset;            // per tissue voxel onset delay, or null
     const int32_t *bnd_dst, *bnd_src;
+    const int32_t *bnd_k;          // with a surrogate: the source's tissue index
     // the same map from the source's side, for the tissue voxels with kCtlGhost:
     // gref[k] >= 0 is the one empty voxel that mirrors voxel k, else ~gref[k] is
     // where its list starts in glist, whose last entry has the sign bit set
@@ -139,6 +140,13 @@ struct PersistArgs {
 int grid_persist_capacity(int dim);
 cudaError_t launch_grid_persist(const GridDev<float> &gd, const StepK &k, int cur, int dim, const PersistArgs &a,
                                 cudaStream_t st);
+// Mirror voxels per SM up to which the listed voxels and they are one launch:
+// one wave of its blocks (two CTAs of 256 threads, four entries a thread).  50
+// steps in macro steps take 822 us so against 917 on a fibre sheet of 500 x 500,
+// 1.71 ms against 1.73 on a shell of 1.1 million voxels; beyond the wave, on
+// one of 7.5 million (485,000 mirror voxels), 9.43 ms against 9.38.
+constexpr int kMergeBndPerSM = 2 * 256 * 4;
+cudaError_t launch_list_ghost(const GridDev<float> &gd, const StepK &k, int cur, int dim, cudaStream_t st);
 cudaError_t launch_sur_step_small(const GridDev<float> &gd, const StepK &k, int cur, int dim, cudaStream_t st);
 // Variants of the V-only substep: minimum CTAs/SM of 256 threads of
 // k_sur_substep (5, 6, 8: one thread per voxel, direct loads), of

@@ -301,11 +301,11 @@ __device__ __forceinline__ void grid_step_voxel(const GridDev<R> &gd, const Step
 
 // The same step as a called function: the list kernel's loop keeps only its
 // own index live across voxels instead of constants hoisted out of the step.
-template <typename R, int DIM>
+template <typename R, int DIM, bool FOLD = false>
 __device__ __noinline__ void grid_step_voxel_call(const GridDev<R> &gd, const StepT<R> &kst, int cur, int64_t k,
                                                   const Clock &ck)
 {
-    grid_step_voxel<R, DIM, false>(gd, kst, cur, k, ck);
+    grid_step_voxel<R, DIM, FOLD>(gd, kst, cur, k, ck);
 }
 
 // BS = CTA width, MINB = minimum resident CTAs per SM the register allocation

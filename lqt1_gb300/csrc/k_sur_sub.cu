@@ -512,6 +512,62 @@ __global__ void __launch_bounds__(128, MINB) k_sur_substep_warp(GridDev<float> g
     }
 }
 
+// What follows the substep in a step inside a macro step, in one launch: the
+// plain step of the listed voxels, which write their mirror voxels themselves
+// (the first nlist blocks), and the mirror voxels of all other sources and the
+// clock (the rest).  For grids whose mirror voxels are one wave of blocks
+// (kMergeBndPerSM): there the two launches, whose blocks mostly find little to
+// do, took as long as the substep.
+template <int DIM> __global__ void __launch_bounds__(256, 2) k_list_ghost(GridDev<float> gd, StepT<float> kst, int cur, int nlist)
+{
+    if ((int)blockIdx.x < nlist) {
+        const int64_t n = *gd.plist_n;
+        int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+        if (i >= n) return;
+        const Clock ck = gd.clk[cur];
+        for (; i < n; i += (int64_t)nlist * blockDim.x)
+            grid_step_voxel_call<float, DIM, true>(gd, kst, cur, gd.plist[i], ck);
+        return;
+    }
+    const int64_t j = ((int64_t)blockIdx.x - nlist) * blockDim.x + threadIdx.x;
+    if (j == 0) advance_clock(gd, cur);
+    float *V = gd.vg[cur ^ 1];
+    // four entries a thread, their loads in flight together
+    int32_t src[4], dst[4], k[4];
+    if (4 * j + 3 < gd.nbnd) {
+        *reinterpret_cast<int4 *>(src) = reinterpret_cast<const int4 *>(gd.bnd_src)[j];
+        *reinterpret_cast<int4 *>(dst) = reinterpret_cast<const int4 *>(gd.bnd_dst)[j];
+        *reinterpret_cast<int4 *>(k) = reinterpret_cast<const int4 *>(gd.bnd_k)[j];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool on = 4 * j + i < gd.nbnd;
+            src[i] = on ? gd.bnd_src[4 * j + i] : -1;
+            dst[i] = on ? gd.bnd_dst[4 * j + i] : 0;
+            k[i] = on ? gd.bnd_k[4 * j + i] : 0;
+        }
+    }
+    float r[4], v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        r[i] = src[i] >= 0 ? gd.srate[k[i]] : __int_as_float(0x7fc00000);
+        v[i] = src[i] >= 0 ? V[src[i]] : 0.f;      // (not used where the list steps the source)
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (r[i] == r[i]) V[dst[i]] = v[i];
+}
+
+cudaError_t launch_list_ghost(const GridDev<float> &gd, const StepK &k, int cur, int dim, cudaStream_t st)
+{
+    const unsigned nl = grid_list_blocks(gd.ntissue), ng = (unsigned)((gd.nbnd + 1023) / 1024 + (gd.nbnd == 0));
+    const StepT<float> kk = step_as<float>(k);
+    if (dim == 1) k_list_ghost<1><<<nl + ng, 256, 0, st>>>(gd, kk, cur, (int)nl);
+    else if (dim == 2) k_list_ghost<2><<<nl + ng, 256, 0, st>>>(gd, kk, cur, (int)nl);
+    else k_list_ghost<3><<<nl + ng, 256, 0, st>>>(gd, kk, cur, (int)nl);
+    return cudaGetLastError();
+}
+
 // A whole step inside a surrogate macro step on a small grid, in one launch:
 // the V-only step of the surrogate voxels, the plain step of the others, the
 // mirror voxels and (block 0) the clock.  There the time of a step is its

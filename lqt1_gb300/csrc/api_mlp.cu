@@ -36,6 +36,8 @@ struct lqt_mlp {
     int layout = 0;                 // descriptor stride-field assignment (0 = LBO along K)
     // training workspace: gradient slices and loss sums
     int ws_slices = 0;
+    int64_t ws_rows = 0;
+    __nv_bfloat16 *grow = nullptr;  // per batch row: output and pre-activation gradients
     float *Gpart = nullptr;
     double *lossp = nullptr;
     DevMem ws;
@@ -76,22 +78,27 @@ static int grad_step(lqt_mlp *m, const __nv_bfloat16 *X, const float *T, int64_t
     // host waits: lqt_mlp_gradients, lqt_mlp_train_step with a loss)
     if (B <= 0 || B % 16 != 0 || B > (int64_t)INT32_MAX) return fail(LQT_ERR_INVALID, "batch must be a positive multiple of 16");
     const int slices = mlp_grad_slices(B);
-    if (slices > m->ws_slices) {
+    if (slices > m->ws_slices || B > m->ws_rows) {
         m->ws.reset();
+        const int ns = std::max(slices, m->ws_slices);
+        const int64_t nr = std::max(B, m->ws_rows);
         m->ws_slices = 0;
-        if (m->ws.alloc((void **)&m->Gpart, (size_t)slices * kNParam * 4) | m->ws.alloc((void **)&m->lossp, slices * 8))
+        m->ws_rows = 0;
+        if (m->ws.alloc((void **)&m->Gpart, (size_t)ns * kNParam * 4) | m->ws.alloc((void **)&m->lossp, ns * 8) |
+            m->ws.alloc((void **)&m->grow, (size_t)nr * kMlpNBias * 2))
             return LQT_ERR_NOMEM;
-        m->ws_slices = slices;
+        m->ws_slices = ns;
+        m->ws_rows = nr;
     }
     const float b1 = 0.9f, b2 = 0.999f;
     float c1 = 1.f, c2 = 1.f;
-    CK(launch_mlp_grad(X, T, B, m->nvalid, m->dev(), m->Gpart, m->lossp, m->err, m->stream));
+    CK(launch_mlp_grad(X, T, B, m->nvalid, m->dev(), m->Gpart, m->lossp, m->grow, m->err, m->stream));
     if (lr > 0) {
         m->adam_t += 1;
         c1 = 1.f - std::pow(b1, (float)m->adam_t);
         c2 = 1.f - std::pow(b2, (float)m->adam_t);
     }
-    CK(launch_mlp_update(m->Gpart, m->lossp, slices, m->G, m->loss, m->P, m->M, m->V, m->Pb, lr, b1, b2, 1e-8f, c1, c2,
+    CK(launch_mlp_update(m->Gpart, m->lossp, slices, m->grow, B, m->G, m->loss, m->P, m->M, m->V, m->Pb, lr, b1, b2, 1e-8f, c1, c2,
                          m->stream));
     return LQT_OK;
 }

@@ -13,12 +13,18 @@
 // W3 those of a data gradient.  Each CTA writes one slice of the gradients (to
 // which its later tiles, in batches above one tile per SM, are added).
 // k_mlp_update: adds the slices in a fixed order (the same bits on every run),
-// and applies Adam to the FP32 master weights and their BF16 copy.
+// the bias gradients by rows, and applies Adam to the FP32 master weights and
+// their BF16 copy.
+//
+// Sixteen steps amplify the last bit of a sum through the weights' BF16
+// rounding, so the sums have one order that does not depend on how the work is
+// laid out: a weight's by slices of at most 1/128 of the batch (whole half
+// tiles), a bias's by row mod 256 and a tree.
 //
 // What bounds it: one tile's serial chain of five GEMMs and their epilogues
-// (a batch of 8192 is 64 tiles on 152 SMs); tensor time and traffic are below
-// 2 us.  As 17 launches that passed every tile through L2 a batch took 254 us
-// with its input preparation (GB300, 16 batches of 8192); this form takes 41.
+// (a batch of 8192 is 128 half tiles on 152 SMs); tensor time and traffic are
+// below 3 us.  As 17 launches that passed every tile through L2 a batch took
+// 253 us with its input preparation (16 batches of 8192); this form takes 43.
 #include <algorithm>
 
 #include <cuda_bf16.h>
@@ -52,7 +58,6 @@ constexpr uint32_t kNBias = 2 * kMlpHid + kMlpOut;
 constexpr uint32_t kOffBar = kOffBias + kNBias * 4;
 constexpr uint32_t kSmemBytes = kOffBar + 32;
 static_assert(kMlpIn == kMlpOut, "one 48-column tile type");
-static_assert((2048 + 16 * kMlpOut) * 4 <= kT48, "bias sums fit the output-gradient tile");
 static_assert(kOffBias % 16 == 0 && kOffBar % 8 == 0 && kSmemBytes <= 227 * 1024, "shared memory");
 
 // TMEM columns: the pre-activations; the outputs, then the two data gradients
@@ -112,24 +117,6 @@ __device__ __forceinline__ void mma_all(uint32_t d, const Operand &a, bool at, c
                      id, (accum || k > 0) ? 1u : 0u);
 }
 
-// Sum over the tile's 128 rows of two neighbouring columns of a BF16 tile of
-// F features, this thread's share of the rows: [row0, row0 + 128 / parts).
-// The lanes of a warp start at different rows, so that their reads fall into
-// different banks.
-__device__ __forceinline__ float2 column_sums(const uint8_t *tile, int F, int col, int row0, int nrows)
-{
-    float2 s = make_float2(0.f, 0.f);
-    const int turn = (col >> 3) & 7;
-#pragma unroll 8
-    for (int r = 0; r < nrows; ++r) {
-        const int row = row0 + (r & ~7) + ((r + turn) & 7);
-        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(tile + tc::kmaj_off(row, col, F)));
-        s.x += v.x;
-        s.y += v.y;
-    }
-    return s;
-}
-
 __device__ __forceinline__ uint32_t pack2(float a, float b)
 {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -138,12 +125,15 @@ __device__ __forceinline__ uint32_t pack2(float a, float b)
 
 }  // namespace
 
-// part: [gridDim.x][kNP] gradient slices; lossp: [gridDim.x] sums of squared
-// errors over the valid outputs.  dY = 2 (Y - T) / (B nvalid).
+// CTA b takes rows [b chunk, (b + 1) chunk) of the batch.  part: its slice of
+// the weight gradients; lossp: its sum of squared errors over the valid
+// outputs; grow: per row the output and pre-activation gradients (dY, dZ2,
+// dZ1), whose column sums are the bias gradients.  dY = 2 (Y - T) / (B nvalid).
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *__restrict__ X,
                                                           const float *__restrict__ T, int64_t B, int nvalid,
                                                           MlpDev w, float *__restrict__ part,
-                                                          double *__restrict__ lossp, int *err)
+                                                          double *__restrict__ lossp,
+                                                          __nv_bfloat16 *__restrict__ grow, int chunk, int *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ double lred[kThreads / 32];
@@ -175,9 +165,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
     uint32_t phase = 0;
     bool ok = true, first = true;
     float lhi = 0.f, llo = 0.f;                        // this thread's squared errors, a compensated pair
-    // bias gradients: two columns and a share of the rows per thread
-    const int bc = (tid & 63) * 2, bs = tid >> 6;      // hidden: 64 pairs x 8 shares of 16 rows
-    const int oc = (tid % 24) * 2, os = tid / 24;      // outputs: 24 pairs x 16 shares of 8 rows (384 threads)
     float *const out = part + (int64_t)blockIdx.x * kNP;
 
     // writes before it are visible to the MMAs, TMEM reads before it are done
@@ -220,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
         }
     };
     // pre-activation gradient: the work columns times SiLU'(z)
-    auto dact = [&](uint32_t col, const float *b, uint8_t *dst) {
+    auto dact = [&](uint32_t col, const float *b, uint8_t *dst, __nv_bfloat16 *keep) {
         float z[32], v[32];
         load_z(col, b, z);
         tc::tmem_ld32(tl + kColWork + c0, v);
@@ -237,17 +224,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
                 }
                 p[j / 2] = pack2(d[0], d[1]);
             }
-            *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + i, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
+            const uint4 q = make_uint4(p[0], p[1], p[2], p[3]);
+            *reinterpret_cast<uint4 *>(dst + tc::kmaj_off(row, c0 + i, kMlpHid)) = q;
+            if (keep) *reinterpret_cast<uint4 *>(keep + c0 + i) = q;
         }
     };
     // a slice element: the first tile's value, later tiles added to it
     auto put = [&](int i, float x) { out[i] = first ? x : out[i] + x; };
 
-    const int64_t ntiles = (B + kTM - 1) / kTM;
-    for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const int64_t m0 = tile * kTM;
-        const int rows = (int)(B - m0 < kTM ? B - m0 : kTM);
+    const int64_t mend = (int64_t)(blockIdx.x + 1) * chunk < B ? (int64_t)(blockIdx.x + 1) * chunk : B;
+    for (int64_t m0 = (int64_t)blockIdx.x * chunk; m0 < mend && ok; m0 += kTM) {
+        const int rows = (int)(mend - m0 < kTM ? mend - m0 : kTM);
         const bool live = row < rows;
+        __nv_bfloat16 *keep = live ? grow + (m0 + row) * kNBias : nullptr;
         stage_tile(smem + kOffX, X + m0 * kMlpIn, kTM, kMlpIn, rows);
         // this thread's targets
         float tg[16];
@@ -309,7 +298,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
                     }
                     p[j / 2] = pack2(g[0], g[1]);
                 }
-                *reinterpret_cast<uint4 *>(smem + kOffDY + tc::kmaj_off(row, o0 + i, kMlpOut)) = make_uint4(p[0], p[1], p[2], p[3]);
+                const uint4 q = make_uint4(p[0], p[1], p[2], p[3]);
+                *reinterpret_cast<uint4 *>(smem + kOffDY + tc::kmaj_off(row, o0 + i, kMlpOut)) = q;
+                if (keep) *reinterpret_cast<uint4 *>(keep + o0 + i) = q;
             }
         }
         publish();
@@ -320,9 +311,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
             // W3 gradient, transposed: [hidden][output]
             mma_all(tm + kColG3, mnmajor(smem + kOffH2, kMlpHid), true, mnmajor(smem + kOffDY, kMlpOut), true, kMlpOut, kTM, false);
         }
-        const float2 g3 = tid < 384 ? column_sums(smem + kOffDY, kMlpOut, oc, os * 8, 8) : make_float2(0.f, 0.f);
         if (!(ok = arrived())) break;
-        dact(kColZ2, bias + kMlpHid, smem + kOffDZ2);
+        dact(kColZ2, bias + kMlpHid, smem + kOffDZ2, keep ? keep + kMlpOut : nullptr);
         publish();
         if (tid == 0) {
             tc::fence_after();
@@ -331,9 +321,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
             // W2 gradient, transposed: [in][out]
             mma_all(tm + kColG2, mnmajor(smem + kOffH1, kMlpHid), true, mnmajor(smem + kOffDZ2, kMlpHid), true, kMlpHid, kTM, false);
         }
-        const float2 g2 = column_sums(smem + kOffDZ2, kMlpHid, bc, bs * 16, 16);
         if (!(ok = arrived())) break;
-        dact(kColZ1, bias, smem + kOffDZ1);
+        dact(kColZ1, bias, smem + kOffDZ1, keep ? keep + kMlpOut + kMlpHid : nullptr);
         publish();
         if (tid == 0) {
             tc::fence_after();
@@ -341,7 +330,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
             mma_all(tm + kColG1, mnmajor(smem + kOffDZ1, kMlpHid), true, mnmajor(smem + kOffX, kMlpIn), true, kMlpIn, kTM, false);
             tc::mma_commit(bar);
         }
-        const float2 g1 = column_sums(smem + kOffDZ1, kMlpHid, bc, bs * 16, 16);
         if (!(ok = arrived())) break;               // and with it every earlier MMA: the tiles may be overwritten
         // the slice; [in][out] accumulators: a warp writes 32 neighbouring inputs of one output
         {
@@ -357,24 +345,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
 #pragma unroll
                 for (int i = 0; i < 16; ++i) put(kOW1 + row * kMlpIn + o0 + i, v[16 + i]);
             }
-        }
-        // bias gradients: the rows' shares added in order
-        float *cs = reinterpret_cast<float *>(smem + kOffDY);          // (the tiles are free now)
-        cs[bs * 128 + bc] = g1.x;
-        cs[bs * 128 + bc + 1] = g1.y;
-        cs[1024 + bs * 128 + bc] = g2.x;
-        cs[1024 + bs * 128 + bc + 1] = g2.y;
-        if (tid < 384) {
-            cs[2048 + os * 48 + oc] = g3.x;
-            cs[2048 + os * 48 + oc + 1] = g3.y;
-        }
-        __syncthreads();
-        if (tid < 2 * kMlpHid + kMlpOut) {
-            const int n = tid < 2 * kMlpHid ? 8 : 16, step = tid < 2 * kMlpHid ? 128 : 48;
-            const float *q = tid < kMlpHid ? cs + tid : (tid < 2 * kMlpHid ? cs + 1024 + tid - kMlpHid : cs + 2048 + tid - 2 * kMlpHid);
-            float s = 0.f;
-            for (int r = 0; r < n; ++r) s += q[r * step];
-            put(tid < kMlpHid ? kOB1 + tid : (tid < 2 * kMlpHid ? kOB2 + tid - kMlpHid : kOB3 + tid - 2 * kMlpHid), s);
         }
         tc::fence_before();
         __syncthreads();                             // before the next tile's inputs and MMAs
@@ -396,72 +366,139 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_grad(const __nv_bfloat16 *_
     if (warp == 0) tc::tmem_dealloc(tm, kTmemCols);
 }
 
-// G[i] = the slices of parameter i added in slice order; with lr > 0 one Adam
-// step with bias correction c1, c2 on the FP32 master weights and their BF16
-// copy.  loss = sum of lossp.  Bound by the latency of the slices' loads: small
-// blocks over all SMs, 32 loads issued together.
-constexpr int kUpThreads = 64;
+constexpr int kUpThreads = 256;
+constexpr int kUpWeights = (kNP + kUpThreads - 1) / kUpThreads, kUpColumns = kNBias / 8;
+static_assert(kNBias % 8 == 0, "columns in groups of 8");
+
+struct AdamArgs {
+    float *g, *p, *m, *v;
+    __nv_bfloat16 *pb;
+    float lr, b1, b2, eps, c1, c2;
+};
+
+// G = the slices of a weight added in slice order, or the row gradients of a
+// bias added by rows (row mod 256, then a tree: independent of the slices);
+// with lr > 0 one Adam step with bias correction c1, c2 on the FP32 master
+// parameters and their BF16 copy.  loss = sum of lossp.  Bound by latency: a
+// thread's loads are all under way before it adds the first.
 __global__ void __launch_bounds__(kUpThreads) k_mlp_update(const float *__restrict__ part,
                                                            const double *__restrict__ lossp, int slices,
-                                                           float *__restrict__ g, double *__restrict__ loss,
-                                                           float *__restrict__ p, float *__restrict__ m,
-                                                           float *__restrict__ v, __nv_bfloat16 *__restrict__ pb, float lr,
-                                                           float b1, float b2, float eps, float c1, float c2)
+                                                           const __nv_bfloat16 *__restrict__ grow, int64_t B,
+                                                           double *__restrict__ loss, AdamArgs a)
 {
-    const int i = blockIdx.x * kUpThreads + threadIdx.x;
-    if (i < kNP) {
-        float gi = 0.f;
-#pragma unroll 32
-        for (int s = 0; s < slices; ++s) gi += part[(int64_t)s * kNP + i];
-        g[i] = gi;
-        if (lr > 0.f) {
-            const float mi = b1 * m[i] + (1.f - b1) * gi;
-            const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-            m[i] = mi;
-            v[i] = vi;
-            const float pn = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-            p[i] = pn;
-            pb[i] = __float2bfloat16(pn);
+    __shared__ float red[8][kUpThreads];
+    __shared__ double sl[kUpThreads];
+    const int t = threadIdx.x;
+    auto finish = [&](int i, float gi, float p0, float m0, float v0) {
+        a.g[i] = gi;
+        if (a.lr > 0.f) {
+            const float mi = fmaf(1.f - a.b1, gi, __fmul_rn(a.b1, m0));
+            const float vi = fmaf(__fmul_rn(1.f - a.b2, gi), gi, __fmul_rn(a.b2, v0));
+            a.m[i] = mi;
+            a.v[i] = vi;
+            const float pn = p0 - __fmul_rn(a.lr, mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+            a.p[i] = pn;
+            a.pb[i] = __float2bfloat16(pn);
         }
-    } else if (i == kNP) {
+    };
+    if ((int)blockIdx.x < kUpWeights) {
+        constexpr int kAhead = 64;
+        const int i = blockIdx.x * kUpThreads + t;
+        const bool bias = (i >= kOB1 && i < kOW2) || (i >= kOB2 && i < kOW3) || i >= kOB3;
+        if (bias) return;
+        const float p0 = a.p[i], m0 = a.m[i], v0 = a.v[i];
+        float gi = 0.f;
+        for (int s = 0; s < slices; s += kAhead) {
+            float x[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
+                if (s + j < slices) x[j] = part[(int64_t)(s + j) * kNP + i];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j)
+                if (s + j < slices) gi += x[j];
+        }
+        finish(i, gi, p0, m0, v0);
+    } else if ((int)blockIdx.x < kUpWeights + kUpColumns) {
+        const int c0 = ((int)blockIdx.x - kUpWeights) * 8;
+        float acc[8] = {};
+        constexpr int kAhead = 16;
+        for (int64_t r = t; r < B; r += kAhead * kUpThreads) {
+            uint4 q[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                q[u] = r + u * kUpThreads < B ? *reinterpret_cast<const uint4 *>(grow + (r + u * kUpThreads) * kNBias + c0)
+                                              : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&q[u]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f = __bfloat1622float2(h[j]);
+                    acc[2 * j] += f.x;
+                    acc[2 * j + 1] += f.y;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) red[j][t] = acc[j];
+        __syncthreads();
+        for (int w = kUpThreads / 2; w > 0; w >>= 1) {
+            if (t < w) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) red[j][t] += red[j][t + w];
+            }
+            __syncthreads();
+        }
+        if (t < 8) {
+            const int c = c0 + t;
+            const int i = c < kMlpOut ? kOB3 + c : (c < kMlpOut + kMlpHid ? kOB2 + c - kMlpOut : kOB1 + c - kMlpOut - kMlpHid);
+            finish(i, red[t][0], a.p[i], a.m[i], a.v[i]);
+        }
+    } else {
         double s = 0.0;
-        for (int k = 0; k < slices; ++k) s += lossp[k];
-        *loss = s;
+        for (int k = 0; k < slices; k += kUpThreads) {
+            if (k + t < slices) sl[t] = lossp[k + t];
+            __syncthreads();
+            if (t == 0)
+                for (int j = 0; j < kUpThreads && k + j < slices; ++j) s += sl[j];
+            __syncthreads();
+        }
+        if (t == 0) *loss = s;
     }
 }
 
-static int device_sms()
+// Rows per slice, a multiple of half a tile: at most 128 slices, each a CTA of
+// its own; up to 16384 rows a slice is one tile (half of one up to 8192: then
+// twice as many SMs work, each for the time of a tile).
+int mlp_grad_chunk(int64_t B)
 {
-    int dev = 0, nsm = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    return nsm;
+    const int64_t want = std::min<int64_t>(128, std::max<int64_t>(1, B / 64));
+    return (int)(((B + want - 1) / want + 63) / 64 * 64);
 }
-
-// One CTA per SM at most (208 KB of shared memory and all of TMEM, so
-// tcgen05.alloc never waits), one tile per CTA while the batch allows it.
 int mlp_grad_slices(int64_t B)
 {
-    const int64_t tiles = (B + kTM - 1) / kTM;
-    return (int)std::min<int64_t>(tiles, device_sms());
+    const int64_t chunk = mlp_grad_chunk(B);
+    return (int)((B + chunk - 1) / chunk);
 }
 
 cudaError_t launch_mlp_grad(const __nv_bfloat16 *X, const float *T, int64_t B, int nvalid, const MlpDev &w, float *part,
-                            double *lossp, int *err, cudaStream_t st)
+                            double *lossp, __nv_bfloat16 *grow, int *err, cudaStream_t st)
 {
     if (B <= 0) return cudaSuccess;
     static std::atomic<uint64_t> attr_done{0};
     cudaError_t e = tc::smem_attr_once(k_mlp_grad, kSmemBytes, attr_done);
     if (e != cudaSuccess) return e;
-    k_mlp_grad<<<(unsigned)mlp_grad_slices(B), kThreads, kSmemBytes, st>>>(X, T, B, nvalid, w, part, lossp, err);
+    k_mlp_grad<<<(unsigned)mlp_grad_slices(B), kThreads, kSmemBytes, st>>>(X, T, B, nvalid, w, part, lossp, grow,
+                                                                           mlp_grad_chunk(B), err);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_update(const float *part, const double *lossp, int slices, float *g, double *loss, float *p,
-                              float *m, float *v, __nv_bfloat16 *pb, float lr, float b1, float b2, float eps, float c1,
-                              float c2, cudaStream_t st)
+cudaError_t launch_mlp_update(const float *part, const double *lossp, int slices, const __nv_bfloat16 *grow, int64_t B,
+                              float *g, double *loss, float *p, float *m, float *v, __nv_bfloat16 *pb, float lr, float b1,
+                              float b2, float eps, float c1, float c2, cudaStream_t st)
 {
-    k_mlp_update<<<kNP / kUpThreads + 1, kUpThreads, 0, st>>>(part, lossp, slices, g, loss, p, m, v, pb, lr, b1, b2, eps, c1, c2);
+    const AdamArgs a{g, p, m, v, pb, lr, b1, b2, eps, c1, c2};
+    k_mlp_update<<<kUpWeights + kUpColumns + 1, kUpThreads, 0, st>>>(part, lossp, slices, grow, B, loss, a);
     return cudaGetLastError();
 }
 

@@ -33,14 +33,16 @@ cudaError_t launch_mlp_infer_tc(const __nv_bfloat16 *X, float *Y, const MlpDev &
                                 cudaStream_t st);
 
 // Training (k_mlp_train.cu): gradient slices of a batch, one per CTA
-// (mlp_grad_slices of them, kMlpNParam32 floats each, and one loss sum each),
-// and their ordered sum with, for lr > 0, one Adam step.
+// (mlp_grad_slices of them, kMlpNParam32 floats each, and one loss sum each)
+// and the row gradients (kMlpNBias values a row); and their ordered sums with,
+// for lr > 0, one Adam step.
 constexpr int kMlpNParam32 = 2 * kMlpIn * kMlpHid + kMlpHid * kMlpHid + 2 * kMlpHid + kMlpOut;
+constexpr int kMlpNBias = 2 * kMlpHid + kMlpOut;
 int mlp_grad_slices(int64_t B);
 cudaError_t launch_mlp_grad(const __nv_bfloat16 *X, const float *T, int64_t B, int nvalid, const MlpDev &w, float *part,
-                            double *lossp, int *err, cudaStream_t st);
-cudaError_t launch_mlp_update(const float *part, const double *lossp, int slices, float *g, double *loss, float *p,
-                              float *m, float *v, __nv_bfloat16 *pb, float lr, float b1, float b2, float eps, float c1,
-                              float c2, cudaStream_t st);
+                            double *lossp, __nv_bfloat16 *grow, int *err, cudaStream_t st);
+cudaError_t launch_mlp_update(const float *part, const double *lossp, int slices, const __nv_bfloat16 *grow, int64_t B,
+                              float *g, double *loss, float *p, float *m, float *v, __nv_bfloat16 *pb, float lr, float b1,
+                              float b2, float eps, float c1, float c2, cudaStream_t st);
 
 }  // namespace lqt

@@ -54,7 +54,7 @@ enum {
 /* ---- precision forms --------------------------------------------------- */
 enum {
     LQT_FP64 = 0,               /* plain FP64 everywhere (the reference's arithmetic) */
-    LQT_MIXED = 1               /* FP32 gates/currents/diffusion, FP64 concentrations */
+    LQT_MIXED = 1               /* FP32; concentrations as pairs of FP32 (hi + lo) */
 };
 
 /* ---- state order (SingleCell/TPORd.cc:200-252) ------------------------- */
@@ -300,7 +300,9 @@ int lqt_sim_tissue_index(const lqt_sim *s, int64_t *grid_index_host);
 
 /* Advance nsteps of dt.  Simulated time accumulates as `time += dt` in FP64,
  * as the reference drivers do (OneD.cc:317).  Returns when the steps have run
- * on the device. */
+ * on the device.  (Blocks of a small grid wait for one another inside one
+ * launch; should such a wait run out, this call, lqt_sim_sync and
+ * lqt_sim_check return LQT_ERR_CUDA and the run is not valid.) */
 int lqt_sim_step(lqt_sim *s, int64_t nsteps);
 /* The same steps, enqueued on the simulation's stream without waiting: a host
  * loop that issues one step at a time (with a read-back per step) keeps the
@@ -641,7 +643,9 @@ int lqt_sim_surrogate_rejections(lqt_sim *s, int64_t *counts);
  * tile's copies of every CTA, so that tile's bounded mbarrier wait runs out;
  * wait_limit sets the polls per wait (0 = the default).  The CTA then sets bit
  * 1 of the surrogate error word, lets its copies in flight land and returns;
- * lqt_sim_check reports it and the context stays usable.  (0, 0) restores. */
+ * lqt_sim_check reports it and the context stays usable.  On a small grid
+ * without a surrogate, block 0 publishes none of its steps, so its neighbours'
+ * waits run out and the step calls report it.  (0, 0) restores. */
 int lqt_sim_set_wait_test(lqt_sim *s, int32_t skip_first_copy, uint32_t wait_limit);
 
 /* ======================================================================== *

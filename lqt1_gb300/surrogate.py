@@ -1,9 +1,9 @@
 """The learned surrogate's network on the GPU (lqt_mlp_*).
 
 48 -> 128 -> 128 -> 48 MLP with SiLU, BF16 weights, FP32 accumulation.
-Inference runs on the tcgen05 tensor cores (TMEM accumulators); training uses
-hand-written BF16 mma.sync GEMMs and Adam.  Device buffers are torch tensors
-owned by the caller.
+Inference and training (forward, backward and weight gradients, with Adam) run
+on the tcgen05 tensor cores with TMEM accumulators.  Device buffers are torch
+tensors owned by the caller.
 """
 from __future__ import annotations
 

@@ -192,14 +192,15 @@ int lqt_initial_state(double v0, double *state40_host)
 // ===========================================================================
 // Cells (Cell interface for N cells)
 // Up to kMappedCells cells keep what the interface sets and reads per cell
-// (inputs, V, dV/dt, currents: 10 doubles) in page-locked host memory that the
-// update kernel addresses: setting and reading are then plain memory accesses,
-// and the loop set inputs / update / read V / read currents costs its one
-// launch.  The kernel touches them once per update, over the link to the host:
-// 21 us an iteration against 56 with device arrays at 1 cell, 44 against 69 at
-// 4096, 66 against 80 at 8192, 109 against 97 at 16384.
+// (inputs, V, dV/dt, currents, and the 40 states on their way in or out) in
+// page-locked host memory that the kernels address: setting and reading are
+// then plain memory accesses, and the loop set inputs / update / read V / read
+// currents costs its one launch.  Microseconds an iteration, mapped against
+// device arrays: that loop 21 / 54 at 1 cell, 24 / 59 at 512; update and all
+// states 28 / 36 at 1, 43 / 43 at 512.  Beyond it the states' way over the
+// link to the host is the longer one (110 / 96 at 8192).
 namespace {
-constexpr int64_t kMappedCells = 8192;
+constexpr int64_t kMappedCells = 512;
 }
 
 struct lqt_cells {
@@ -210,7 +211,7 @@ struct lqt_cells {
     uint8_t *ctype = nullptr;
     double *ist = nullptr, *dvgap = nullptr, *dvdt = nullptr, *aos = nullptr, *cur = nullptr;   // device addresses
     double *vout = nullptr;
-    double *hio = nullptr;          // mapped: ist[n], dvgap[n], V[n], dV/dt[n], currents[6n]
+    double *hio = nullptr;          // mapped: ist[n], dvgap[n], V[n], dV/dt[n], currents[6n], states[40n]
     ~lqt_cells()
     {
         if (hio) cudaFreeHost(hio);
@@ -246,7 +247,7 @@ int lqt_cells_create(int64_t n, const uint8_t *types_host, int precision, const 
     rc = 0;
     double *io = nullptr;           // the same ten doubles per cell as the device addresses them
     if (n <= kMappedCells) {
-        if (cudaHostAlloc((void **)&c->hio, n * 10 * 8, cudaHostAllocMapped) != cudaSuccess ||
+        if (cudaHostAlloc((void **)&c->hio, n * 50 * 8, cudaHostAllocMapped) != cudaSuccess ||
             cudaHostGetDevicePointer((void **)&io, c->hio, 0) != cudaSuccess) {
             delete c;
             return fail(LQT_ERR_NOMEM, "lqt_cells_create: page-locked host memory");
@@ -261,7 +262,9 @@ int lqt_cells_create(int64_t n, const uint8_t *types_host, int precision, const 
     c->vout = io + 2 * n;
     c->dvdt = io + 3 * n;
     c->cur = io + 4 * n;
-    rc = rc | c->mem.alloc((void **)&c->ctype, n) | c->mem.alloc((void **)&c->aos, n * 40 * 8) | c->mem.alloc(&c->v, c->ld * rsz) |
+    if (c->hio) c->aos = io + 10 * n;
+    else rc = rc | c->mem.alloc((void **)&c->aos, n * 40 * 8);
+    rc = rc | c->mem.alloc((void **)&c->ctype, n) | c->mem.alloc(&c->v, c->ld * rsz) |
          c->mem.alloc(&c->gate, c->ld * rsz * kNGate) | c->mem.alloc((void **)&c->conc, c->ld * 8 * kNConc) |
          c->mem.alloc((void **)&c->modelk, sizeof(ModelK));
     if (rc) {
@@ -274,7 +277,8 @@ int lqt_cells_create(int64_t n, const uint8_t *types_host, int precision, const 
     cudaError_t e = cudaMemcpyAsync(c->ctype, types_host, n, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->modelk, &mk, sizeof(mk), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess && !c->hio) e = cudaMemsetAsync(io, 0, n * 10 * 8, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c->aos, init.data(), n * 320, cudaMemcpyHostToDevice, c->stream);
+    if (c->hio) std::memcpy(c->hio + 10 * n, init.data(), n * 320);
+    else if (e == cudaSuccess) e = cudaMemcpyAsync(c->aos, init.data(), n * 320, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
         e = precision == LQT_FP64 ? launch_pack<double>(c->aos, c->soa<double>(), n, c->stream)
                                   : launch_pack<float>(c->aos, c->soa<float>(), n, c->stream);
@@ -294,7 +298,8 @@ int64_t lqt_cells_count(const lqt_cells *c) { return c ? c->n : -1; }
 int lqt_cells_set_state(lqt_cells *c, const double *state_host)
 {
     if (!c || !state_host) return fail(LQT_ERR_INVALID, "lqt_cells_set_state: NULL");
-    CK(cudaMemcpyAsync(c->aos, state_host, c->n * 320, cudaMemcpyHostToDevice, c->stream));
+    if (c->hio) std::memcpy(c->hio + 10 * c->n, state_host, c->n * 320);
+    else CK(cudaMemcpyAsync(c->aos, state_host, c->n * 320, cudaMemcpyHostToDevice, c->stream));
     CK(c->precision == LQT_FP64 ? launch_pack<double>(c->aos, c->soa<double>(), c->n, c->stream)
                                 : launch_pack<float>(c->aos, c->soa<float>(), c->n, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -309,8 +314,9 @@ int lqt_cells_get_state(lqt_cells *c, double *state_host)
     if (!c || !state_host) return fail(LQT_ERR_INVALID, "lqt_cells_get_state: NULL");
     CK(c->precision == LQT_FP64 ? launch_unpack<double>(c->soa<double>(), c->aos, c->n, c->stream)
                                 : launch_unpack<float>(c->soa<float>(), c->aos, c->n, c->stream));
-    CK(cudaMemcpyAsync(state_host, c->aos, c->n * 320, cudaMemcpyDeviceToHost, c->stream));
+    if (!c->hio) CK(cudaMemcpyAsync(state_host, c->aos, c->n * 320, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (c->hio) std::memcpy(state_host, c->hio + 10 * c->n, c->n * 320);
     return LQT_OK;
 }
 

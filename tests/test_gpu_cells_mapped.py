@@ -6,7 +6,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-EDGE = 8192
+EDGE = 512
 
 
 @pytest.fixture(scope="module")

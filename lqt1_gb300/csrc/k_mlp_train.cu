@@ -2,16 +2,17 @@
 // (48 -> 128 -> 128 -> 48, SiLU, BF16 operands, FP32 accumulation) in two
 // kernels.
 //
-// k_mlp_grad: forward, loss gradient, backward and weight gradients of 128
-// batch rows per CTA without leaving the SM.  The weights (56 KB), the row
+// k_mlp_grad: forward, loss gradient, backward and weight gradients of up to
+// 128 batch rows per CTA without leaving the SM.  The weights (56 KB), the row
 // tile's inputs, both hidden tiles and the three gradient tiles live in shared
 // memory (208 KB), the accumulators in TMEM (480 of 512 columns).  Every tile
 // is stored once, as 8 x 8 core matrices of 8 rows x 16 bytes: read K-major it
 // is the operand of a forward or data-gradient GEMM, read MN-major (the
 // descriptor's strides exchanged, the transpose bits of the instruction set)
 // the same bytes are the transposed operand of a weight gradient, and W2 and
-// W3 those of a data gradient.  Each CTA writes one slice of the gradients (to
-// which its later tiles, in batches above one tile per SM, are added).
+// W3 those of a data gradient.  Each CTA writes one slice of the weight gradients
+// (to which its later tiles, in batches above 16384 rows, are added) and its
+// rows' output and pre-activation gradients.
 // k_mlp_update: adds the slices in a fixed order (the same bits on every run),
 // the bias gradients by rows, and applies Adam to the FP32 master weights and
 // their BF16 copy.

@@ -14,7 +14,8 @@
 // and its mirror voxels; publish.  A block's fifth warp waits, publishes and
 // keeps the clock, so that no voxel does.  The wait also guards the other
 // grid: a block that has published step s has read everything of step s - 1,
-// whose grid the next V goes to, and the relation is symmetric.
+// whose grid the next V goes to, and the relation is symmetric.  Blocks that
+// exchange no V, directly or through others, are not ordered by it.
 //
 // The launch is cooperative: every block is resident, so every wait ends.  It
 // is bounded all the same; one that runs out sets *err, the blocks leave, and
@@ -39,6 +40,14 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
 __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// A bounded wait until a block has published `step`.
+__device__ __forceinline__ bool reached(const uint32_t *flag, uint32_t step, uint32_t limit)
+{
+    uint32_t polls = 0;
+    while ((int32_t)(ld_acquire(flag) - step) < 0 && polls < limit) ++polls;
+    return polls < limit;
 }
 
 // What a voxel's diffusion needs besides V, for the whole launch.
@@ -102,15 +111,18 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
         const int2 dep = a.dep[b];
         const uint32_t base = a.flags[b];
         const uint32_t limit = gd.sub_wait_limit ? gd.sub_wait_limit : kPersistPolls;
+        // Block 0 leaves the clock of the launch's end.  After an even number of
+        // steps that is the slot every block starts from, so all of them, not only
+        // the blocks it exchanges V with, must have begun by then: a block has read
+        // the clock before it publishes its first step.
+        const bool last_clock = b == 0 && (a.nsteps & 1) == 0;
         for (int s = 0; s < a.nsteps; ++s) {
             if (lane == 0) clk[(s + 1) % 3] = next_clock(gd, clk[s % 3]);
             bool ok = true;
             if (s > 0) {
-                for (int i = dep.x + lane; i <= dep.y; i += 32) {
-                    uint32_t polls = 0;
-                    while ((int32_t)(ld_acquire(a.flags + i) - (base + s)) < 0 && polls < limit) ++polls;
-                    ok = ok && polls < limit;
-                }
+                for (int i = dep.x + lane; i <= dep.y; i += 32) ok = reached(a.flags + i, base + s, limit) && ok;
+                if (last_clock && s == a.nsteps - 1)
+                    for (int i = lane; i < (int)gridDim.x; i += 32) ok = reached(a.flags + i, base + 1, limit) && ok;
             }
             ok = __all_sync(0xffffffffu, ok);
             if (lane == 0) {

@@ -14,7 +14,8 @@
 //   * the terms are arranged as in tpord_f32.cuh (rates for time constants,
 //     shared reciprocals and exponentials), without its bounds: exponentials
 //     saturate at 2^+-100, far outside their effect on any term, and products
-//     of several stay finite.
+//     of several stay finite; a shared reciprocal's product of a calcium
+//     concentration is kept off zero by 1e-60 (kTinyD).
 // Each of these is within a few units of 2^-53, as the expressions they stand
 // for; results agree with the oracle to 1e-12 and better.  Measured (GB300):
 // shell of 78k voxels 684 -> 297 us a step.
@@ -91,14 +92,17 @@ static __device__ const double kEx2Table[256] = {
     0x1.fa7c1819e90d8p+0, 0x1.fbdba3692d514p+0, 0x1.fd3c22b8f71f1p+0, 0x1.fe9d96b2a23d9p+0
 };
 
-// 2^x, saturating at 2^+-100 (NaN stays NaN).  |x| is first held at 1000 by
-// its high word, so that 256 x fits the sum's low word.
+constexpr double kTinyD = 1e-60;
+
+// 2^x, saturating at 2^+-100, at infinities too (NaN stays NaN: x comes from
+// arithmetic, so a NaN's high word is above infinity's).  |x| is first held at
+// 1000 by its high word, so that 256 x fits the sum's low word.
 __device__ __forceinline__ double ex2d(double x)
 {
     constexpr double shift = 26388279066624.0;   // 1.5 * 2^44: the sum's low word is round(256 x)
     constexpr int top = 0x408F4000;              // high word of 1000.0
     const int hx = __double2hiint(x), ha = hx & 0x7fffffff;
-    const bool far = (unsigned)(ha - top) < (unsigned)(0x7ff00000 - top);
+    const bool far = (unsigned)(ha - top) <= (unsigned)(0x7ff00000 - top);
     x = __hiloint2double(far ? (hx & (int)0x80000000) | top : hx, __double2loint(x));
     const double t = x + shift;
     const double r = x - (t - shift);
@@ -111,7 +115,7 @@ __device__ __forceinline__ double ex2d(double x)
     return fma(T, p * r, T);
 }
 
-// 1 / x
+// 1 / x, x finite and not zero
 __device__ __forceinline__ double rcpd(double x)
 {
     double r;
@@ -120,8 +124,9 @@ __device__ __forceinline__ double rcpd(double x)
     return fma(r, fma(e, e, e), r);
 }
 
-// log2(x), x normal and positive (NaN for others): an FP32 estimate from x's high word, rounded
-// to k/256; x 2^(-k/256) = 1 + d with |d| < 1.4e-3
+// log2(x): an FP32 estimate from x's high word, rounded to k/256;
+// x 2^(-k/256) = 1 + d with |d| < 1.4e-3.  -infinity at zero (and subnormal x),
+// infinity at infinity, NaN for the others that are not normal and positive.
 __device__ __forceinline__ double lg2d(double x)
 {
     const int hi = __double2hiint(x);
@@ -135,7 +140,8 @@ __device__ __forceinline__ double lg2d(double x)
     const double p = fma(fma(fma(fma(0.2, d, -0.25), d, 1.0 / 3.0), d, -0.5), d, 1.0);
     // k/256 exactly, by the sum that ex2d takes apart
     const double kd = __hiloint2double(0x42B80000 + (k >> 31), k) - 26388279066624.0;
-    return (unsigned)(hi - 0x00100000) < 0x7fe00000u ? fma(p * d, 1.4426950408889634, kd) : __hiloint2double(0x7ff80000, 0);
+    const int end = (hi & 0x7fffffff) < 0x00100000 ? (int)0xfff00000 : (hi == 0x7ff00000 ? hi : 0x7ff80000);
+    return (unsigned)(hi - 0x00100000) < 0x7fe00000u ? fma(p * d, 1.4426950408889634, kd) : __hiloint2double(end, 0);
 }
 
 // exp((v + a) / k)
@@ -185,7 +191,7 @@ __device__ __forceinline__ void tpord_step_f64(CellState<double> &c, int ctype, 
 
     // CaMK, TPORd.cc:430-433; 1/cass and 1/(cass + KmCaM) from one reciprocal
     const double cq = cass + 0.0015;
-    const double r_cc = rcpd(cass * cq);
+    const double r_cc = rcpd(fma(cass, cq, kTinyD));
     const double rcass = r_cc * cq;
     const double CaMKb = 0.05 * (1.0 - c.CaMKt) * (r_cc * cass) * cass;
     const double CaMKa = CaMKb + c.CaMKt;
@@ -524,7 +530,7 @@ __device__ __forceinline__ void tpord_step_f64(CellState<double> &c, int ctype, 
         // 1/(1 + (1.5/cajsr)^8) and 1/cajsr from one reciprocal
         const double j2 = cajsr * cajsr, j4 = j2 * j2, j8 = (j4 * j4);
         const double dj = j8 + 25.62890625;
-        const double r = rcpd(dj * cajsr);
+        const double r = rcpd(fma(dj, cajsr, kTinyD));
         const double rel = (mid ? 1.7 : 1.0) * -ICaL * j8 * (r * cajsr);
         // 1/tau_rel; tau_rel below 0.005, negative ones too (cajsr < 0), is 0.005: the
         // sign bit makes a negative rate's high word the larger unsigned number

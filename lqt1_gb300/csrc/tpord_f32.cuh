@@ -458,7 +458,8 @@ __device__ __forceinline__ void tpord_step_f32(CellState<float> &c, int ctype, c
     const float Jtr = mulp(cdiff(c.cansr, c.cajsr), 0.01f);
     {
         // 1/(1 + (1.5/cajsr)^8) and 1/cajsr from one reciprocal
-        const float j2 = cajsr * cajsr, j4 = j2 * j2, j8 = mulp(j4, j4);
+        // (bounded: beyond 200 mM the first is 1, and j8 itself would overflow from 65,000 on)
+        const float j2 = cajsr * cajsr, j4 = j2 * j2, j8 = fminf(mulp(j4, j4), 1e18f);
         const float dj = j8 + 25.62890625f;
         const float r = rcpf_(fmaf(dj, cajsr, kTiny));
         const float rel = (mid ? 1.7f : 1.0f) * -ICaL * j8 * (r * cajsr);

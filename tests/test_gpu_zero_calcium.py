@@ -1,6 +1,7 @@
 """A calcium concentration of exactly zero (an empty sarcoplasmic store, subspace
-or cytosol) in both forms of the cell step against the FP64 oracle: the
-reference's formulas are finite there (1 / (1 + K / 0) = 0).
+or cytosol), or a store's far above any real one, in both forms of the cell step
+against the FP64 oracle: the reference's formulas are finite there
+(1 / (1 + K / 0) = 0, 1 / (1 + (1.5 / c)^8) = 1).
 
 Tolerances: those of the same quantities in test_gpu_step_f32.py and
 test_gpu_step_f64.py."""
@@ -50,6 +51,26 @@ def test_zero_calcium(which, zero, precision):
     for j in (37, 38):
         scale = np.maximum(np.abs(ref[:, j]), np.abs(s0[:, j]))
         assert np.all(np.abs(got[:, j] - ref[:, j]) <= 4e-5 * np.maximum(scale, 1e-9))
+
+
+@pytest.mark.parametrize("precision", [lq.MIXED, lq.FP64])
+@pytest.mark.parametrize("cajsr", [199.0, 201.0, 6e4, 7e4, 1e7, -1e7])
+def test_large_store(cajsr, precision):
+    s0 = orc.random_states(64, seed=22)
+    s0[:, 9:] = s0[:, 9:].astype(np.float32)
+    s0[:, CAJSR] = cajsr
+    types = np.arange(64).astype(np.uint8) % 5
+    ref = orc.cells_update(s0.copy(), types, orc.model("default"), nsteps=1)
+    c = lq.TPORdCells(types, precision=precision, model="default")
+    c.set_state(s0)
+    c.update(1)
+    got = c.get_state()
+    c.close()
+    assert np.all(np.isfinite(ref)) and np.all(np.isfinite(got))
+    tol = 4e-5 if precision == lq.MIXED else 1e-12
+    for j in (CAJSR, 37, 38):
+        scale = np.maximum(np.abs(ref[:, j]), np.abs(s0[:, j]))
+        assert np.all(np.abs(got[:, j] - ref[:, j]) <= tol * np.maximum(scale, 1e-9))
 
 
 @pytest.mark.parametrize("precision", [lq.MIXED, lq.FP64])

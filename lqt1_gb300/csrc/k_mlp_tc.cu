@@ -83,13 +83,16 @@ __device__ __forceinline__ float mlp_rcp(float x)
 // once by its remainder, which an FMA gives exactly (Markstein's correction),
 // so it is within 2^-40 or so of the division before it is rounded.  (The
 // reciprocals and quotients are carried negated: the remainder is then one
-// FMA.)  exp(-x) is held at 1e18 (x < -41): the product of two stays finite,
-// and the result there, below 1e-16, is lost beside any other activation.
-__device__ __forceinline__ uint32_t silu2_bf16(uint64_t x)
+// FMA.)  That holds for |x| up to 43, where the product of two denominators,
+// at most e^86, and its reciprocal are normal numbers; top keeps the largest
+// |x| (a NaN stays), for silu_plain to see what is beyond.
+__device__ __forceinline__ uint32_t silu2_bf16(uint64_t x, float &top)
 {
-    float a0, a1, d0, d1, q0, q1;
+    float x0, x1, a0, a1, d0, d1, q0, q1;
+    tc::split2(x, x0, x1);
+    asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(top) : "f"(fabsf(x0)), "f"(fabsf(x1)));
     tc::split2(tc::mul2(x, tc::pair2(-1.4426950408889634f, -1.4426950408889634f)), a0, a1);
-    const uint64_t d = tc::add2(tc::pair2(fminf(mlp_ex2(a0), 1e18f), fminf(mlp_ex2(a1), 1e18f)), tc::pair2(1.0f, 1.0f));
+    const uint64_t d = tc::add2(tc::pair2(mlp_ex2(a0), mlp_ex2(a1)), tc::pair2(1.0f, 1.0f));
     tc::split2(d, d0, d1);
     const float r = mlp_rcp(d0 * -d1);
     const uint64_t nr = tc::pair2(r * d1, r * d0);
@@ -97,6 +100,20 @@ __device__ __forceinline__ uint32_t silu2_bf16(uint64_t x)
     nq = tc::fma2(tc::fma2(nq, d, x), nr, nq);
     tc::split2(nq, q0, q1);
     const __nv_bfloat162 h = __floats2bfloat162_rn(-q0, -q1);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// Whether the values behind top are all in silu2_bf16's range.  (One maximum of
+// three operands a pair costs what bounding the two exponentials did, 155 us for
+// a million rows; the extremes of the exponentials or of x with its sign, which
+// would let large positive x pass, take 163.)
+__device__ __forceinline__ bool silu_plain(float top) { return top <= 43.f; }
+
+// The division itself, for the others: 0 for large negative x, x for large
+// positive, infinities and NaN as the formula gives them.
+__device__ __forceinline__ uint32_t silu2_div(float x0, float x1)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x0 / (1.0f + __expf(-x0)), x1 / (1.0f + __expf(-x1)));
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
@@ -209,6 +226,7 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_infer_tc(const __nv_bf
             // hidden layer: TMEM -> bias, SiLU -> BF16 operand (over the bytes
             // of the operand that the finished MMA no longer needs)
             const float4 *bs = reinterpret_cast<const float4 *>(bias + layer * kMlpHid);
+            float top = 0.f;
 #pragma unroll 1
             for (int c = 0; c < kMlpHid; c += 32) {
                 float v[32];
@@ -220,10 +238,26 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_infer_tc(const __nv_bf
                     for (int i = 0; i < 2; ++i) {
                         const float4 b = bs[(c >> 2) + q * 2 + i];
                         const float *u = v + q * 8 + 4 * i;
-                        p[2 * i] = silu2_bf16(tc::add2(tc::pair2(u[0], u[1]), tc::pair2(b.x, b.y)));
-                        p[2 * i + 1] = silu2_bf16(tc::add2(tc::pair2(u[2], u[3]), tc::pair2(b.z, b.w)));
+                        p[2 * i] = silu2_bf16(tc::add2(tc::pair2(u[0], u[1]), tc::pair2(b.x, b.y)), top);
+                        p[2 * i + 1] = silu2_bf16(tc::add2(tc::pair2(u[2], u[3]), tc::pair2(b.z, b.w)), top);
                     }
                     *reinterpret_cast<uint4 *>(xh + tc::kmaj_off(t, c + q * 8, kMlpHid)) = make_uint4(p[0], p[1], p[2], p[3]);
+                }
+            }
+            // (a warp whose rows hold a value out of range: its columns again)
+            if (__any_sync(0xffffffffu, !silu_plain(top))) {
+#pragma unroll 1
+                for (int c = 0; c < kMlpHid; c += 16) {
+                    float v[16];
+                    tc::tmem_ld16(t_acc + c, v);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float4 b = bs[(c >> 2) + q * 2], e = bs[(c >> 2) + q * 2 + 1];
+                        const float *u = v + q * 8;
+                        *reinterpret_cast<uint4 *>(xh + tc::kmaj_off(t, c + q * 8, kMlpHid)) =
+                            make_uint4(silu2_div(u[0] + b.x, u[1] + b.y), silu2_div(u[2] + b.z, u[3] + b.w),
+                                       silu2_div(u[4] + e.x, u[5] + e.y), silu2_div(u[6] + e.z, u[7] + e.w));
+                    }
                 }
             }
             tc::fence_before();

@@ -73,13 +73,14 @@ static_assert(kNP == kMlpNParam32, "parameter block");
 
 // 1 / (1 + exp(-z)): the hardware reciprocal with one Newton step on its exact
 // residual (an FMA), which is the correctly rounded quotient but for about one
-// argument in a million; exp(-z) is held at 1e30, where the result is 0 beside
-// anything it is added to.
+// argument in a million.  exp(-z) is held at the largest finite value, whose
+// reciprocal is flushed to 0 (as from z = -87 on), so that z * sigm(z) is 0 for
+// any z below.
 __device__ __forceinline__ float sigm(float z)
 {
     float e, r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
-    const float d = 1.0f + fminf(e, 1e30f);
+    const float d = 1.0f + fminf(e, 3.402823466e38f);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(fmaf(-d, r, 1.0f), r, r);
 }

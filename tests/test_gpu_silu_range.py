@@ -74,3 +74,23 @@ def test_infinite_activation_stays_infinite():
     y = torch.empty(130, OUT, device="cuda")
     m.infer(X.bfloat16().cuda(), y)
     assert bool((y == float("-inf")).all())
+
+
+def test_training():
+    """The loss and the second layer's bias gradient with one activation at a
+    large negative pre-activation, where SiLU and its derivative are 0."""
+    from lqt1_gb300.surrogate import Mlp
+    m = Mlp(seed=1)
+    m.set_params(network(False, 0))
+    for x in (-3e38, -3e32, -1e30, -1e20, -200.0, -88.0, -60.0):
+        X = torch.zeros(128, IN)
+        X[:, 0] = x
+        t = torch.zeros(128, OUT)
+        loss = m.gradients(X.bfloat16().cuda(), t.cuda())
+        g = m.grads()
+        # y = 50 in every valid column (nvalid = 38 of the 48): loss is their mean square
+        assert abs(loss / 2500.0 - 1.0) <= 4 * 2.0 ** -9 * 2, x
+        b1 = g[HID * IN: HID * IN + HID]
+        assert np.all(np.abs(b1) <= 1e-18), x       # SiLU'(-60) = -5e-25, over 128 rows
+        b2 = g[HID * IN + HID + HID * HID: HID * IN + HID + HID * HID + HID]
+        assert np.all(np.isfinite(g)) and b2[3] > 0 and np.all(b2[np.arange(HID) != 3] == 0.0)

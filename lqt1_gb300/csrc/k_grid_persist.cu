@@ -37,17 +37,15 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p)
+{
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// A bounded wait until a block has published `step`.
-__device__ __forceinline__ bool reached(const uint32_t *flag, uint32_t step, uint32_t limit)
-{
-    uint32_t polls = 0;
-    while ((int32_t)(ld_acquire(flag) - step) < 0 && polls < limit) ++polls;
-    return polls < limit;
 }
 
 // What a voxel's diffusion needs besides V, for the whole launch.
@@ -103,26 +101,27 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
     // three clocks: the detector of step s runs beside the making of s + 2's
     __shared__ Clock clk[3];
     __shared__ int go;
+    __shared__ uint32_t base;             // steps published when the launch begins
     const int t = threadIdx.x, b = blockIdx.x;
-    if (t == kPersistBlock) clk[0] = gd.clk[cur];
+    const uint32_t limit = gd.sub_wait_limit ? gd.sub_wait_limit : kPersistPolls;
+    if (t == kPersistBlock) {
+        clk[0] = gd.clk[cur];
+        base = a.flags[b];
+    }
     __syncthreads();
     if (t >= kPersistBlock) {
         const int lane = t - kPersistBlock;
         const int2 dep = a.dep[b];
-        const uint32_t base = a.flags[b];
-        const uint32_t limit = gd.sub_wait_limit ? gd.sub_wait_limit : kPersistPolls;
-        // Block 0 leaves the clock of the launch's end.  After an even number of
-        // steps that is the slot every block starts from, so all of them, not only
-        // the blocks it exchanges V with, must have begun by then: a block has read
-        // the clock before it publishes its first step.
-        const bool last_clock = b == 0 && (a.nsteps & 1) == 0;
+        const uint32_t base0 = base;
+        bool ok = true;
         for (int s = 0; s < a.nsteps; ++s) {
             if (lane == 0) clk[(s + 1) % 3] = next_clock(gd, clk[s % 3]);
-            bool ok = true;
             if (s > 0) {
-                for (int i = dep.x + lane; i <= dep.y; i += 32) ok = reached(a.flags + i, base + s, limit) && ok;
-                if (last_clock && s == a.nsteps - 1)
-                    for (int i = lane; i < (int)gridDim.x; i += 32) ok = reached(a.flags + i, base + 1, limit) && ok;
+                for (int i = dep.x + lane; i <= dep.y; i += 32) {
+                    uint32_t polls = 0;
+                    while ((int32_t)(ld_acquire(a.flags + i) - (base0 + s)) < 0 && polls < limit) ++polls;
+                    ok = ok && polls < limit;
+                }
             }
             ok = __all_sync(0xffffffffu, ok);
             if (lane == 0) {
@@ -135,10 +134,12 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
             // (a failure-path test keeps block 0 from publishing)
             if (lane == 0 && !(b == 0 && gd.sub_skip_copy)) {
                 __threadfence();
-                st_release(a.flags + b, base + s + 1);
+                st_release(a.flags + b, base0 + s + 1);
             }
         }
-        if (b == 0 && lane == 0) gd.clk[(cur + a.nsteps) & 1] = clk[a.nsteps % 3];
+        // Block 0 leaves the clock of the launch's end, once every block has read
+        // the one of its beginning (the voxels' threads look, below).
+        if (b == 0 && __syncthreads_and(ok) && lane == 0) gd.clk[(cur + a.nsteps) & 1] = clk[a.nsteps % 3];
         return;
     }
 
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
             for (int i = 0; i < 3; ++i) d.B[i] = gd.b3[3 * k + i];
         }
     }
+    bool ran = true;
     for (int s = 0; s < a.nsteps; ++s) {
         const Clock &ck = clk[s % 3];
         const float vc = c.v;
@@ -175,7 +177,10 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
             tpord_update(c, ctl & kCtlType, gd.model, kst, grid_stim(gd, ck, ctl, k), 0.f, &o);
         }
         __syncthreads();
-        if (!go) break;
+        if (!go) {
+            ran = false;
+            break;
+        }
         if (on) {
             const float du = persist_du<DIM>(gd, gd.vg[(cur + s) & 1], g, vc, d);
             c.v = fmaf(o.dvdt + du, kst.dt, vc);
@@ -188,6 +193,25 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
         }
     }
     if (on) store_cell(c, gd.s, k);
+    if (b == 0) {
+        // After an even number of steps the slot of the end is the one that every
+        // block starts from.  Blocks that exchange no V with this one are not
+        // ordered with it, so all must have published their first step, which
+        // they do after reading the clock.
+        bool begun = ran;
+        if (ran && (a.nsteps & 1) == 0) {
+            const uint32_t first = base + 1;
+            begun = false;
+            for (uint32_t polls = 0; !begun && polls < limit; ++polls) {
+                begun = true;
+                for (int i = t; i < (int)gridDim.x; i += kPersistBlock)
+                    begun = begun && (int32_t)(ld_relaxed(a.flags + i) - first) >= 0;
+            }
+            __threadfence();
+            if (!begun) atomicExch(a.err, 1);
+        }
+        __syncthreads_and(begun);
+    }
 }
 
 int grid_persist_capacity(int dim)

@@ -301,8 +301,9 @@ int lqt_sim_tissue_index(const lqt_sim *s, int64_t *grid_index_host);
 /* Advance nsteps of dt.  Simulated time accumulates as `time += dt` in FP64,
  * as the reference drivers do (OneD.cc:317).  Returns when the steps have run
  * on the device.  (Blocks of a small grid wait for one another inside one
- * launch; should such a wait run out, this call, lqt_sim_sync and
- * lqt_sim_check return LQT_ERR_CUDA and the run is not valid.) */
+ * launch; should such a wait run out, this call, lqt_sim_sync,
+ * lqt_sim_check and every call that reads results return LQT_ERR_CUDA, and
+ * further steps are refused: the run is not valid.) */
 int lqt_sim_step(lqt_sim *s, int64_t nsteps);
 /* The same steps, enqueued on the simulation's stream without waiting: a host
  * loop that issues one step at a time (with a read-back per step) keeps the

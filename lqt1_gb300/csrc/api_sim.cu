@@ -391,7 +391,8 @@ std::vector<int2> persist_deps(const TissueMap &tm, int dim, int64_t ny, int64_t
     return dep;
 }
 
-// Waits and device errors that a finished step left behind.
+// A wait that ran out inside a finished launch of many steps.  Every call that
+// starts steps, waits for them or hands out what they computed reports it.
 int persist_status(const lqt_sim *s)
 {
     if (s->persist_err && *(volatile int32_t *)s->persist_err)
@@ -968,6 +969,7 @@ int lqt_sim_set_protocol(lqt_sim *s, const lqt_protocol *q)
 // fit, single steps elsewhere); the host does not wait for them.
 static int sim_advance(lqt_sim *s, int64_t nsteps)
 {
+    if (const int rc = persist_status(s)) return rc;
     if (s->has_protocol && s->step + nsteps + kGraphChunk > s->win_horizon) {
         int rc = refresh_windows(s, s->step + nsteps + 200000);
         if (rc) return rc;
@@ -988,8 +990,6 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
             const bool ecg = s->nel > 0 && s->ecg_every > 0;
             int64_t m = std::min<int64_t>(left, kPersistMax);
             if (ecg) m = std::min<int64_t>(m, s->ecg_every - s->step % s->ecg_every);
-            int rc = persist_status(s);
-            if (rc) return rc;
             const PersistArgs a{s->persist_dep, s->persist_flags, s->persist_err_dev, (int)m};
             CK(launch_grid_persist(devf<float>(s), make_stepk(s->p.dt), s->cur, s->dim, a, s->stream));
             s->cur ^= (int)(m & 1);
@@ -997,7 +997,7 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
             for (int64_t i = 0; i < m; ++i) s->time += s->p.dt;
             left -= m;
             if (ecg && s->step % s->ecg_every == 0) {
-                rc = launch_ecg_now(s);
+                const int rc = launch_ecg_now(s);
                 if (rc) return rc;
             }
             continue;
@@ -1068,7 +1068,7 @@ int lqt_sim_get_v(lqt_sim *s, void *v_host, int as_double)
     }
     CK(cudaMemcpyAsync(v_host, tmp, n * esz, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_get_v_async(lqt_sim *s, void *v_host, int as_double)
@@ -1130,7 +1130,7 @@ int lqt_sim_wait_v(lqt_sim *s)
     if (!s) return fail(LQT_ERR_INVALID, "lqt_sim_wait_v: NULL");
     for (cudaStream_t c : s->copy_stream)
         if (c) CK(cudaStreamSynchronize(c));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_wait_v_upto(lqt_sim *s, int64_t seq)
@@ -1142,7 +1142,7 @@ int lqt_sim_wait_v_upto(lqt_sim *s, int64_t seq)
     // copies complete in order (each one's chunks join on copy stream 0);
     // the ones older than the last kVDone were waited for at issue
     if (seq >= s->v_issued - lqt_sim::kVDone) CK(cudaEventSynchronize(s->vdone[seq % lqt_sim::kVDone]));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_get_state(lqt_sim *s, double *state_host)
@@ -1165,7 +1165,7 @@ int lqt_sim_get_state(lqt_sim *s, double *state_host)
     if (e == cudaSuccess) e = cudaMemcpyAsync(state_host, s->aos, n * 320, cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return fail(LQT_ERR_CUDA, std::string("lqt_sim_get_state: ") + cudaGetErrorString(e));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_set_state(lqt_sim *s, const double *state_host)
@@ -1252,7 +1252,7 @@ int lqt_sim_get_ecg(lqt_sim *s, int64_t max_samples, double *phi, double *t, int
         std::memcpy(phi, buf.data(), m * s->nel * 8);
     }
     if (m > 0 && t) CK(cudaMemcpy(t, s->ecg_t, m * 8, cudaMemcpyDeviceToHost));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_get_detect(lqt_sim *s, float *t_act, float *apd90, uint8_t *ead)
@@ -1274,7 +1274,7 @@ int lqt_sim_get_detect(lqt_sim *s, float *t_act, float *apd90, uint8_t *ead)
         for (int64_t k = 0; k < n; ++k)
             if (!(apd90[k] == apd90[k])) apd90[k] = -1.f;
     }
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_tune(lqt_sim *s, int32_t variant, int32_t *chosen, float *ms_per_variant)
@@ -1292,6 +1292,7 @@ int lqt_sim_tune(lqt_sim *s, int32_t variant, int32_t *chosen, float *ms_per_var
         s->graph_valid = false;
     } else {
         int64_t used = 0;
+        if (const int bad = persist_status(s)) return bad;
         s->step_forced = false;
         int rc = autotune(s, 5, &used);
         if (rc) return rc;
@@ -1321,6 +1322,7 @@ int lqt_sim_substep_variant(lqt_sim *s, int32_t variant, int32_t *chosen, float 
 int lqt_sim_profile(lqt_sim *s, int64_t nsteps, double *ms_step, double *ms_ghost, double *ms_sur)
 {
     if (!s || nsteps <= 0) return fail(LQT_ERR_INVALID, "lqt_sim_profile: NULL handle or nsteps <= 0");
+    if (const int bad = persist_status(s)) return bad;
     cudaEvent_t ev[5];
     for (auto &e : ev) CK(cudaEventCreate(&e));
     double t_step = 0, t_ghost = 0, t_sur = 0;
@@ -1413,7 +1415,7 @@ int lqt_sim_sample_v(lqt_sim *s, int32_t stride, double *out_host, int64_t cap, 
     if (rc) return rc;
     CK(cudaMemcpyAsync(out_host, s->samp, cnt * 8, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    return LQT_OK;
+    return persist_status(s);
 }
 
 int lqt_sim_set_surrogate(lqt_sim *s, lqt_mlp *m, const lqt_sur_config *cfg)
@@ -1622,6 +1624,8 @@ struct lqt_vtk_writer {
             if (cudaEventSynchronize(ev[job.first]) != cudaSuccess) {
                 rc = LQT_ERR_CUDA;
                 msg = "lqt_vtk_writer: device copy failed";
+            } else if ((rc = persist_status(s)) != LQT_OK) {
+                msg = g_err;
             } else {
                 rc = write_vtk_file(job.second.c_str(), hbuf[job.first], s->nx, s->ny, s->nz, stride);
                 if (rc) msg = g_err;

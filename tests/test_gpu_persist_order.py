@@ -88,3 +88,31 @@ def test_every_block_steps_with_its_own_clock(kind, stim):
     for sim in many:
         for a, b in zip(outputs(sim), want):
             np.testing.assert_array_equal(a, b)
+
+
+def broken():
+    sim = make(islands((20, 30)), "window")
+    sim.step(10)
+    sim.set_wait_test(True, 2000)        # block 0 publishes nothing: its neighbours' waits run out
+    return sim
+
+
+def test_every_reader_reports_a_wait_that_ran_out(tmp_path):
+    """Results of steps that did not complete are not handed out as if they had."""
+    import torch
+    sim = broken()
+    sim.set_electrodes([(1.0, 1.0, 5.0)], every=50)
+    host = torch.empty(sim.n, dtype=torch.float32).pin_memory()
+    sim.step_async(10)
+    sim.get_v_async(host.numpy())
+    vtk = sim.vtk_writer(1)
+    vtk.submit(str(tmp_path / "v.vtk"))
+    for call in (lambda: sim.wait_v(upto=0), sim.wait_v, sim.sync, sim.get_v, sim.get_state, sim.detect, sim.ecg, sim.check,
+                 lambda: sim.sample_v(1), lambda: sim.checkpoint(str(tmp_path / "c.bin")), vtk.flush,
+                 lambda: sim.step_async(1), lambda: sim.step(2), lambda: sim.step(100),
+                 lambda: sim.tune(-1), lambda: sim.profile(2)):
+        with pytest.raises(lq.LqtError):
+            call()
+    vtk.close()
+    assert not (tmp_path / "v.vtk").exists() and not (tmp_path / "c.bin").exists()
+    sim.close()

@@ -813,11 +813,11 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
         const std::vector<int2> dep = persist_deps(s->tm, dim, ny, nz, n);
         int2 *d = nullptr;
         bool ok = !s->mem.alloc((void **)&d, dep.size() * sizeof(int2)) &&
-                  !s->mem.alloc((void **)&s->persist_flags, dep.size() * 4) &&
+                  !s->mem.alloc((void **)&s->persist_flags, (dep.size() + 1) * 4) &&
                   cudaHostAlloc((void **)&s->persist_err, 4, cudaHostAllocMapped) == cudaSuccess &&
                   cudaHostGetDevicePointer((void **)&s->persist_err_dev, s->persist_err, 0) == cudaSuccess &&
                   cudaMemcpy(d, dep.data(), dep.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemset(s->persist_flags, 0, dep.size() * 4) == cudaSuccess;
+                  cudaMemset(s->persist_flags, 0, (dep.size() + 1) * 4) == cudaSuccess;
         if (!ok) {
             delete s;
             return fail(LQT_ERR_NOMEM, "lqt_sim_create: step flags");

@@ -132,7 +132,8 @@ constexpr int kSmallPerSM = 512;
 constexpr int kPersistBlock = 128, kPersistPerSM = 1, kPersistMin = 3, kPersistMax = 500;
 struct PersistArgs {
     const int2 *dep;               // per block: the blocks whose V it reads or that read its V, [x, y]
-    uint32_t *flags;               // per block: steps published, the same in all blocks between launches
+    uint32_t *flags;               // per block: steps published, the same in all blocks between launches;
+                                   // then one word, not 0 once a wait has run out
     int32_t *err;                  // set when a wait ran out
     int nsteps;
 };

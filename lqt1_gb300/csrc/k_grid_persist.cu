@@ -19,7 +19,9 @@
 //
 // The launch is cooperative: every block is resident, so every wait ends.  It
 // is bounded all the same; one that runs out sets *err, the blocks leave, and
-// the run is reported as failed.
+// the run is reported as failed.  It also sets the word behind the flags, by
+// which launches that are queued already leave at once instead of waiting in
+// their turn.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -29,7 +31,7 @@ namespace lqt {
 
 namespace {
 
-constexpr uint32_t kPersistPolls = 1u << 23;     // seconds
+constexpr uint32_t kPersistPolls = 1u << 23;     // a second or more
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
 {
@@ -46,6 +48,12 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p)
 __device__ __forceinline__ void st_release(uint32_t *p, uint32_t v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void ran_out(const PersistArgs &a)
+{
+    atomicExch(a.err, 1);
+    atomicExch(a.flags + gridDim.x, 1u);
 }
 
 // What a voxel's diffusion needs besides V, for the whole launch.
@@ -101,19 +109,20 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
     // three clocks: the detector of step s runs beside the making of s + 2's
     __shared__ Clock clk[3];
     __shared__ int go;
-    __shared__ uint32_t base;             // steps published when the launch begins
+    __shared__ uint32_t base, dead;       // steps published, or a wait run out, when the launch begins
     const int t = threadIdx.x, b = blockIdx.x;
     const uint32_t limit = gd.sub_wait_limit ? gd.sub_wait_limit : kPersistPolls;
     if (t == kPersistBlock) {
         clk[0] = gd.clk[cur];
         base = a.flags[b];
+        dead = ld_relaxed(a.flags + gridDim.x);
     }
     __syncthreads();
     if (t >= kPersistBlock) {
         const int lane = t - kPersistBlock;
         const int2 dep = a.dep[b];
         const uint32_t base0 = base;
-        bool ok = true;
+        bool ok = dead == 0;
         for (int s = 0; s < a.nsteps; ++s) {
             if (lane == 0) clk[(s + 1) % 3] = next_clock(gd, clk[s % 3]);
             if (s > 0) {
@@ -126,7 +135,7 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
             ok = __all_sync(0xffffffffu, ok);
             if (lane == 0) {
                 go = ok;
-                if (!ok) atomicExch(a.err, 1);
+                if (!ok) ran_out(a);
             }
             __syncthreads();
             if (!ok) break;
@@ -208,7 +217,7 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
                     begun = begun && (int32_t)(ld_relaxed(a.flags + i) - first) >= 0;
             }
             __threadfence();
-            if (!begun) atomicExch(a.err, 1);
+            if (!begun) ran_out(a);
         }
         __syncthreads_and(begun);
     }

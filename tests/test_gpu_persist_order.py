@@ -116,3 +116,20 @@ def test_every_reader_reports_a_wait_that_ran_out(tmp_path):
     vtk.close()
     assert not (tmp_path / "v.vtk").exists() and not (tmp_path / "c.bin").exists()
     sim.close()
+
+
+def test_queued_launches_leave_once_a_wait_has_run_out():
+    """With a bound of 2^21 polls per wait (0.3 s at the 150 ns of a poll), 40
+    launches queued behind the one whose wait runs out would take over ten
+    seconds; they end with it."""
+    import time
+    sim = broken()
+    sim.set_wait_test(True, 1 << 21)
+    t0 = time.perf_counter()
+    with pytest.raises(lq.LqtError):
+        for _ in range(40):
+            sim.step_async(10)
+        sim.sync()
+    one = time.perf_counter() - t0
+    sim.close()
+    assert one < 5.0

@@ -303,7 +303,8 @@ int lqt_sim_tissue_index(const lqt_sim *s, int64_t *grid_index_host);
  * on the device.  (Blocks of a small grid wait for one another inside one
  * launch; should such a wait run out, this call, lqt_sim_sync,
  * lqt_sim_check and every call that reads results return LQT_ERR_CUDA, and
- * further steps are refused: the run is not valid.) */
+ * further steps are refused, until lqt_sim_set_state or lqt_sim_restore gives
+ * the simulation a whole new state: the run is not valid.) */
 int lqt_sim_step(lqt_sim *s, int64_t nsteps);
 /* The same steps, enqueued on the simulation's stream without waiting: a host
  * loop that issues one step at a time (with a read-back per step) keeps the

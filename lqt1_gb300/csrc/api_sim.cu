@@ -89,6 +89,7 @@ struct lqt_sim {
     // published steps, and the error word in mapped host memory
     int2 *persist_dep = nullptr;
     uint32_t *persist_flags = nullptr;
+    int64_t persist_nflags = 0;
     int32_t *persist_err = nullptr, *persist_err_dev = nullptr;
     bool step_forced = false;       // set by lqt_sim_tune with a variant
     bool sub_forced = false;        // set by lqt_sim_substep_variant: the autotuner keeps it
@@ -811,13 +812,14 @@ int lqt_sim_create(const lqt_sim_params *params, const lqt_geometry *geom, lqt_s
     }
     if (!s->fp64() && (n + kPersistBlock - 1) / kPersistBlock <= grid_persist_capacity(dim)) {
         const std::vector<int2> dep = persist_deps(s->tm, dim, ny, nz, n);
+        s->persist_nflags = (int64_t)dep.size() + 1;
         int2 *d = nullptr;
         bool ok = !s->mem.alloc((void **)&d, dep.size() * sizeof(int2)) &&
-                  !s->mem.alloc((void **)&s->persist_flags, (dep.size() + 1) * 4) &&
+                  !s->mem.alloc((void **)&s->persist_flags, s->persist_nflags * 4) &&
                   cudaHostAlloc((void **)&s->persist_err, 4, cudaHostAllocMapped) == cudaSuccess &&
                   cudaHostGetDevicePointer((void **)&s->persist_err_dev, s->persist_err, 0) == cudaSuccess &&
                   cudaMemcpy(d, dep.data(), dep.size() * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemset(s->persist_flags, 0, (dep.size() + 1) * 4) == cudaSuccess;
+                  cudaMemset(s->persist_flags, 0, s->persist_nflags * 4) == cudaSuccess;
         if (!ok) {
             delete s;
             return fail(LQT_ERR_NOMEM, "lqt_sim_create: step flags");
@@ -1192,6 +1194,13 @@ int lqt_sim_set_state(lqt_sim *s, const double *state_host)
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return fail(LQT_ERR_CUDA, std::string("lqt_sim_set_state: ") + cudaGetErrorString(e));
+    // a whole new state is a valid one again after a wait that ran out: the
+    // blocks, whose counts of steps differ since, start from equal flags
+    if (s->persist_err && *(volatile int32_t *)s->persist_err) {
+        CK(cudaMemsetAsync(s->persist_flags, 0, s->persist_nflags * 4, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        *(volatile int32_t *)s->persist_err = 0;
+    }
     // a new state ends any macro step in progress: every voxel runs the plain
     // step until the next macro-step boundary
     if (s->srate) CK(cudaMemset(s->srate, 0xff, s->ntissue * 4));

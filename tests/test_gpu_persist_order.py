@@ -133,3 +133,28 @@ def test_queued_launches_leave_once_a_wait_has_run_out():
     one = time.perf_counter() - t0
     sim.close()
     assert one < 5.0
+
+
+def test_new_state_after_a_wait_that_ran_out(tmp_path):
+    """A restored checkpoint runs on as it would have without the failure."""
+    path = str(tmp_path / "c.bin")
+    res = []
+    for fail in (False, True):
+        sim = make(islands((20, 30)), "window")
+        sim.step(10)
+        sim.checkpoint(path)
+        if fail:
+            sim.set_wait_test(True, 2000)
+            sim.step_async(10)
+            with pytest.raises(lq.LqtError):
+                sim.sync()
+            sim.set_wait_test(False)
+            with pytest.raises(lq.LqtError):
+                sim.step(4)
+            sim.restore(path)
+        sim.step(4)
+        sim.step(20)
+        res.append([sim.get_state(), np.array([sim.time])])
+        sim.close()
+    for a, b in zip(*res):
+        np.testing.assert_array_equal(a, b)

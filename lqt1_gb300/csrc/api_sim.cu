@@ -988,10 +988,14 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
         left -= used;
     }
     while (left > 0) {
-        if (persist && left >= kPersistMin) {
-            const bool ecg = s->nel > 0 && s->ecg_every > 0;
-            int64_t m = std::min<int64_t>(left, kPersistMax);
-            if (ecg) m = std::min<int64_t>(m, s->ecg_every - s->step % s->ecg_every);
+        // graph replay fits: a whole chunk from a chunk boundary
+        const bool replay = left >= kGraphChunk && s->step % kGraphChunk == 0 &&
+                            (s->ecg_every <= 0 || kGraphChunk % s->ecg_every == 0);
+        // a launch of many steps ends where the pseudo-ECG samples V
+        const bool ecg = s->nel > 0 && s->ecg_every > 0;
+        int64_t m = std::min<int64_t>(left, kPersistMax);
+        if (ecg) m = std::min<int64_t>(m, s->ecg_every - s->step % s->ecg_every);
+        if (persist && m >= kPersistMin && !(replay && ecg && s->ecg_every < kPersistEcg)) {
             const PersistArgs a{s->persist_dep, s->persist_flags, s->persist_err_dev, (int)m};
             CK(launch_grid_persist(devf<float>(s), make_stepk(s->p.dt), s->cur, s->dim, a, s->stream));
             s->cur ^= (int)(m & 1);
@@ -1004,9 +1008,7 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
             }
             continue;
         }
-        // graph replay for whole chunks starting on a chunk boundary
-        if (left >= kGraphChunk && s->step % kGraphChunk == 0 &&
-            (s->ecg_every <= 0 || kGraphChunk % s->ecg_every == 0)) {
+        if (replay) {
             if (!s->graph_valid || s->graph_cur != s->cur) {
                 int rc = build_graph(s);
                 if (rc) return rc;

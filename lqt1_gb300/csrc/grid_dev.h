@@ -128,8 +128,11 @@ constexpr int kSmallPerSM = 512;
 // 128 voxels per SM in the mixed form, for runs of at least kPersistMin steps.
 // Up to there a step takes 2.6..3.0 us against 5.5 in a launch of its own; with
 // two blocks per SM 4.2..5.9 against 4.5..5.0, so larger grids stay with the
-// launch per step.
-constexpr int kPersistBlock = 128, kPersistPerSM = 1, kPersistMin = 3, kPersistMax = 500;
+// launch per step.  A launch ends where the pseudo-ECG samples V; with samples
+// closer than kPersistEcg steps a replayed graph of single steps is faster (97 x
+// 64 voxels, us a step: every 2 steps 6.8 against 9.3, every 5 5.0 against 5.2,
+// every 10 4.4 against 4.0).
+constexpr int kPersistBlock = 128, kPersistPerSM = 1, kPersistMin = 3, kPersistMax = 500, kPersistEcg = 10;
 struct PersistArgs {
     const int2 *dep;               // per block: the blocks whose V it reads or that read its V, [x, y]
     uint32_t *flags;               // per block: steps published, the same in all blocks between launches;

@@ -113,9 +113,12 @@ __global__ void __launch_bounds__(kPersistBlock + 32, 3)
     const int t = threadIdx.x, b = blockIdx.x;
     const uint32_t limit = gd.sub_wait_limit ? gd.sub_wait_limit : kPersistPolls;
     if (t == kPersistBlock) {
-        clk[0] = gd.clk[cur];
-        base = a.flags[b];
-        dead = ld_relaxed(a.flags + gridDim.x);
+        // (three loads in flight together)
+        const uint32_t f = ld_relaxed(a.flags + b), out = ld_relaxed(a.flags + gridDim.x);
+        const Clock c0 = gd.clk[cur];
+        clk[0] = c0;
+        base = f;
+        dead = out;
     }
     __syncthreads();
     if (t >= kPersistBlock) {

@@ -158,3 +158,22 @@ def test_new_state_after_a_wait_that_ran_out(tmp_path):
         sim.close()
     for a, b in zip(*res):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("every", [1, 2, 5, 10, 100])
+def test_ecg_cadence(every):
+    """Launches of many steps, replayed graphs and single steps take turns as the
+    pseudo-ECG's cadence and the calls cut them: the same bits and samples."""
+    t = islands((20, 30))
+    res = []
+    for forced in (False, True):
+        sim = make(t, "window")
+        sim.set_electrodes([(2.0, 3.0, 4.0)], every=every)
+        if forced:
+            sim.tune(2)
+        for n in (3, 4, 43, 50, 100, 7, 93, 111):
+            sim.step(n)
+        res.append([sim.get_state(), *sim.ecg()])
+        sim.close()
+    for a, b in zip(*res):
+        np.testing.assert_array_equal(a, b)

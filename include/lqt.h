@@ -370,9 +370,10 @@ int lqt_sim_get_detect(lqt_sim *s, float *t_act_host, float *apd90_host,
  * the variant of the V-only substep kernel).  The first lqt_sim_step call of at
  * least 64 steps, and of no fewer than the rounds take, autotunes by itself
  * unless a variant was forced.  Small grids (at most 512 voxels per SM) in the
- * mixed form use a kernel of their own unless a variant is forced.  All variants
- * give bit-identical results.
- * ms_per_variant: up to 4 timings (or NULL). */
+ * mixed form use a kernel of their own unless a variant is forced; there is
+ * nothing to choose there, and the autotuner steps and times that kernel alone.
+ * All variants give bit-identical results.
+ * ms_per_variant: up to 4 timings, 0 for variants that were not timed (or NULL). */
 int lqt_sim_tune(lqt_sim *s, int32_t variant, int32_t *chosen, float *ms_per_variant);
 
 /* Kernel of the V-only substep inside a surrogate macro step: 5, 6, 8 = one

@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstring>
 #include <deque>
+#include <iterator>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -494,6 +495,15 @@ int step_once(lqt_sim *s)
     return LQT_OK;
 }
 
+// What the autotuner has to choose from: variants of the plain step (one where
+// all are the same kernel: strands, and small grids, whose step is one launch of
+// its own), and whether those of the substep.
+int tune_variants(const lqt_sim *s)
+{
+    return s->dim == 1 || s->folds() ? 1 : (s->fp64() ? 2 : kGridNVariantsF32);
+}
+bool tunes_substep(const lqt_sim *s) { return s->sur && !s->fp64() && !s->sub_forced && !s->folds(); }
+
 // Autotuner: time `per` real steps with each occupancy variant of the step
 // kernels (CUDA events around the step kernels only) and keep the fastest.
 // The variants take turns step by step, so each sees the same phases of the
@@ -504,7 +514,7 @@ int step_once(lqt_sim *s)
 int autotune(lqt_sim *s, int per, int64_t *consumed)
 {
     const int *cand = s->fp64() ? kGridVariantsF64 : kGridVariantsF32;
-    const int ncand = s->dim == 1 ? 1 : (s->fp64() ? 2 : kGridNVariantsF32);
+    const int ncand = tune_variants(s);
     cudaEvent_t a, b;
     CK(cudaEventCreate(&a));
     CK(cudaEventCreate(&b));
@@ -537,6 +547,7 @@ int autotune(lqt_sim *s, int per, int64_t *consumed)
     }
     float best = 1e30f;
     int best_m = cand[0];
+    std::fill(std::begin(s->tune_ms), std::end(s->tune_ms), 0.f);
     for (int c = 0; c < ncand; ++c) {
         const float avg = per > 1 ? tot[c] / (per - 1) : tot[c];
         s->tune_ms[c] = avg;
@@ -548,7 +559,7 @@ int autotune(lqt_sim *s, int per, int64_t *consumed)
     s->minb = best_m;
     // with a surrogate attached: the V-only substep's variant, timed the same
     // way (variants in turn, whole steps, the first round discarded)
-    if (rc == LQT_OK && s->sur && !s->fp64() && !s->sub_forced && !s->folds()) {
+    if (rc == LQT_OK && tunes_substep(s)) {
         float ts[kSubNVariants] = {};
         for (int i = 0; i < per && rc == LQT_OK; ++i) {
             for (int c = 0; c < kSubNVariants && rc == LQT_OK; ++c) {
@@ -977,11 +988,10 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
         if (rc) return rc;
     }
     int64_t left = nsteps;
-    // (a call shorter than the autotuner's steps does not start it)
-    // (with many steps in one launch the autotuner has nothing to choose)
     const bool persist = s->persists();
+    // (a call shorter than the autotuner's steps does not start it)
     const int64_t tune_steps = 5 * ((s->fp64() ? 2 : kGridNVariantsF32) + (s->sur ? kSubNVariants : 0));
-    if (!persist && !s->tuned && left >= std::max<int64_t>(64, tune_steps)) {
+    if (!s->tuned && left >= std::max<int64_t>(64, tune_steps) && (tune_variants(s) > 1 || tunes_substep(s))) {
         int64_t used = 0;
         int rc = autotune(s, 5, &used);
         if (rc) return rc;

@@ -368,7 +368,7 @@ int lqt_sim_get_detect(lqt_sim *s, float *t_act_host, float *apd90_host,
  * now (real steps, the variants in turn, five rounds, each timed with CUDA
  * events, the fastest kept; with a surrogate attached, five more rounds pick
  * the variant of the V-only substep kernel).  The first lqt_sim_step call of at
- * least 64 steps, and of no fewer than the rounds take, autotunes by itself
+ * least 64 steps autotunes by itself, with as many rounds as it has steps for,
  * unless a variant was forced.  Small grids (at most 512 voxels per SM) in the
  * mixed form use a kernel of their own unless a variant is forced; there is
  * nothing to choose there, and the autotuner steps and times that kernel alone.

@@ -989,11 +989,12 @@ static int sim_advance(lqt_sim *s, int64_t nsteps)
     }
     int64_t left = nsteps;
     const bool persist = s->persists();
-    // (a call shorter than the autotuner's steps does not start it)
-    const int64_t tune_steps = 5 * ((s->fp64() ? 2 : kGridNVariantsF32) + (s->sur ? kSubNVariants : 0));
-    if (!s->tuned && left >= std::max<int64_t>(64, tune_steps) && (tune_variants(s) > 1 || tunes_substep(s))) {
+    // A call of 64 steps or more starts the autotuner, where there is something
+    // to choose, with as many rounds as the call holds, five at the most.
+    const int round = tune_variants(s) + (tunes_substep(s) ? kSubNVariants : 0);
+    if (!s->tuned && left >= 64 && round > 1) {
         int64_t used = 0;
-        int rc = autotune(s, 5, &used);
+        int rc = autotune(s, (int)std::min<int64_t>(5, left / round), &used);
         if (rc) return rc;
         left -= used;
     }

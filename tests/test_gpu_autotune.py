@@ -1,5 +1,6 @@
-"""Where the autotuner has nothing to choose: small grids, whose step is one launch
-of its own kernel."""
+"""When the autotuner runs: a call of 64 steps starts it and steps 64 steps, with a
+surrogate attached too; small grids, whose step is one launch of its own kernel,
+have nothing to choose and say so."""
 import numpy as np
 import pytest
 
@@ -15,6 +16,17 @@ def sheet(n, **kw):
     sim = lq.Sim(types=sh.types, fibre=f, dx=0.15, model=lq.model("baseline", gks_scale=0.5, pca_scale=2.0, gks_iso_scale=1.5), **kw)
     sim.set_protocol(bcl=500.0, s1_mask=sh.s1_mask)
     return sim
+
+
+@pytest.mark.parametrize("nsteps", [63, 64, 74, 75, 100])
+def test_call_that_starts_it(nsteps):
+    sim = sheet(300)                     # above the small grids (77,824 voxels at 152 SMs)
+    sim.set_surrogate(lq.surrogate.load())
+    sim.step(nsteps)
+    assert abs(sim.time - 0.02 * nsteps) < 1e-9
+    ms = sim.substep_variant(-1, timings=True)[1]
+    assert bool((np.asarray(ms) > 0).all()) == (nsteps >= 64)
+    sim.close()
 
 
 @pytest.mark.parametrize("n", [40, 200])

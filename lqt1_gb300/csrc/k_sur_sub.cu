@@ -542,16 +542,17 @@ template <int DIM> __global__ void __launch_bounds__(256, 2) k_list_ghost(GridDe
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const bool on = 4 * j + i < gd.nbnd;
-            src[i] = on ? gd.bnd_src[4 * j + i] : -1;
+            src[i] = on ? gd.bnd_src[4 * j + i] : 0;
             dst[i] = on ? gd.bnd_dst[4 * j + i] : 0;
-            k[i] = on ? gd.bnd_k[4 * j + i] : 0;
+            k[i] = on ? gd.bnd_k[4 * j + i] : -1;
         }
     }
+    // (k < 0: no entry, or one without a tissue source, which has nothing to copy)
     float r[4], v[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        r[i] = src[i] >= 0 ? gd.srate[k[i]] : __int_as_float(0x7fc00000);
-        v[i] = src[i] >= 0 ? V[src[i]] : 0.f;      // (not used where the list steps the source)
+        r[i] = k[i] >= 0 ? gd.srate[k[i]] : __int_as_float(0x7fc00000);
+        v[i] = k[i] >= 0 ? V[src[i]] : 0.f;        // (not used where the list steps the source)
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)

@@ -53,7 +53,7 @@ enum {
 
 /* ---- precision forms --------------------------------------------------- */
 enum {
-    LQT_FP64 = 0,               /* plain FP64 everywhere (the reference's arithmetic) */
+    LQT_FP64 = 0,               /* FP64 everywhere (the reference's formulas in double precision) */
     LQT_MIXED = 1               /* FP32; concentrations as pairs of FP32 (hi + lo) */
 };
 

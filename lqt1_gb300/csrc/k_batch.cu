@@ -128,7 +128,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(BatchDev<R> b, StepT<R> k)
         // hundred instructions): rec_in steps to the next recorded one, which
         // is sample rec_slot
         int64_t rec_in = 0, rec_slot = 0;
-        // this cell's electrode weight, -1/r^2
+        // this cell's electrode weight, -1/r^2 (once: a sample's term then has one
+        // FP64 rounding more than dividing by r^2 each time)
         const bool ecg = item.ecg_seg >= 0;
         double ecg_w = 0.0;
         if (ecg && active) {

@@ -19,8 +19,8 @@
 //
 // Sixteen steps amplify the last bit of a sum through the weights' BF16
 // rounding, so the sums have one order that does not depend on how the work is
-// laid out: a weight's by slices of at most 1/128 of the batch (whole half
-// tiles), a bias's by row mod 256 and a tree.
+// laid out: a weight's by at most 128 slices of whole half tiles, a bias's by
+// row mod 256 and a tree.
 //
 // What bounds it: one tile's serial chain of five GEMMs and their epilogues
 // (a batch of 8192 is 128 half tiles on 152 SMs); tensor time and traffic are

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sur_grid(GridDev<float> gd, Sur
         nrm[2 * kMlpIn + 2 * j + 1] = sg.kappa * sg.norm[3 * kMlpIn + j];
     }
     if (use_net) {
-        // hidden layers halved (see silu2_bf16); biases as an extra k-step
+        // hidden layers halved (see silu2_f16); biases as an extra k-step
         stage_kmajor(smem + kOffW1, sg.w.w1t, kMlpHid, kMlpIn, 0.5f);
         stage_kmajor_f16(smem + kOffW2, sg.w.w2f, kMlpHid, kMlpHid, 0.5f);
         stage_kmajor_f16(smem + kOffW3, sg.w.w3f, kMlpOut, kMlpHid, 1.0f);

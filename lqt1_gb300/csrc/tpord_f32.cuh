@@ -25,10 +25,17 @@
 // Measured (GB300): 20,011 cells x 1000 updates 2.62 -> 1.84 ms, 320 x 320 x
 // 420 ventricle with the surrogate, 50 steps, 11.40 -> 10.36 ms, mixed shell of
 // 1.11 M voxels, 50 steps, 5.65 -> 5.22 ms; errors against 64 bits unchanged
-// (7.6e-7 of the state after 1000 updates in both writings).  The batch kernel
-// (k_batch.cu) keeps the term-by-term writing of tpord.cuh: its results carry
-// activation times rounded to the step, and a last-bit change of V moves a few
-// of them by one step.
+// (7.6e-7 of the state after 1000 updates in both writings).  Single
+// exponentials are not all as close as term by term: exp((v + a) / k) is one FMA
+// with a / k rounded to FP32, so near v = -a its argument is off by up to half a
+// unit of a number of 2..17 (1e-6 of the result at the most), as much as half a
+// unit of v itself is worth; and e^x - 1 of the GHK terms beyond |x| = 0.5 is a
+// difference of the hardware's ex2 (a few 2^-23).
+// The batch kernel (k_batch.cu) keeps the term-by-term writing of tpord.cuh.  A
+// last-bit change of V moves a few activation times, which are multiples of the
+// step, by one step, and their bits are kept.  It is no nearer to 64 bits: of
+// 36,132 activations of a sweep of strands 14 differ from the FP64 form's, 15
+// with the writing here.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -18,10 +18,10 @@
 //     concentration is kept off zero by 1e-60 (kTinyD).
 // Each of these is within a few units of 2^-53; the argument (v + a) / k of an
 // exponential is one FMA with a / k rounded, so near v = -a, where the sum
-// cancels, it is up to 25 such units off and not a fraction of one.  A state
-// after one step agrees with the oracle to 6e-12 of its size at the worst and
-// 3e-14 in 99.9 of 100 states (20,000 cells, -120 to 80 mV), V to 3e-16 of its
-// change's terms.  Measured (GB300): shell of 78k voxels 684 -> 297 us a step.
+// cancels, it is up to 25 such units off and not a fraction of one.  After one
+// step of 20,000 cells (-120 to 80 mV) the state values agree with the oracle to
+// 6e-12 of their size at the worst and 99.9% of them to 3e-14, V to 3e-16.
+// Measured (GB300): shell of 78k voxels 684 -> 297 us a step.
 #pragma once
 #include <cuda_runtime.h>
 
